@@ -72,7 +72,6 @@ CorrPlanDev corr_plan_dev(bool exact, bool three) {
 }
 
 Engine::Engine(int dev) : device(dev) {
-    if (const char* v = getenv("ZCMIR_B200_ROW_PASS")) row_pass = v;
     if (const char* v = getenv("ZCMIR_B200_SPECTRA_CACHE")) spectra_cache_ = atoi(v) != 0;
     cudaSetDevice(dev);
     cudaGetDeviceProperties(&prop, dev);
@@ -499,7 +498,6 @@ bool Engine::plan_map(const Mat3& Hm, bool exact, bool calibrated, unsigned cap,
     const CorrPlanDev& P = job.plan;
     if (!line_plan(g.nx, job.row) || !line_plan(g.ny, job.col)) return false;
     job.S = row_split(g.nx, P.n_corr);
-    if (job.S == 0) return fail("shift_map: row of " + std::to_string(g.nx) + " does not split to fit shared memory");
     if (!line_plan(g.nx / job.S, job.line)) return false;
     const unsigned floor_n = min_overlap > 0 ? (unsigned)std::floor(min_overlap * (double)g.cw * (double)g.ch) : 0u;
     const double gcell = (double)g.W / (double)g.cw;
@@ -653,22 +651,28 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
     // the correlation area (from both sides' autocorrelations) enters the row pass's score
     if (!finish_acf()) return false;
     job.cp.area = std::max(1.0, pair_area() * (1.0 / (job.gcell * job.gcell)));
-    const bool tmem = row_pass != "split" && rows_tmem_supported(g.nx, job.plan.n_corr);
-    if (tmem && host_map) {
-        // the map's rows in chunks of whole waves (one block per SM per row), each chunk copied to
-        // the host on the copy stream while the next chunk runs; the last chunk is the smallest,
-        // so little copy is left after the last kernel
+    const bool tmem = rows_tmem_supported(g.nx, job.plan.n_corr);
+    if (!tmem &&
+        !cuda_ok(inverse_rows(q_.as<float2>(), g, job.plan, job.line, job.S, twiddles(g.nx), st), "inverse rows"))
+        return false;
+    auto scores = [&](int y0, int rows) {
+        if (tmem)
+            return cuda_ok(inverse_rows_score_tmem(q_.as<float2>(), g, job.plan, twiddles(g.nx), job.cp, n00,
+                                                   map_.as<float>(), best, zero, st, y0, rows),
+                           "inverse rows (tensor memory)");
+        return cuda_ok(map_scores(q_.as<float2>(), g, job.cp, n00, map_.as<float>(), best, zero, st, 1, 0, 0, y0, rows),
+                       "scores");
+    };
+    if (host_map) {
+        // the map's rows in chunks, each copied to the host on the copy stream while the next chunk
+        // is scored; the last chunk is the smallest, so little copy is left after the last kernel
         if (!copy_st_ && !cuda_ok(cudaStreamCreateWithFlags(&copy_st_, cudaStreamNonBlocking), "shift_map")) return false;
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        const int big = 4 * sms;
+        // (whole waves of the tensor-memory pass, one block per SM and row)
+        const int big = tmem ? 4 * std::max(1, prop.multiProcessorCount) : std::max(64, (1 << 20) / g.nx);
         int y0 = 0, c = 0;
         while (y0 < g.ny) {
-            const int rows = (g.ny - y0 > big + sms) ? big : g.ny - y0;
-            if (!cuda_ok(inverse_rows_score_tmem(q_.as<float2>(), g, job.plan, twiddles(g.nx), job.cp, n00,
-                                                 map_.as<float>(), best, zero, st, y0, rows),
-                         "inverse rows (tensor memory)"))
-                return false;
+            const int rows = (g.ny - y0 > big + big / 4) ? big : g.ny - y0;
+            if (!scores(y0, rows)) return false;
             if (!chunk_ev_[c] && !cuda_ok(cudaEventCreateWithFlags(&chunk_ev_[c], cudaEventDisableTiming), "shift_map"))
                 return false;
             const size_t off = (size_t)y0 * g.nx;
@@ -682,17 +686,11 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
             c = (c + 1) % kChunkEvents;
         }
         counts[2]++;
-    } else if (tmem) {
-        if (!cuda_ok(inverse_rows_score_tmem(q_.as<float2>(), g, job.plan, twiddles(g.nx), job.cp, n00, map_.as<float>(),
-                                             best, zero, st),
-                     "inverse rows (tensor memory)"))
-            return false;
-    } else if (!cuda_ok(inverse_rows_score(q_.as<float2>(), g, job.plan, job.line, job.S, twiddles(g.nx), job.cp, n00,
-                                           map_.as<float>(), best, zero, st),
-                        "inverse rows"))
+    } else if (!scores(0, -1)) {
         return false;
+    }
     rec(5);
-    counts[0] += (job.identity_grid ? 10 : 12) - (have[0] ? (job.identity_grid ? 3 : 4) : 0) -
+    counts[0] += (job.identity_grid ? 11 : 13) - (have[0] ? (job.identity_grid ? 3 : 4) : 0) -
                  (have[1] ? (job.identity_grid ? 3 : 4) : 0);
     return true;
 }
@@ -706,18 +704,12 @@ bool Engine::shift_map(const Mat3& Hm, bool exact, bool calibrated, unsigned cap
     cudaEvent_t ev[kNumStages + 1];
     if (profiling)
         for (auto& e : ev) cudaEventCreate(&e);
-    // with the tensor-memory row pass the map leaves in row chunks during the pass (copy_st_)
-    const bool chunked = map && row_pass != "split" && rows_tmem_supported(job.g.nx, job.plan.n_corr);
-    if (!run_map(job, profiling ? ev : nullptr, chunked ? map : nullptr)) return false;
+    if (!run_map(job, profiling ? ev : nullptr, map)) return false;
     unsigned char host[32];
     if (!cuda_ok(cudaMemcpyAsync(host, res_.p, 32, cudaMemcpyDeviceToHost, st), "shift_map")) return false;
     counts[2]++;
-    if (map && !chunked) {
-        if (!cuda_ok(cudaMemcpyAsync(map, map_.p, nn * 4, cudaMemcpyDeviceToHost, st), "shift_map")) return false;
-        counts[2]++;
-    }
     if (!cuda_ok(cudaStreamSynchronize(st), "shift_map") ||
-        (chunked && !cuda_ok(cudaStreamSynchronize(copy_st_), "shift_map")))
+        (map && !cuda_ok(cudaStreamSynchronize(copy_st_), "shift_map")))
         return false;
     counts[1]++;
     counts[3]++;

@@ -187,7 +187,6 @@ class Engine {
     bool profiling = false;
     // the last pass: "tmem" (sums in tensor memory, whole rows) or "split" (rows split S ways,
     // sums in shared memory); from ZCMIR_B200_ROW_PASS at creation, "tmem" by default
-    std::string row_pass = "tmem";
     std::map<std::string, std::pair<double, uint32_t>> prof;  // name → (ms, count)
 
     bool fail(const std::string& m);

@@ -84,7 +84,6 @@ bool Engine::ncc_shift_map(const Mat3& H, zc_shift_result* out, float* map, size
     LinePlan row, col, line;
     if (!line_plan(g.nx, row) || !line_plan(g.ny, col)) return false;
     const int S = row_split(g.nx, plan.n_corr);
-    if (S == 0) return fail("shift_map: a row of " + std::to_string(g.nx) + " does not fit the row pass");
     if (!line_plan(g.nx / S, line)) return false;
     const float2* tw = twiddles(g.nx);
     if (!tw) return fail("shift_map: twiddles: out of device memory");
@@ -118,14 +117,15 @@ bool Engine::ncc_shift_map(const Mat3& H, zc_shift_result* out, float* map, size
         !cuda_ok(forward_cols(half_b_.as<float2>(), g, plan, col, st), "shift_map") ||
         !cuda_ok(inverse_columns(half_a_.as<float2>(), half_b_.as<float2>(), g, plan, col, q_.as<float2>(), st),
                  "shift_map") ||
-        !cuda_ok(inverse_rows_score(q_.as<float2>(), g, plan, line, S, tw, cp, den, map_.as<float>(), best, zero, st),
+        !cuda_ok(inverse_rows(q_.as<float2>(), g, plan, line, S, tw, st), "shift_map") ||
+        !cuda_ok(map_scores(q_.as<float2>(), g, cp, den, map_.as<float>(), best, zero, st),
                  "shift_map"))
         return false;
     unsigned char host[16];
     ok = cuda_ok(cudaMemcpyAsync(host, res, 16, cudaMemcpyDeviceToHost, st), "shift_map");
     if (ok && map) ok = cuda_ok(cudaMemcpyAsync(map, map_.p, nn * 4, cudaMemcpyDeviceToHost, st), "shift_map");
     if (!ok || !cuda_ok(cudaStreamSynchronize(st), "shift_map")) return false;
-    counts[0] += 11;
+    counts[0] += 12;
     counts[1]++;
     counts[2] += map ? 2 : 1;
     counts[3]++;

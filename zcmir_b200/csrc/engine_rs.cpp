@@ -68,7 +68,6 @@ bool Engine::rs_map_one(const Mat3& H, const double c[2], double r0_opt, double 
     LinePlan row, col, line;
     if (!line_plan(g.nx, row) || !line_plan(g.ny, col)) return false;
     const int S = row_split(g.nx, plan.n_corr);
-    if (S == 0) return fail("rs_map: a row of " + std::to_string(g.nx) + " does not fit the row pass");
     if (!line_plan(g.nx / S, line)) return false;
     const float2* tw = twiddles(g.nx);
     if (!tw) return fail("rs_map: twiddles: out of device memory");
@@ -114,11 +113,11 @@ bool Engine::rs_map_one(const Mat3& H, const double c[2], double r0_opt, double 
         !cuda_ok(forward_cols(half_b_.as<float2>(), g, plan, col, st), "rs_map") ||
         !cuda_ok(inverse_columns(half_a_.as<float2>(), half_b_.as<float2>(), g, plan, col, q_.as<float2>(), st),
                  "rs_map") ||
-        !cuda_ok(inverse_rows_score(q_.as<float2>(), g, plan, line, S, tw, cp, n00, dst.as<float>(), nullptr, nullptr,
-                                    st),
+        !cuda_ok(inverse_rows(q_.as<float2>(), g, plan, line, S, tw, st), "rs_map") ||
+        !cuda_ok(map_scores(q_.as<float2>(), g, cp, n00, dst.as<float>(), nullptr, nullptr, st),
                  "rs_map"))
         return false;
-    counts[0] += 11;
+    counts[0] += 12;
     return true;
 }
 

@@ -172,7 +172,6 @@ bool Engine::sweep_maps(const Mat3& H0, const SweepGrid& gv, int G, bool exact, 
         // line plans and twiddles now: nothing may allocate while the launches are captured
         if (!line_plan(c.nx, c.row) || !line_plan(c.ny, c.col)) return false;
         c.S = row_split(c.nx, plan.n_corr);
-        if (c.S == 0) return fail("sweep: a plane row of " + std::to_string(c.nx) + " does not fit the row pass");
         if (!line_plan(c.nx / c.S, c.line)) return false;
         c.tw = twiddles(c.nx);
         if (!c.tw) return fail("sweep: twiddles: out of device memory");
@@ -253,15 +252,15 @@ bool Engine::sweep_maps(const Mat3& H0, const SweepGrid& gv, int G, bool exact, 
                     !cuda_ok(inverse_columns(sw_half_.as<float2>(), sw_fhalf_.as<float2>(), gm, plan, c.col,
                                              sw_q_.as<float2>(), st, b, hs, 0, qs),
                              "sweep") ||
-                    !cuda_ok(inverse_rows_score(sw_q_.as<float2>(), gm, plan, c.line, c.S, c.tw, cpc,
-                                                sw_n0_.as<double>(), sw_map_.as<float>(), nullptr, nullptr, st, b, qs,
-                                                (size_t)c.nx * c.ny),
+                    !cuda_ok(inverse_rows(sw_q_.as<float2>(), gm, plan, c.line, c.S, c.tw, st, b, qs), "sweep") ||
+                    !cuda_ok(map_scores(sw_q_.as<float2>(), gm, cpc, sw_n0_.as<double>(), sw_map_.as<float>(), nullptr,
+                                        nullptr, st, b, qs, (size_t)c.nx * c.ny),
                              "sweep") ||
                     !cuda_ok(sweep_peaks(sw_map_.as<float>(), c.nx, c.ny, (size_t)c.nx * c.ny, b, n_peak, c0,
                                          sw_ps_.as<float>(), sw_pi_.as<uint32_t>(), st),
                              "sweep"))
                     return -1;
-                launches += 6;
+                launches += 7;
             }
         }
         if (!cev.empty()) cudaEventRecord(cev.back(), st);

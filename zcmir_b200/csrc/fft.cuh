@@ -300,25 +300,137 @@ struct Mix {
     static constexpr int radix(int s) { return mix_radix(N, s); }
 };
 
-// One stage of a compile-time line; OFF: this stage's twiddle table (stage_tw_off).
-template <int R, int NS, int N, int TL, bool INV, int OFF>
+// Several consecutive stages run in registers as one pass through shared memory: the stages
+// S .. S + CNT − 1 of radices R_S, …, product P, take the P points j + t·N/P of group j and leave
+// the P outputs of the last of them, NS apart (the same butterflies, twiddles and rounding as
+// stage by stage, with CNT − 1 fewer exchanges and barriers). Lines with factors of 3 need it:
+// 1458 = 2·3⁶ is 7 stages but 3 passes (18 · 9 · 9). P ≤ 18 keeps a thread's points and twiddles
+// within the 64 registers that two 512-thread blocks per SM leave. A 1296 × 1536 map's passes
+// against the runtime plan: inverse columns 801 → 386 µs, forward rows 584 → 121, forward columns
+// 538 → 152.
+constexpr int kGroupMax = 18;
+__host__ __device__ constexpr int radix_prod(int n, int s, int cnt) {
+    int p = 1;
+    for (int i = 0; i < cnt; ++i) p *= mix_radix(n, s + i);
+    return p;
+}
+// the split of stages s.. into groups: the fewest groups, then the most even products
+__host__ __device__ constexpr int group_cost(int n, int s) {
+    if (s >= mix_stages(n)) return 0;
+    int best = 1 << 30;
+    for (int c = 1; s + c <= mix_stages(n); ++c) {
+        const int p = radix_prod(n, s, c);
+        if (c > 1 && p > kGroupMax) break;
+        const int v = 100000 + p * p + group_cost(n, s + c);
+        if (v < best) best = v;
+    }
+    return best;
+}
+__host__ __device__ constexpr int group_len(int n, int s) {
+    for (int c = 1; s + c <= mix_stages(n); ++c) {
+        const int p = radix_prod(n, s, c);
+        if (c > 1 && p > kGroupMax) break;
+        if (100000 + p * p + group_cost(n, s + c) == group_cost(n, s)) return c;
+    }
+    return 1;
+}
+// Threads per line: as many as leave every thread at most 18 points of each pass (N/16 for a power
+// of two), and no more than a block's 512.
+__host__ __device__ constexpr int line_tl(int n) {
+    int tl = 1;
+    for (int s = 0; s < mix_stages(n); s += group_len(n, s)) {
+        const int p = radix_prod(n, s, group_len(n, s)), per = kGroupMax / p, t = (n / p + per - 1) / per;
+        if (t > tl) tl = t;
+    }
+    return tl < 512 ? tl : 512;
+}
+
+// Stages S .. S + CNT − 1 on the P points v of group k (k = j mod NS), in registers. LO: the
+// points v[t], t ≥ P/2, are zero (the line's upper half; only for an even first radix).
+template <int N, int S, int CNT, int NS, bool INV, bool LO, int P>
+__device__ __forceinline__ void group_apply(float2 (&v)[P], const float2* __restrict__ tw, int k) {
+    static_assert(P == radix_prod(N, S, CNT), "points of the group");
+    if constexpr (CNT == 1) {
+        if constexpr (NS > 1) {
+#pragma unroll
+            for (int r = 1; r < P; ++r) {
+                float2 w = __ldg(&tw[N + stage_tw_off(N, S) + (r - 1) * NS + k]);
+                if (INV) w.y = -w.y;
+                v[r] = cmul(v[r], w);
+            }
+        }
+        if constexpr (LO && P % 2 == 0) dft_lo<P, INV>(v);
+        else dft<P, INV>(v);
+    } else {
+        constexpr int RL = mix_radix(N, S + CNT - 1), PP = P / RL, NSL = NS * PP;
+        float2 y[RL][PP];
+#pragma unroll
+        for (int l = 0; l < RL; ++l) {
+            float2 q[PP];
+#pragma unroll
+            for (int p = 0; p < PP; ++p) q[p] = v[l + RL * p];
+            group_apply<N, S, CNT - 1, NS, INV, LO, PP>(q, tw, k);
+#pragma unroll
+            for (int p = 0; p < PP; ++p) y[l][p] = q[p];
+        }
+#pragma unroll
+        for (int u = 0; u < PP; ++u) {
+            float2 z[RL];
+            z[0] = y[0][u];
+#pragma unroll
+            for (int l = 1; l < RL; ++l) {
+                z[l] = y[l][u];
+                if (NS > 1 || u > 0) {  // else the twiddle is 1
+                    float2 w = __ldg(&tw[N + stage_tw_off(N, S + CNT - 1) + (l - 1) * NSL + k + NS * u]);
+                    if (INV) w.y = -w.y;
+                    z[l] = cmul(z[l], w);
+                }
+            }
+            dft<RL, INV>(z);
+#pragma unroll
+            for (int l = 0; l < RL; ++l) v[u + PP * l] = z[l];
+        }
+    }
+}
+
+// The P points of group j, N/P apart, from the line buffer.
+template <int P, int N>
+__device__ __forceinline__ void group_load(float2 (&v)[P], const float2* __restrict__ buf, int j) {
+    constexpr int M = N / P;
+    if constexpr (M % 16 == 0) {
+        const int p = pad_idx(j);
+#pragma unroll
+        for (int r = 0; r < P; ++r) v[r] = buf[pad_at<M>(p, r)];
+    } else {
+#pragma unroll
+        for (int r = 0; r < P; ++r) v[r] = buf[pad_idx(j + r * M)];
+    }
+}
+// The P outputs of group j to the line buffer, NS apart from (j − k)·P + k.
+template <int P, int NS>
+__device__ __forceinline__ void group_store(const float2 (&v)[P], float2* __restrict__ buf, int j, int k) {
+    const int base = (j - k) * P + k;
+    // outputs NS apart; when P·NS divides 16 they lie in one aligned group of 16 (k < NS)
+    if constexpr (NS % 16 == 0 || 16 % (P * NS) == 0) {
+        const int p = pad_idx(base);
+#pragma unroll
+        for (int r = 0; r < P; ++r) buf[pad_at<NS, (NS % 16 != 0)>(p, r)] = v[r];
+    } else {
+#pragma unroll
+        for (int r = 0; r < P; ++r) buf[pad_idx(base + r * NS)] = v[r];
+    }
+}
+
+// One pass of a compile-time line through its buffer: the stages from S that share it.
+template <int N, int TL, bool INV, int S, int NS>
 __device__ __forceinline__ void mix_stage(float2* __restrict__ buf, const float2* __restrict__ tw, int t, bool act) {
-    constexpr int M = N / R, BM = (M + TL - 1) / TL;
-    float2 v[BM][R];
+    constexpr int CNT = group_len(N, S), P = radix_prod(N, S, CNT), M = N / P, BM = (M + TL - 1) / TL;
+    float2 v[BM][P];
     if (act) {
 #pragma unroll
         for (int b = 0; b < BM; ++b) {
             const int j = t + b * TL;
-            if (M % TL == 0 || j < M) {
-                if constexpr (M % 16 == 0) {
-                    const int p = pad_idx(j);
-#pragma unroll
-                    for (int r = 0; r < R; ++r) v[b][r] = buf[pad_at<M>(p, r)];
-                } else {
-#pragma unroll
-                    for (int r = 0; r < R; ++r) v[b][r] = buf[pad_idx(j + r * M)];
-                }
-            }
+            if (M % TL == 0 || j < M) group_load<P, N>(v[b], buf, j);
         }
     }
     __syncthreads();
@@ -328,185 +440,107 @@ __device__ __forceinline__ void mix_stage(float2* __restrict__ buf, const float2
             const int j = t + b * TL;
             if (M % TL == 0 || j < M) {
                 const int k = j % NS;
-                if (NS > 1) {
-#pragma unroll
-                    for (int r = 1; r < R; ++r) {
-                        float2 w = __ldg(&tw[N + OFF + (r - 1) * NS + k]);
-                        if (INV) w.y = -w.y;
-                        v[b][r] = cmul(v[b][r], w);
-                    }
-                }
-                dft<R, INV>(v[b]);
-                const int base = (j - k) * R + k;
-                // a butterfly's outputs are R points NS apart from base; when R·NS divides 16
-                // they lie in one aligned group of 16 (base mod R·NS = k < NS)
-                if constexpr (NS % 16 == 0 || 16 % (R * NS) == 0) {
-                    const int p = pad_idx(base);
-#pragma unroll
-                    for (int r = 0; r < R; ++r) buf[pad_at<NS, (NS % 16 != 0)>(p, r)] = v[b][r];
-                } else {
-#pragma unroll
-                    for (int r = 0; r < R; ++r) buf[pad_idx(base + r * NS)] = v[b][r];
-                }
+                group_apply<N, S, CNT, NS, INV, false, P>(v[b], tw, k);
+                group_store<P, NS>(v[b], buf, j, k);
             }
         }
     }
     __syncthreads();
 }
 
-template <int N, int TL, bool INV, int S = 0, int NS = 1>
-__device__ __forceinline__ void mix_fft(float2* __restrict__ buf, const float2* __restrict__ tw, int t, bool act) {
-    if constexpr (S < Mix<N>::kStages) {
-        constexpr int R = Mix<N>::radix(S);
-        mix_stage<R, NS, N, TL, INV, stage_tw_off(N, S)>(buf, tw, t, act);
-        mix_fft<N, TL, INV, S + 1, NS * R>(buf, tw, t, act);
+// the passes from stage S to the end (LAST) or up to the last one
+template <int N, int TL, bool INV, int S, int NS, bool LAST>
+__device__ __forceinline__ void mix_run(float2* __restrict__ buf, const float2* __restrict__ tw, int t, bool act) {
+    if constexpr (S < Mix<N>::kStages && (LAST || S + group_len(N, S) < Mix<N>::kStages)) {
+        constexpr int CNT = group_len(N, S), P = radix_prod(N, S, CNT);
+        mix_stage<N, TL, INV, S, NS>(buf, tw, t, act);
+        mix_run<N, TL, INV, S + CNT, NS * P, LAST>(buf, tw, t, act);
     }
 }
 
-// The stages after the first and before the last (S = 1 .. kStages − 2), through shared memory.
-template <int N, int TL, bool INV, int S, int NS>
-__device__ __forceinline__ void mix_mid(float2* __restrict__ buf, const float2* __restrict__ tw, int t, bool act) {
-    if constexpr (S < Mix<N>::kStages - 1) {
-        constexpr int R = Mix<N>::radix(S);
-        mix_stage<R, NS, N, TL, INV, stage_tw_off(N, S)>(buf, tw, t, act);
-        mix_mid<N, TL, INV, S + 1, NS * R>(buf, tw, t, act);
-    }
+// the first stage of the last group
+__host__ __device__ constexpr int last_group(int n) {
+    int s = 0;
+    while (s + group_len(n, s) < mix_stages(n)) s += group_len(n, s);
+    return s;
 }
 
-// the last stage of a compile-time line, its outputs to out(y, v)
+// the last pass of a compile-time line, its outputs to out(y, v)
 template <int N, int TL, bool INV, class Out>
 __device__ __forceinline__ void mix_last(float2* __restrict__ buf, const float2* __restrict__ tw, int t, bool act,
                                          Out&& out) {
-    using MX = Mix<N>;
-    constexpr int RL = MX::radix(MX::kStages - 1), NSL = N / RL, ML = N / RL, BML = (ML + TL - 1) / TL;
+    constexpr int S = last_group(N), CNT = group_len(N, S), P = radix_prod(N, S, CNT), M = N / P, BM = (M + TL - 1) / TL;
     if (act) {
 #pragma unroll 1
-        for (int b = 0; b < BML; ++b) {
+        for (int b = 0; b < BM; ++b) {
             const int j = t + b * TL;
-            if (ML % TL == 0 || j < ML) {
-                float2 v[RL];
-                if constexpr (ML % 16 == 0) {
-                    const int p = pad_idx(j);
+            if (M % TL == 0 || j < M) {
+                float2 v[P];
+                group_load<P, N>(v, buf, j);
+                group_apply<N, S, CNT, M, INV, false, P>(v, tw, j);  // k = j mod M = j
 #pragma unroll
-                    for (int r = 0; r < RL; ++r) v[r] = buf[pad_at<ML>(p, r)];
-                } else {
-#pragma unroll
-                    for (int r = 0; r < RL; ++r) v[r] = buf[pad_idx(j + r * ML)];
-                }
-                // k = j mod NSL = j
-                constexpr int OFFL = stage_tw_off(N, MX::kStages - 1);
-#pragma unroll
-                for (int r = 1; r < RL; ++r) {
-                    float2 w = __ldg(&tw[N + OFFL + (r - 1) * NSL + j]);
-                    if (INV) w.y = -w.y;
-                    v[r] = cmul(v[r], w);
-                }
-                dft<RL, INV>(v);
-#pragma unroll
-                for (int r = 0; r < RL; ++r) out(j + r * NSL, v[r]);
+                for (int r = 0; r < P; ++r) out(j + r * M, v[r]);
             }
         }
     }
 }
 
-// The first stage's butterfly j from in(y), y = j + r·M0: all R0 points, or with LO (the line's
-// points y ≥ N/2 are zero, R0 even) only the lower R0/2, and the transformed points left in v.
-template <int R0, int M0, bool INV, bool LO, class In>
-__device__ __forceinline__ void first_in(float2 (&v)[R0], int j, In& in) {
-    if constexpr (LO && R0 % 2 == 0) {
+// The first pass's groups, their points from in(y), y = j + t·N/P (with LO and an even first
+// radix only the lower half is read), their outputs to the line buffer.
+template <int N, int TL, bool INV, bool LO, class In>
+__device__ __forceinline__ void mix_first(float2* __restrict__ buf, const float2* __restrict__ tw, int t, bool act, In& in) {
+    constexpr int CNT = group_len(N, 0), P = radix_prod(N, 0, CNT), M = N / P, BM = (M + TL - 1) / TL;
+    constexpr bool HALF = LO && mix_radix(N, 0) % 2 == 0;
+    if (act) {
 #pragma unroll
-        for (int r = 0; r < R0 / 2; ++r) v[r] = in(j + r * M0);
-        dft_lo<R0, INV>(v);
-    } else {
+        for (int b = 0; b < BM; ++b) {
+            const int j = t + b * TL;
+            if (M % TL == 0 || j < M) {
+                float2 v[P];
 #pragma unroll
-        for (int r = 0; r < R0; ++r) v[r] = in(j + r * M0);
-        dft<R0, INV>(v);
+                for (int r = 0; r < P; ++r) v[r] = HALF && r >= P / 2 ? make_float2(0.f, 0.f) : in(j + r * M);
+                group_apply<N, 0, CNT, 1, INV, HALF, P>(v, tw, 0);
+                group_store<P, 1>(v, buf, j, 0);
+            }
+        }
     }
 }
 
-// The whole line with its ends in registers: the first stage's butterflies take their inputs
-// straight from in(y) (point y of the line, typically a global load) and the last stage hands
-// its outputs to out(y, v), so the line is staged into and out of shared memory by neither the
-// caller nor this function (two shared-memory passes fewer than run()). Every thread of the
-// block calls it; buf is this thread's line buffer (padded_len(N) points). On return the
-// buffer may still be read by other threads of the line: synchronise before reusing it.
+// The whole line with its ends in registers: the first pass's groups take their inputs straight
+// from in(y) (point y of the line, typically a global load) and the last pass hands its outputs
+// to out(y, v), so neither end is staged through shared memory. Every thread of the block calls
+// it; buf is this thread's line buffer (padded_len(N) points). On return the buffer may still be
+// read by other threads of the line: synchronise before reusing it.
 template <int N, int TL, bool INV, bool LO = false, class In, class Out>
 __device__ __forceinline__ void mix_fft_io(float2* __restrict__ buf, const float2* __restrict__ tw, int t, bool act,
                                            In&& in, Out&& out) {
-    using MX = Mix<N>;
-    static_assert(MX::kStages >= 2, "a line of one stage has no middle to run through shared memory");
-    constexpr int R0 = MX::radix(0), M0 = N / R0, BM0 = (M0 + TL - 1) / TL;
-    if (act) {
-#pragma unroll
-        for (int b = 0; b < BM0; ++b) {
-            const int j = t + b * TL;
-            if (M0 % TL == 0 || j < M0) {
-                float2 v[R0];
-                first_in<R0, M0, INV, LO>(v, j, in);
-#pragma unroll
-                for (int r = 0; r < R0; ++r) buf[first_slot<R0>(j, r)] = v[r];
-            }
-        }
-    }
+    constexpr int CNT = group_len(N, 0);
+    static_assert(CNT < Mix<N>::kStages, "a line of one pass has no shared-memory exchange");
+    mix_first<N, TL, INV, LO>(buf, tw, t, act, in);
     __syncthreads();
-    mix_mid<N, TL, INV, 1, R0>(buf, tw, t, act);
+    mix_run<N, TL, INV, CNT, radix_prod(N, 0, CNT), false>(buf, tw, t, act);
     mix_last<N, TL, INV>(buf, tw, t, act, out);
 }
 
-// The whole line with its first stage's inputs already in registers: v = this thread's one
-// butterfly (j = t, so the first stage's butterflies must number exactly TL), then as mix_fft_io,
-// with between() called once the first stage has consumed v. Lets a caller start loading the next
-// line's inputs while this one transforms.
-template <int N, int TL, bool INV, class Out, class Between>
-__device__ __forceinline__ void mix_fft_regs(float2* __restrict__ buf, const float2* __restrict__ tw, int t, bool act,
-                                             float2 (&v)[Mix<N>::radix(0)], Out&& out, Between&& between) {
-    constexpr int R0 = Mix<N>::radix(0);
-    static_assert(N / R0 == TL, "one first-stage butterfly per thread");
-    if (act) {
-        dft<R0, INV>(v);
-#pragma unroll
-        for (int r = 0; r < R0; ++r) buf[first_slot<R0>(t, r)] = v[r];
-    }
-    __syncthreads();
-    between();  // after the first stage: v is consumed, so the caller may refill its source
-    mix_mid<N, TL, INV, 1, R0>(buf, tw, t, act);
-    mix_last<N, TL, INV>(buf, tw, t, act, out);
-}
-
-
-// The whole line with its first stage fed from in(y) (as mix_fft_io) and the result left in buf
+// The whole line with its first pass fed from in(y) (as mix_fft_io) and the result left in buf
 // in natural order, the block synchronised, as run() leaves it.
 template <int N, int TL, bool INV, bool LO = false, class In>
 __device__ __forceinline__ void mix_fft_in(float2* __restrict__ buf, const float2* __restrict__ tw, int t, bool act,
                                            In&& in) {
-    constexpr int R0 = Mix<N>::radix(0), M0 = N / R0, BM0 = (M0 + TL - 1) / TL;
-    if (act) {
-#pragma unroll
-        for (int b = 0; b < BM0; ++b) {
-            const int j = t + b * TL;
-            if (M0 % TL == 0 || j < M0) {
-                float2 v[R0];
-                first_in<R0, M0, INV, LO>(v, j, in);
-#pragma unroll
-                for (int r = 0; r < R0; ++r) buf[first_slot<R0>(j, r)] = v[r];
-            }
-        }
-    }
+    constexpr int CNT = group_len(N, 0);
+    mix_first<N, TL, INV, LO>(buf, tw, t, act, in);
     __syncthreads();
-    mix_fft<N, TL, INV, 1, R0>(buf, tw, t, act);
+    mix_run<N, TL, INV, CNT, radix_prod(N, 0, CNT), true>(buf, tw, t, act);
 }
 
-// Line-FFT policies the map kernels are written against: n(), threads per line, run<INV>(),
+// Line-FFT policies the map kernels are written against: n(), threads per line,
 // run_io<INV, LO>(buf, t, act, in, out) (mix_fft_io's contract) and run_in<INV, LO>(buf, t, act,
 // in); LO: the caller guarantees in(y) = 0 for y ≥ n/2, so a compile-time line reads only y < n/2.
 struct GenericLine {
     LinePlan p;
+    __device__ __forceinline__ const GenericLine& fresh() const { return *this; }
     __host__ __device__ __forceinline__ int n() const { return p.n; }
     __host__ __device__ __forceinline__ int tl() const { return p.tl; }
-    template <bool INV>
-    __device__ __forceinline__ void run(float2* buf, int t, bool act) const {
-        line_fft<INV>(buf, p, act ? t : (1 << 30));
-    }
     // runtime lines stage through shared memory around the transform (LO: no shortcut)
     template <bool INV, bool LO = false, class In, class Out>
     __device__ __forceinline__ void run_io(float2* buf, int t, bool act, In&& in, Out&& out) const {
@@ -528,18 +562,19 @@ struct GenericLine {
     }
 };
 
-// A compile-time line of N = 2^a·3^b points. TPL: threads per line (N/16 by default: one
-// radix-16 butterfly each; N/8 gives every thread 8 points of the loads and stores around the
-// transform, half of them idle in radix-16 stages)
-template <int N, int TPL = N / 16>
+// A compile-time line of N = 2^a·3^b points, TPL threads per line.
+template <int N, int TPL = line_tl(N)>
 struct FixedLine {
     const float2* tw;
+    // the same line with a twiddle pointer the compiler takes for a new one: a loop over lines then
+    // reads its twiddles through L1 each time instead of hoisting dozens of them into spills
+    __device__ __forceinline__ FixedLine fresh() const {
+        FixedLine f = *this;
+        asm volatile("" : "+l"(f.tw));
+        return f;
+    }
     __host__ __device__ __forceinline__ static constexpr int n() { return N; }
     __host__ __device__ __forceinline__ static constexpr int tl() { return TPL; }
-    template <bool INV>
-    __device__ __forceinline__ void run(float2* buf, int t, bool act) const {
-        mix_fft<N, TPL, INV>(buf, tw, t, act && t < TPL);
-    }
     template <bool INV, bool LO = false, class In, class Out>
     __device__ __forceinline__ void run_io(float2* buf, int t, bool act, In&& in, Out&& out) const {
         mix_fft_io<N, TPL, INV, LO>(buf, tw, t, act && t < TPL, in, out);
@@ -549,8 +584,5 @@ struct FixedLine {
         mix_fft_in<N, TPL, INV, LO>(buf, tw, t, act && t < TPL, in);
     }
 };
-
-template <int N, int TPL = N / 16>
-using Pow2Line = FixedLine<N, TPL>;
 
 }  // namespace zc

@@ -386,7 +386,7 @@ cudaError_t launch_tma(const float2* ha, const float2* hb, const MapGeom& g, con
 }  // namespace
 
 bool inverse_columns_tma_supported(const MapGeom& g, int batch) {
-    return batch == 1 && g.nx == g.ny && (g.ny == 1024 || g.ny == 2048) && g.WP % 2 == 0 && encode_fn() != nullptr;
+    return batch == 1 && (g.ny == 1024 || g.ny == 2048) && g.WP % 2 == 0 && encode_fn() != nullptr;
 }
 
 cudaError_t inverse_columns_tma(const float2* ha, const float2* hb, const MapGeom& g, const CorrPlanDev& plan,

@@ -91,31 +91,33 @@ cudaError_t forward_cols_tc(float2* half, float2* scratch, const MapGeom& g, con
                             const LinePlan& col, int pieces, unsigned* fault, cudaStream_t st);
 // products and inverse column FFTs: Q[slot][ny][WP] (b_stride 0: one fixed side for every item).
 // fault (nullable, device memory): 1 is or-ed into it if the TMA-fed pass (1024- and 2048-point
-// square maps, one item) gave up waiting for a copy, 2 if its staging was misaligned; its Q is
-// then not valid. ZCMIR_B200_INV_COLS=pipe selects the register-prefetch pass instead.
+// columns, one item) gave up waiting for a copy, 2 if its staging was misaligned; its Q is then
+// not valid.
 cudaError_t inverse_columns(const float2* half_a, const float2* half_b, const MapGeom& g, const CorrPlanDev& plan,
                             const LinePlan& col, float2* Q, cudaStream_t st, int batch = 1, size_t a_stride = 0,
                             size_t b_stride = 0, size_t q_stride = 0, unsigned* fault = nullptr);
 bool inverse_columns_tma_supported(const MapGeom& g, int batch);
 cudaError_t inverse_columns_tma(const float2* half_a, const float2* half_b, const MapGeom& g, const CorrPlanDev& plan,
                                 const float2* tw, float2* Q, cudaStream_t st, unsigned* fault);
-// inverse row FFTs fused with the per-shift score and the argmax: map (ny × nx f32), best key
-// (u64), zero-lag score (best and zero may be null); n00: one zero-lag overlap per item
-cudaError_t inverse_rows_score(const float2* Q, const MapGeom& g, const CorrPlanDev& plan, const LinePlan& line,
-                               int S, const float2* tw_nx, const CombineParams& cp, const double* n00, float* map,
-                               unsigned long long* best, float* zero, cudaStream_t st, int batch = 1,
-                               size_t q_stride = 0, size_t map_stride = 0);
-// the same pass with the sums in tensor memory: a whole row per block (nx ∈ {512, 1024, 2048})
+// inverse row FFTs in place: every correlation pair's half spectra rows Q[2p], Q[2p + 1] become the
+// two correlations' real rows (nx floats in a row of WP complex). S: the split (row_split); line:
+// the plan of nx / S points; tw_nx: the twiddles of nx points
+cudaError_t inverse_rows(float2* Q, const MapGeom& g, const CorrPlanDev& plan, const LinePlan& line, int S,
+                         const float2* tw_nx, cudaStream_t st, int batch = 1, size_t q_stride = 0);
+// the per-shift score and the argmax from those real rows: map (ny × nx f32), best key (u64),
+// zero-lag score (best and zero may be null); n00: one zero-lag overlap per item. Rows y0 ..
+// y0 + rows − 1 (rows < 0: to the last), so a caller can copy the map out in row chunks while the
+// later rows run
+cudaError_t map_scores(const float2* Q, const MapGeom& g, const CombineParams& cp, const double* n00, float* map,
+                       unsigned long long* best, float* zero, cudaStream_t st, int batch = 1, size_t q_stride = 0,
+                       size_t map_stride = 0, int y0 = 0, int rows = -1);
+// both passes in one with the sums in tensor memory, a whole row per block (nx = 2048)
 bool rows_tmem_supported(int nx, int n_corr);
-// rows y0 .. y0 + rows − 1 of the map (rows < 0: to the last), so a caller can copy the map out
-// in row chunks while the later rows run
 cudaError_t inverse_rows_score_tmem(const float2* Q, const MapGeom& g, const CorrPlanDev& plan, const float2* tw_nx,
                                     const CombineParams& cp, const double* n00, float* map, unsigned long long* best,
                                     float* zero, cudaStream_t st, int y0 = 0, int rows = -1);
-// the split S of the row pass for nx (smallest divisor keeping its shared memory in budget); 0
-// when none fits
+// the split S (1 or 2) of the row pass for rows of nx points of a plan of n_corr correlations
 int row_split(int nx, int n_corr);
-size_t row_pass_smem(int L, int n_corr, int tl);
 
 // ── the rotation × scale sweep (sweep.cu) ──
 // The sweep's G×G canvas of cells: cell (cx, cy) spans dest pixels [ox + cx·cell, …) (1-based).

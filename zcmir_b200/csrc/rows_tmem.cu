@@ -62,25 +62,21 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 
 constexpr int kTmemSlots = 32;
 
-// Lines of N ≥ 1024 run with 128 threads each and their ends in registers (run_io): the first
-// butterflies read the Hermitian row straight from the half spectra, and the last hand each
-// thread the outputs m ≡ t (mod 128) of its line thread t — exactly the TMEM lane that thread's
-// warp reaches — so the sums go from registers to TMEM with no pass through shared memory.
-template <int N>
-constexpr bool rows_io() { return N >= 1024; }
-template <int N>
-constexpr int rows_tl() { return rows_io<N>() ? 128 : N / 8; }
+// Lines run with 128 threads each and their ends in registers (run_io): the first butterflies
+// read the Hermitian row straight from the half spectra, and the last hand each thread the
+// outputs m ≡ t (mod 128) of its line thread t — exactly the TMEM lane that thread's warp reaches —
+// so the sums go from registers to TMEM with no pass through shared memory.
+constexpr int kTl = 128;
 
 template <int N, int NF, bool EXACT, bool CALIB>
 __global__ void __launch_bounds__(512, 1) k_rows_tmem(const float2* __restrict__ Q, size_t pstride, int WP, int n_corr,
                                                       const float2* __restrict__ tw, CombineParams cp,
                                                       const double* __restrict__ n00p, float* __restrict__ map,
                                                       unsigned long long* best, float* zero_out, int y0) {
-    constexpr int TL = rows_tl<N>();           // threads per line
+    constexpr int TL = kTl;                    // threads per line
     constexpr int LINES = 512 / TL;            // lines per round
     constexpr int J = N / 128;                 // cells per TMEM lane
     constexpr int TCOLS = J * kTmemSlots;      // columns allocated (power of two ≥ 32)
-    constexpr int PER = (N / 2) / TL;          // half-row points per thread (4)
     static_assert(TCOLS >= 32 && TCOLS <= 512 && (TCOLS & (TCOLS - 1)) == 0, "TMEM columns");
     extern __shared__ float2 smem[];
     __shared__ uint32_t tbase_sh;
@@ -103,9 +99,9 @@ __global__ void __launch_bounds__(512, 1) k_rows_tmem(const float2* __restrict__
     const int line = threadIdx.x / TL, t = threadIdx.x - line * TL;
     float2* buf = lines + line * PL;
     const int npairs = (n_corr + 1) / 2;
-    const Pow2Line<N, TL> fft{tw};
+    const FixedLine<N, TL> fft{tw};
 
-    if constexpr (rows_io<N>()) {
+    {
         static_assert(N / Mix<N>::radix(Mix<N>::kStages - 1) % 128 == 0, "last-stage outputs must fall in lane t");
         const int n_tm = n_corr < kTmemSlots ? n_corr : kTmemSlots;
         for (int p0 = 0; p0 < npairs; p0 += LINES) {
@@ -142,70 +138,6 @@ __global__ void __launch_bounds__(512, 1) k_rows_tmem(const float2* __restrict__
             }
             __syncthreads();  // the line buffers are refilled next round
         }
-    } else {
-
-    float2 pa[PER], pb[PER], na = make_float2(0.f, 0.f), nb = make_float2(0.f, 0.f);
-    auto fetch = [&](int pr) {
-        const int k1 = 2 * pr, k2 = 2 * pr + 1;
-        const float2* q1 = Q + (size_t)k1 * pstride + (size_t)y * WP;
-        const float2* q2 = Q + (size_t)(k2 < n_corr ? k2 : k1) * pstride + (size_t)y * WP;
-        const bool h2 = k2 < n_corr;
-#pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            pa[i] = __ldg(&q1[t + TL * i]);
-            pb[i] = h2 ? __ldg(&q2[t + TL * i]) : make_float2(0.f, 0.f);
-        }
-        if (t == 0) {
-            na = __ldg(&q1[N / 2]);
-            nb = h2 ? __ldg(&q2[N / 2]) : make_float2(0.f, 0.f);
-        }
-    };
-    if (line < npairs) fetch(line);
-
-    for (int p0 = 0; p0 < npairs; p0 += LINES) {
-        const int pr = p0 + line;
-        const bool act = pr < npairs;
-        if (act) {
-#pragma unroll
-            for (int i = 0; i < PER; ++i) {
-                const int ix = t + TL * i;
-                const float2 a = pa[i], b = pb[i];
-                buf[pad_idx(ix)] = make_float2(a.x - b.y, a.y + b.x);
-                if (ix > 0) buf[pad_idx(N - ix)] = make_float2(a.x + b.y, b.x - a.y);
-            }
-            if (t == 0) buf[pad_idx(N / 2)] = make_float2(na.x - nb.y, na.y + nb.x);
-            if (pr + LINES < npairs) fetch(pr + LINES);  // next round's rows, in flight during the FFT
-        }
-        __syncthreads();
-        fft.template run<true>(buf, t, act);
-        // scatter the round's sums: TMEM slots by whole warps, the rest to shared memory
-#pragma unroll 1
-        for (int l = 0; l < LINES; ++l) {
-            const int prl = p0 + l;
-            if (prl >= npairs) break;
-            const float2* bl = lines + l * PL;
-#pragma unroll
-            for (int comp = 0; comp < 2; ++comp) {
-                const int slot = 2 * prl + comp;
-                if (slot >= n_corr) break;
-                if (slot < kTmemSlots) {
-#pragma unroll
-                    for (int j = grp; j < J; j += 4) {
-                        const int m = 32 * (w & 3) + lane + 128 * j;
-                        const float2 z = bl[pad_idx(m)];
-                        tmem_st1(tq + (uint32_t)(j * kTmemSlots + slot), comp ? z.y : z.x);
-                    }
-                } else {
-                    float* dst = cs + (size_t)(slot - kTmemSlots) * N;
-                    for (int m = threadIdx.x; m < N; m += 512) {
-                        const float2 z = bl[pad_idx(m)];
-                        dst[m] = comp ? z.y : z.x;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
     }
     tmem_wait_st();
     tc_fence_before();
@@ -249,7 +181,7 @@ template <int N, int NF, bool EXACT, bool CALIB>
 cudaError_t launch_tmem(const float2* Q, const MapGeom& g, int n_corr, const float2* tw, const CombineParams& cp,
                         const double* n00, float* map, unsigned long long* best, float* zero, cudaStream_t st, int y0,
                         int rows) {
-    constexpr int TL = rows_tl<N>(), LINES = 512 / TL;
+    constexpr int TL = kTl, LINES = 512 / TL;
     const int extra = n_corr > kTmemSlots ? n_corr - kTmemSlots : 0;
     const size_t sm = (size_t)LINES * padded_len(N) * sizeof(float2) + (size_t)extra * N * sizeof(float);
     auto k = k_rows_tmem<N, NF, EXACT, CALIB>;
@@ -274,19 +206,17 @@ cudaError_t dispatch_tmem(const float2* Q, const MapGeom& g, int n_corr, const f
 
 }  // namespace
 
-bool rows_tmem_supported(int nx, int n_corr) { return (nx == 512 || nx == 1024 || nx == 2048) && n_corr <= 45; }
+// 2048-point rows: the fused pass takes 0.48 ms for the 45 correlations of a 2048² map, the rows pass
+// and the score pass 0.39 + 0.24 ms. At 1024 points they are level (0.120 against 0.085 + 0.039 ms),
+// at 512 the two passes are ahead (0.053 against 0.024 + 0.015 ms).
+bool rows_tmem_supported(int nx, int n_corr) { return nx == 2048 && n_corr <= 45; }
 
 cudaError_t inverse_rows_score_tmem(const float2* Q, const MapGeom& g, const CorrPlanDev& plan, const float2* tw_nx,
                                     const CombineParams& cp, const double* n00, float* map, unsigned long long* best,
                                     float* zero, cudaStream_t st, int y0, int rows) {
     if (rows < 0) rows = g.ny - y0;
-    if (y0 < 0 || rows <= 0 || y0 + rows > g.ny) return cudaErrorInvalidValue;
-    switch (g.nx) {
-        case 512: return dispatch_tmem<512>(Q, g, plan.n_corr, tw_nx, cp, n00, map, best, zero, st, y0, rows);
-        case 1024: return dispatch_tmem<1024>(Q, g, plan.n_corr, tw_nx, cp, n00, map, best, zero, st, y0, rows);
-        case 2048: return dispatch_tmem<2048>(Q, g, plan.n_corr, tw_nx, cp, n00, map, best, zero, st, y0, rows);
-        default: return cudaErrorNotSupported;
-    }
+    if (g.nx != 2048 || y0 < 0 || rows <= 0 || y0 + rows > g.ny) return cudaErrorInvalidValue;
+    return dispatch_tmem<2048>(Q, g, plan.n_corr, tw_nx, cp, n00, map, best, zero, st, y0, rows);
 }
 
 }  // namespace zc

@@ -9,13 +9,8 @@
 //      5 stack values, two per complex row, row-FFT'd (rows < ch only), unpacked into P half
 //      spectra (columns 0..nx/2), then column-FFT'd (rows ≥ ch are zero).
 //   3. inverse_columns: per correlation and column tile, A·conj(B) and the inverse column FFT.
-//   4. inverse_rows_score: per row, correlations paired as c1 + i·c2 on the Hermitian full row,
-//      inverse row FFT, and the per-shift score in float64 with its argmax, without writing a
-//      correlation plane to memory. Rows longer than shared memory holds for all C correlations
-//      are split S ways by one decimation-in-frequency step (output shifts x ≡ s mod S).
-#include <cstdlib>
-#include <string>
-
+//   4. inverse_rows: per row, correlations paired as c1 + i·c2 on the Hermitian full row, inverse
+//      row FFT, in place; then map_scores (score.cu): the per-shift score in float64 and its argmax.
 #include "passes.cuh"
 
 namespace zc {
@@ -165,19 +160,10 @@ namespace {
 // the runtime mixed-radix plan otherwise.
 cudaError_t dispatch_pass(Pass p, const LinePlan& L, const PassArgs& a, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
-    if (pass_lines_a(p, L, a, st, &e) || pass_lines_b(p, L, a, st, &e) || pass_lines_c(p, L, a, st, &e)) return e;
-    switch (L.n) {
-        case 1024: return run_fixed<1024, true>(p, L.tw, a, st);
-        case 2048: return run_fixed<2048, true>(p, L.tw, a, st);
-        default: break;
-    }
-    const GenericLine f{L};
-    switch (p) {
-        case Pass::FwdRows: return run_pass<Pass::FwdRows, GenericLine, true>(f, a, st);
-        case Pass::FwdCols: return run_pass<Pass::FwdCols, GenericLine, true>(f, a, st);
-        case Pass::InvCols: return run_pass<Pass::InvCols, GenericLine, true>(f, a, st);
-        default: return run_pass<Pass::Rows, GenericLine, true>(f, a, st);
-    }
+    for (auto unit : {pass_lines_0, pass_lines_1, pass_lines_2, pass_lines_3, pass_lines_4, pass_lines_5, pass_lines_6,
+                      pass_lines_7})
+        if (unit(p, L, a, st, &e)) return e;
+    return run_pass(p, GenericLine{L}, a, st);
 }
 
 PassArgs pass_args(const MapGeom& g, const CorrPlanDev& plan, int batch) {
@@ -211,17 +197,13 @@ cudaError_t forward_cols_generic(float2* half, const MapGeom& g, const CorrPlanD
                                  cudaStream_t st) {
     PassArgs a = pass_args(g, plan, 1);
     a.half = half;
-    return run_pass<Pass::FwdCols, GenericLine, true>(GenericLine{col}, a, st);
+    return run_pass(Pass::FwdCols, GenericLine{col}, a, st);
 }
 
 cudaError_t inverse_columns(const float2* ha, const float2* hb, const MapGeom& g, const CorrPlanDev& plan,
                             const LinePlan& col, float2* Q, cudaStream_t st, int batch, size_t a_stride,
                             size_t b_stride, size_t q_stride, unsigned* fault) {
-    static const bool pipe = [] {
-        const char* v = getenv("ZCMIR_B200_INV_COLS");
-        return v && std::string(v) == "pipe";
-    }();
-    if (!pipe && col.n == g.ny && inverse_columns_tma_supported(g, batch))
+    if (col.n == g.ny && inverse_columns_tma_supported(g, batch))
         return inverse_columns_tma(ha, hb, g, plan, col.tw, Q, st, fault);
     PassArgs a = pass_args(g, plan, batch);
     a.half = const_cast<float2*>(ha);
@@ -233,38 +215,20 @@ cudaError_t inverse_columns(const float2* ha, const float2* hb, const MapGeom& g
     return dispatch_pass(Pass::InvCols, col, a, st);
 }
 
-size_t row_pass_smem(int L, int n_corr, int tl) {
-    return (size_t)split_lines(tl) * padded_len(L) * sizeof(float2) + (size_t)n_corr * L * sizeof(float);
-}
-
+// Rows of 972 to 1944 points (but 1024) of plans whose row of sums is large are split in two. The
+// transform takes the same time either way; the split keeps the rounding of the sums, and with it
+// which shifts sit on the overlap floor, that these rows have always had.
 int row_split(int nx, int n_corr) {
-    for (int S = 1; S <= 64; ++S) {
-        if (nx % S) continue;
-        const int L = nx / S;
-        if (L > kMaxLine) continue;
-        const int tl = row_tl(L);
-        if (tl > 512) continue;
-        const size_t sm = S == 1 ? multi_row_smem(L, n_corr, tl, 1) : row_pass_smem(L, n_corr, tl);
-        if (sm <= kRowSmem) return S;
-    }
-    return 0;
+    return nx % 2 == 0 && nx != 1024 && nx < 2048 && n_corr * nx > 40000 ? 2 : 1;
 }
 
-cudaError_t inverse_rows_score(const float2* Q, const MapGeom& g, const CorrPlanDev& plan, const LinePlan& line,
-                               int S, const float2* tw_nx, const CombineParams& cp, const double* n00, float* map,
-                               unsigned long long* best, float* zero, cudaStream_t st, int batch, size_t q_stride,
-                               size_t map_stride) {
+cudaError_t inverse_rows(float2* Q, const MapGeom& g, const CorrPlanDev& plan, const LinePlan& line, int S,
+                         const float2* tw_nx, cudaStream_t st, int batch, size_t q_stride) {
     PassArgs a = pass_args(g, plan, batch);
-    a.Q = const_cast<float2*>(Q);
+    a.Q = Q;
     a.q_stride = q_stride;
     a.S = S;
     a.tw_nx = tw_nx;
-    a.cp = &cp;
-    a.n00 = n00;
-    a.map = map;
-    a.map_stride = map_stride;
-    a.best = best;
-    a.zero = zero;
     return dispatch_pass(Pass::Rows, line, a, st);
 }
 
