@@ -129,15 +129,18 @@ class Clocks:
 
 def stage_bytes(p):
     """Algorithmic bytes of each stage of one map (one launch of that kernel per side where it
-    runs per side): its compulsory reads and writes in this decomposition."""
+    runs per side): its compulsory reads and writes in this decomposition. P: the planes both sides
+    transform; the canvas stage also reads the samples twice and writes the moment tables (64 bytes
+    a cell) of the sides whose moments are not transformed."""
     nx, ny, cw, ch, P, C = p["nx"], p["ny"], p["cw"], p["ch"], p["n_real"], p["n_corr"]
     half = (nx // 2 + 1) * 8
+    tables = {18: 2, 11: 2, 32: 1, 20: 1}.get(C, 0)
     return {
-        "canvas": 2 * (5 * p["canvas_w"] * p["canvas_h"] * 4) * 2,
-        "fwd_rows": 2 * (5 * cw * ch * 4 + P * ch * half),
-        "fwd_cols": 2 * (P * ch * half + P * ny * half),
-        "inv_cols": 2 * P * ny * half + C * ny * half,
-        "inv_rows_score": C * ny * half + nx * ny * 4,
+        "canvas": 2 * (5 * p["canvas_w"] * p["canvas_h"] * 4) * 2 + tables * cw * ch * (2 * 20 + 64),
+        "fwd_rows": 2 * 5 * cw * ch * 4 + P * ch * half,
+        "fwd_cols": P * ch * half + P * ny * half,
+        "inv_cols": P * ny * half + C * ny * half,
+        "inv_rows_score": C * ny * half + tables * cw * ch * 64 + nx * ny * 4,
     }
 
 
@@ -198,17 +201,18 @@ def sweep_work(tuned, Fx, Fy):
 
 
 def survey_bytes(p):
-    """The whole map's compulsory HBM bytes (both stacks read, both sides' half spectra written and
-    read once, the map written)."""
-    nx, ny, P = p["nx"], p["ny"], p["n_real"]
+    """The whole map's compulsory HBM bytes (both stacks read, both sides' half spectra of all 15
+    planes written and read once, the map written)."""
+    nx, ny, P = p["nx"], p["ny"], 15
     return 2 * 5 * p["canvas_w"] * p["canvas_h"] * 4 + 2 * (2 * P * nx * (ny // 2 + 1) * 8) + nx * ny * 4
 
 
 def survey_flops(p):
     """The whole map's FP32 flops by the survey's counting rule: both sides' forward FFTs over the
     canvas rows and all columns (packed complex lines), the inverse 2-D FFTs of the packed
-    correlations, the conjugate products and about 300 flops of scoring per shift."""
-    nx, ny, ch, P, C = p["nx"], p["ny"], p["ch"], p["n_real"], p["n_corr"]
+    correlations, the conjugate products and about 300 flops of scoring per shift. The rule counts the
+    method's 15 planes and 45 correlations, of which a map transforms those in its plan."""
+    nx, ny, ch, P, C = p["nx"], p["ny"], p["ch"], 15, 45
     lx, ly = np.log2(nx), np.log2(ny)
     fwd = 2 * ((P + 1) // 2) * 5 * (nx * lx * ch + ny * ly * nx)
     inv = ((C + 1) // 2) * 5 * nx * ny * np.log2(nx * ny)

@@ -15,8 +15,8 @@ extern "C" {
  * (CUDA events around replays of one CUDA graph of the map's passes; the instrumented maps' time
  * when the graph cannot be captured), [1..5] per-stage ms of event-instrumented maps (canvas,
  * forward rows, forward columns, inverse columns, inverse rows + score), [6] ms per instrumented
- * map, [7] canvas height, [8..15] nx, ny, cw, ch, real planes, correlations, row split, canvas
- * width. 0 / -1 with zc_error. */
+ * map, [7] canvas height, [8..15] nx, ny, cw, ch, real planes transformed (both sides),
+ * correlations transformed (the others' sums come from moment tables), row split, canvas width. 0 / -1 with zc_error. */
 int32_t zcb_bench_maps(zc_engine* e, const double H[9], uint32_t flags, uint32_t cap, uint32_t warmup, uint32_t steps,
                        double* out, size_t out_len);
 

@@ -2,6 +2,7 @@
 // shaders/smi.wgsl:825-915), shared by the row-pass kernels.
 #pragma once
 
+#include "box.cuh"
 #include "kernels.hpp"
 
 namespace zc {
@@ -18,14 +19,58 @@ __host__ __device__ constexpr bool fourth_plane(int p) { return p == 4 || p == 8
 __host__ __device__ constexpr bool corr_kept(int c, bool three) {
     return !three || (!fourth_plane(corr_a(c)) && !fourth_plane(corr_b(c)));
 }
-__host__ __device__ constexpr int corr_slot(int c, bool three) {
-    int s = 0;
-    for (int i = 0; i < c; ++i) s += corr_kept(i, three) ? 1 : 0;
-    return s;
+// Which correlations a map transforms: all of the plan (mode 0); without side A's moments over the
+// fixed image's box (1: A's feature sums but the first and A's products); and without side B's over
+// the moving image's box (2). Correlation 1 stays: it shares correlation 0's transforms.
+__host__ __device__ constexpr bool corr_fft(int c, int mode) {
+    return mode == 0 || !((c >= 2 && c <= 4) || (c >= 25 && c <= 34) || (mode == 2 && ((c >= 5 && c <= 8) || c >= 35)));
+}
+// Where correlation c's sum comes from, for every c: a slot of those kept and transformed (src 0), or
+// a comp of side A's (1) or side B's (2) table, with n added back (diag). Tables rather than functions,
+// so that a use at a compile-time c folds to a constant.
+struct CorrSource {
+    signed char src[45], at[45];
+    bool diag[45];
+};
+template <int NF, int MODE>
+__host__ __device__ constexpr CorrSource corr_source() {
+    CorrSource t{};
+    int slot = 0;
+    for (int c = 0; c < 45; ++c) {
+        t.src[c] = 0, t.at[c] = 0, t.diag[c] = false;
+        if (!corr_kept(c, NF == 3)) continue;
+        if (corr_fft(c, MODE)) {
+            t.at[c] = (signed char)slot++;
+            continue;
+        }
+        t.src[c] = c <= 4 || (c >= 25 && c <= 34) ? 1 : 2;
+        if (c <= 8) {
+            t.at[c] = (signed char)(c <= 4 ? c - 1 : c - 5);
+        } else {
+            const int k = c >= 35 ? c - 35 : c - 25, i = box_i(k, 4), j = box_j(k, 4);
+            t.at[c] = (signed char)box_comp(i, j, NF);
+            t.diag[c] = i == j;
+        }
+    }
+    return t;
+}
+
+// how many slots a map of the given plan transforms (NF = 1: the NCC map's one)
+template <int NF, bool EXACT, int MODE>
+__host__ __device__ constexpr int corr_slots() {
+    if (NF == 1) return 1;
+    int n = 0;
+    for (int c = 0; c < (EXACT ? 45 : 25); ++c) n += corr_kept(c, NF == 3) && corr_fft(c, MODE) ? 1 : 0;
+    return n;
 }
 
 __host__ __device__ constexpr int tri_kc(int i, int j) {
     return (i < j ? i : j) * 4 - ((i < j ? i : j) * ((i < j ? i : j) + 1)) / 2 + (i < j ? j : i);
+}
+
+// the correlation area where it lives in device memory
+__device__ __forceinline__ void read_area(CombineParams& cp) {
+    if (cp.area_dev) cp.area = *cp.area_dev;
 }
 
 // The score's parameters for the shifts of row y of an ny-row map: a log-polar map scales row
@@ -43,33 +88,35 @@ __device__ __forceinline__ double lag0_units(const CombineParams& cp, double n00
     return cp.lp_dlam != 0.0 ? n00 * cp.lp_dlam * cp.lp_dth : n00;
 }
 
+// Whether a shift's overlap n is above the floors (else its score is 0; a NaN overlap is not below).
+template <bool CALIB>
+__device__ __forceinline__ bool overlap_alive(double n, const CombineParams& p, double n00) {
+    const double floor_n = CALIB ? (double)p.min_n : fmax((double)p.min_n, 0.08 * fmax(n00, 0.0));
+    return !(n < floor_n || (CALIB && n / fmax(p.area, 1.0) <= 10.0));
+}
+
 // Per-shift score (smi.wgsl:825-915, combine_cell): centring, ridge, Cholesky factors and the
 // whitened norm in float64, the calibrated map's Wilson–Hilferty transform in float32; every
 // index known at compile time (NF features, exact or global whitening, calibrated or not), so the 4×4 algebra stays in
-// registers. `get(slot)` returns this shift's (unscaled) sum of the plan's slot `slot`; the
-// slots follow the plan (NF = 3 drops the fourth feature's correlations), and every slot passed
-// to it is a compile-time constant. Each Cholesky pivot is inverted once (rsqrt) and the
+// registers. n: this shift's overlap; `mean(c, 1 / n)` returns correlation c's sum over n (of the 45;
+// NF = 3 asks for none of the fourth feature's), and every c passed to it is a compile-time constant. Each Cholesky pivot is inverted once (rsqrt) and the
 // substitutions multiply by it.
 template <int NF, bool EXACT, bool CALIB, class G>
-__device__ __forceinline__ float combine_smi(G&& get, const CombineParams& p, double n00) {
-    constexpr bool THREE = NF == 3;
-    auto S = [&](int c) -> double { return (double)get(corr_slot(c, THREE)) * p.inv_nn; };
-    const double n = S(0);
+__device__ __forceinline__ float combine_smi(G&& mean, double n, const CombineParams& p, double n00) {
     const double neff = n / fmax(p.area, 1.0);
-    double floor_n = fmax((double)p.min_n, 0.08 * fmax(n00, 0.0));
-    if (CALIB) floor_n = (double)p.min_n;
-    if (n < floor_n || (CALIB && neff <= 10.0)) return 0.f;
+    if (!overlap_alive<CALIB>(n, p, n00)) return 0.f;
     const double rn = 1.0 / fmax(n, 1e-8);
+    auto S = [&](int c) -> double { return mean(c, rn); };
     double ma[NF], mb[NF], C[NF][NF];
 #pragma unroll
     for (int i = 0; i < NF; ++i) {
-        ma[i] = S(1 + i) * rn;
-        mb[i] = S(5 + i) * rn;
+        ma[i] = S(1 + i);
+        mb[i] = S(5 + i);
     }
 #pragma unroll
     for (int i = 0; i < NF; ++i)
 #pragma unroll
-        for (int j = 0; j < NF; ++j) C[i][j] = S(9 + 4 * i + j) * rn - ma[i] * mb[j];
+        for (int j = 0; j < NF; ++j) C[i][j] = S(9 + 4 * i + j) - ma[i] * mb[j];
     if (!EXACT) {
         double s = 0.0;
 #pragma unroll
@@ -88,8 +135,8 @@ __device__ __forceinline__ float combine_smi(G&& get, const CombineParams& p, do
     for (int i = 0; i < NF; ++i) {
 #pragma unroll
         for (int j = 0; j <= i; ++j) {
-            A[i][j] = S(25 + tri_kc(i, j)) * rn - ma[i] * ma[j];
-            B[i][j] = S(35 + tri_kc(i, j)) * rn - mb[i] * mb[j];
+            A[i][j] = S(25 + tri_kc(i, j)) - ma[i] * ma[j];
+            B[i][j] = S(35 + tri_kc(i, j)) - mb[i] * mb[j];
         }
         tra += A[i][i];
         trb += B[i][i];
@@ -166,19 +213,27 @@ __device__ __forceinline__ float combine_smi(G&& get, const CombineParams& p, do
 
 // The NCC map's value at a lag (src/overlay.zig:256-258): the mean-free correlation over the
 // product of the planes' norms (den, carried in the n00 slot), clamped to ±1.5.
-template <class G>
-__device__ __forceinline__ float combine_ncc(G&& get, const CombineParams& p, double den) {
-    const double v = (double)get(0) * p.inv_nn / den;
-    return (float)fmin(1.5, fmax(-1.5, v));
+__device__ __forceinline__ float combine_ncc(double sum, double den) {
+    return (float)fmin(1.5, fmax(-1.5, sum / den));
 }
 
-// NF = 1 selects the NCC map, 3 or 4 the SMI score over that many features.
+// A shift whose sums are all transformed ones: raw(c) the unscaled float sum of correlation c. NF = 1
+// selects the NCC map, 3 or 4 the SMI score over that many features.
 template <int NF, bool EXACT, bool CALIB, class G>
-__device__ __forceinline__ float combine_t(G&& get, const CombineParams& p, double n00) {
-    if constexpr (NF == 1)
-        return combine_ncc(get, p, n00);
-    else
-        return combine_smi<NF, EXACT, CALIB>(get, p, n00);
+__device__ __forceinline__ float combine_t(G&& raw, const CombineParams& p, double n00) {
+    const double n = (double)raw(0) * p.inv_nn;
+    if constexpr (NF == 1) {
+        return combine_ncc(n, n00);
+    } else {
+        double scale = 0.0;  // inv_nn / n, once per shift
+        bool have = false;
+        return combine_smi<NF, EXACT, CALIB>(
+            [&](int c, double rn) -> double {
+                if (!have) scale = p.inv_nn * rn, have = true;
+                return (double)raw(c) * scale;
+            },
+            n, p, n00);
+    }
 }
 
 }  // namespace zc

@@ -3,6 +3,8 @@
 // shiftMapOpts 795-819, shiftMap 822-829) and src/smi.zig (prepare 348-400, shiftMapFrom 552-572).
 #include "engine.hpp"
 
+#include "combine.cuh"
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -37,7 +39,7 @@ void DevBuf::release() {
 // The correlation plan (src/smi.zig:90-158): the real planes kept (15 exact, 5 global; without
 // the fourth feature's planes when `three`) and, per correlation slot, its moving and fixed
 // plane slots and its number in the full 45-correlation order.
-CorrPlanDev corr_plan_dev(bool exact, bool three) {
+CorrPlanDev corr_plan_dev(bool exact, bool three, int box_mode) {
     int lst_a[45], lst_b[45], nl = 0;
     lst_a[nl] = 0, lst_b[nl++] = 0;
     for (int i = 0; i < 4; ++i) lst_a[nl] = 1 + i, lst_b[nl++] = 0;
@@ -62,7 +64,7 @@ CorrPlanDev corr_plan_dev(bool exact, bool three) {
     }
     for (int c = 0; c < nl; ++c) {
         const int sa = slot[lst_a[c]], sb = slot[lst_b[c]];
-        if (sa < 0 || sb < 0) continue;
+        if (sa < 0 || sb < 0 || !corr_fft(c, box_mode)) continue;
         P.ca[P.n_corr] = sa;
         P.cb[P.n_corr] = sb;
         P.cnum[P.n_corr] = c;
@@ -108,7 +110,7 @@ Engine::~Engine() {
         cudaStreamDestroy(acf_st_);
     }
     for (DevBuf* b : {&fs_stats_, &fs_hist_, &fs_wt_, &fs_acfpart_, &fs_acf_, &rank_tmp_, &canvas_a_, &canvas_b_,
-                      &grid_a_, &grid_b_, &half_a_, &half_b_, &q_, &map_, &res_, &flush_, &pose_hinv_, &pose_sums_,
+                      &grid_a_, &grid_b_, &half_a_, &half_b_, &box_a_, &box_b_, &box_tmp_, &q_, &map_, &res_, &flush_, &pose_hinv_, &pose_sums_,
                       &pose_coef_, &pose_score_, &pose_tsum_, &pose_gens_, &pose_part_, &pose_ticket_, &dft_scratch_, &sw_il_[0], &sw_il_[1], &sw_poses_,
                       &sw_fgrid_, &sw_fhalf_, &sw_grid_, &sw_half_, &sw_q_, &sw_map_, &sw_n0_, &sw_ps_, &sw_pi_})
         b->release();
@@ -129,6 +131,9 @@ Engine::~Engine() {
     for (auto& kv : tw_) cudaFree(kv.second);
     for (cudaEvent_t e : chunk_ev_)
         if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : aux_ev_)
+        if (e) cudaEventDestroy(e);
+    if (aux_st_) cudaStreamDestroy(aux_st_);
     if (copy_st_) cudaStreamDestroy(copy_st_);
     if (branch_st_) cudaStreamDestroy(branch_st_);
     for (cudaEvent_t e : {fork_ev_, join_ev_})
@@ -282,7 +287,7 @@ bool Engine::build_side(int s) {
               cuda_ok(sd.mag.ensure(n * 4), "features") && cuda_ok(sd.stack.ensure(n * 20), "features") &&
               cuda_ok(rtmp.ensure(n * 4), "features") && cuda_ok(stats.ensure(22 * 8), "features") &&
               cuda_ok(hist.ensure(256 * 4), "features") && cuda_ok(wt.ensure(20 * 4), "features") &&
-              cuda_ok(part.ensure((size_t)ntiles * 1156 * 4), "features") &&
+              cuda_ok(part.ensure((size_t)ntiles * kAcfSums * 4), "features") &&
               cuda_ok(sd.acf_dev.ensure(1156 * 8), "features");
     if (!ok) return false;
     fsc.stats = stats.as<double>();
@@ -462,6 +467,39 @@ bool Engine::line_plan(int n, LinePlan& p) {
 
 // ── shift map ─────────────────────────────────────────────────────────────────────────────────
 
+// Which moments of a map come from summed-area tables: on a grid of whole canvas pixels the fixed
+// image's weight is 1 on its rectangle and 0 elsewhere, always; the moving image's too under a
+// translation, on the pixels whose sample position falls inside it (the canvas kernel's float
+// arithmetic: its products with 1 and 0 and the division by 1 are exact). On coarser grids the edge
+// cells' weights are fractions and every correlation is transformed.
+BoxSums Engine::box_sums(const MapJob& job) const {
+    BoxSums b;
+    const MapGeom& g = job.g;
+    if (!job.exact || !job.identity_grid) return b;
+    const Side &A = side[0], &B = side[1];
+    b.mode = 1;
+    b.cw = g.cw, b.ch = g.ch;
+    b.b = Box{-g.ox, -g.ox + B.w, -g.oy, -g.oy + B.h};
+    const Mat3 hi = inv3_plain(job.Hc);
+    const bool shift = (float)hi[0] == 1.f && (float)hi[1] == 0.f && (float)hi[3] == 0.f && (float)hi[4] == 1.f &&
+                       (float)hi[6] == 0.f && (float)hi[7] == 0.f && (float)hi[8] == 1.f;
+    if (!shift || std::fabs(det3(job.Hc)) < 1e-12) return b;
+    auto span = [](float t, int n, int w, int& lo, int& hi_) {
+        auto in = [&](int x) {
+            const float q = ((float)x + 1.0f) + t, f = q - 1.0f;
+            return !(f < 0.f || f > (float)(w - 1));
+        };
+        lo = 0;
+        while (lo < n && !in(lo)) ++lo;
+        hi_ = lo;
+        while (hi_ < n && in(hi_)) ++hi_;
+    };
+    span((float)hi[2], g.cw, A.w, b.a.x0, b.a.x1);
+    span((float)hi[5], g.ch, A.h, b.a.y0, b.a.y1);
+    b.mode = 2;
+    return b;
+}
+
 bool Engine::plan_map(const Mat3& Hm, bool exact, bool calibrated, unsigned cap, double min_overlap, MapJob& job) {
     // the features only enqueued, side 1's build not yet joined: run_map queues side 0's passes
     // first and joins side 1 before its own; the correlation area the calibrated score needs is
@@ -494,10 +532,15 @@ bool Engine::plan_map(const Mat3& Hm, bool exact, bool calibrated, unsigned cap,
     g.WP = ((g.nx / 2 + 1) + 7) / 8 * 8;
     job.identity_grid = (g.cw == g.W && g.ch == g.Hh);
     const bool three = side[0].mode == 1;
-    job.plan = corr_plan_dev(exact, three);
+    job.box = box_sums(job);
+    job.plan = corr_plan_dev(exact, three, job.box.mode);
     const CorrPlanDev& P = job.plan;
+    // a side whose moments are tabled transforms its samples only, not their products
+    const int n_plain = three ? 4 : 5;
+    job.n_side[0] = job.box.mode >= 1 ? n_plain : P.n_real;
+    job.n_side[1] = job.box.mode == 2 ? n_plain : P.n_real;
     if (!line_plan(g.nx, job.row) || !line_plan(g.ny, job.col)) return false;
-    job.S = row_split(g.nx, P.n_corr);
+    job.S = row_split(g.nx, exact ? (three ? 28 : 45) : P.n_corr);
     if (!line_plan(g.nx / job.S, job.line)) return false;
     const unsigned floor_n = min_overlap > 0 ? (unsigned)std::floor(min_overlap * (double)g.cw * (double)g.ch) : 0u;
     const double gcell = (double)g.W / (double)g.cw;
@@ -506,7 +549,7 @@ bool Engine::plan_map(const Mat3& Hm, bool exact, bool calibrated, unsigned cap,
     cp.calib = job.calibrated ? 1 : 0;
     cp.nf = three ? 3 : 4;
     cp.min_n = (float)std::max(12u, floor_n);
-    cp.area = 0.0;  // set by run_map
+    cp.area = 0.0;  // run_map sets area_dev
     job.gcell = gcell;
     cp.ridge = 1e-4;
     cp.inv_nn = 1.0 / ((double)g.nx * (double)g.ny);
@@ -516,21 +559,26 @@ bool Engine::plan_map(const Mat3& Hm, bool exact, bool calibrated, unsigned cap,
 bool Engine::map_buffers(const MapJob& job) {
     const MapGeom& g = job.g;
     const size_t cn = (size_t)g.W * g.Hh, gn = (size_t)g.cw * g.ch;
-    const size_t hs = (size_t)job.plan.n_real * g.ny * g.WP * sizeof(float2);
+    const size_t hp = (size_t)g.ny * g.WP * sizeof(float2), hs = std::max(job.n_side[0], job.n_side[1]) * hp;
     const size_t qs = (size_t)job.plan.n_corr * g.ny * g.WP * sizeof(float2);
     bool ok = cuda_ok(canvas_a_.ensure(cn * 20), "shift_map") && cuda_ok(canvas_b_.ensure(cn * 20), "shift_map") &&
-              cuda_ok(half_a_.ensure(hs), "shift_map") && cuda_ok(half_b_.ensure(hs), "shift_map") &&
+              cuda_ok(half_a_.ensure(job.n_side[0] * hp), "shift_map") &&
+              cuda_ok(half_b_.ensure(job.plan.n_real * hp), "shift_map") &&  // room for a turned pose's products
               cuda_ok(q_.ensure(qs), "shift_map") && cuda_ok(map_.ensure((size_t)g.nx * g.ny * 4), "shift_map") &&
               cuda_ok(res_.ensure(64), "shift_map");
     if (ok && !job.identity_grid)
         ok = cuda_ok(grid_a_.ensure(gn * 20), "shift_map") && cuda_ok(grid_b_.ensure(gn * 20), "shift_map");
+    const size_t bt = box_table_bytes(job.cp.nf, g.cw, g.ch);
+    if (ok && job.box.mode >= 1)
+        ok = cuda_ok(box_a_.ensure(bt), "shift_map") &&
+             cuda_ok(box_tmp_.ensure(box_scratch_bytes(job.cp.nf, g.cw, g.ch)), "shift_map");
+    if (ok && job.box.mode == 2) ok = cuda_ok(box_b_.ensure(bt), "shift_map");
     if (ok && dft_pieces_) ok = cuda_ok(dft_scratch_.ensure(hs), "dft stage");
     return ok;
 }
 
 bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
     const MapGeom& g = job.g;
-    const size_t hs = (size_t)job.plan.n_real * g.ny * g.WP * sizeof(float2);
     if (!map_buffers(job)) return false;
     auto rec = [&](int i) {
         if (ev) cudaEventRecord(ev[i], st);
@@ -559,39 +607,63 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
         return true;
     };
     unsigned* fault = reinterpret_cast<unsigned*>(res + 24);  // the inverse columns' fault word
-    auto lag0 = [&](const float* ga, const float* gb) {
-        return cuda_ok(lag0_count(ga, gb, g.cw, g.ch, n00, st), "lag0") &&
-               cuda_ok(cudaMemsetAsync(best, 0, 8, st), "shift_map") &&
-               cuda_ok(cudaMemsetAsync(fault, 0, 4, st), "shift_map");
+    // What only the score reads — the zero-lag overlap and the moment tables — is made on a stream of
+    // its own beside the transforms (a 256² map's two tables take 50 µs, mostly launches and short
+    // chains): it waits for the canvases, the score waits for it.
+    if (!aux_st_ && (!cuda_ok(cudaStreamCreateWithPriority(&aux_st_, cudaStreamNonBlocking, std::min(prio_hi_ + 1, prio_lo_)), "shift_map") ||
+                     !cuda_ok(cudaEventCreateWithFlags(&aux_ev_[0], cudaEventDisableTiming), "shift_map") ||
+                     !cuda_ok(cudaEventCreateWithFlags(&aux_ev_[1], cudaEventDisableTiming), "shift_map")))
+        return false;
+    auto aux_after_st = [&] {
+        return cuda_ok(cudaEventRecord(aux_ev_[0], st), "shift_map") &&
+               cuda_ok(cudaStreamWaitEvent(aux_st_, aux_ev_[0], 0), "shift_map");
     };
-    auto rows_of = [&](int s, const float* grid) {
-        return cuda_ok(forward_rows(grid, g, job.plan, job.row, (s == 0 ? half_a_ : half_b_).as<float2>(), st),
-                       "forward rows");
+    auto st_after_aux = [&] {
+        return cuda_ok(cudaEventRecord(aux_ev_[1], aux_st_), "shift_map") &&
+               cuda_ok(cudaStreamWaitEvent(st, aux_ev_[1], 0), "shift_map");
+    };
+    auto lag0 = [&](const float* ga, const float* gb) {
+        return cuda_ok(cudaMemsetAsync(best, 0, 8, st), "shift_map") && cuda_ok(cudaMemsetAsync(fault, 0, 4, st), "shift_map") &&
+               aux_after_st() && cuda_ok(lag0_count(ga, gb, g.cw, g.ch, n00, aux_st_), "lag0");
+    };
+    // a side's planes [p0, p1): the samples' planes and their products in launches of their own when
+    // the side may have been asked for its samples alone, so that a plane's bits do not depend on it
+    auto half_of = [&](int s, int p0) { return (s == 0 ? half_a_ : half_b_).as<float2>() + (size_t)p0 * g.ny * g.WP; };
+    const int n_plain = job.cp.nf + 1;
+    auto rows_of = [&](int s, const float* grid, int p0, int p1) {
+        while (p0 < p1) {
+            const int to = job.box.mode >= 1 && p0 < n_plain ? std::min(p1, n_plain) : p1;
+            if (!cuda_ok(forward_rows(grid, g, job.planes(p0, to), job.row, half_of(s, p0), st), "forward rows")) return false;
+            counts[0] += 1;
+            p0 = to;
+        }
+        return true;
     };
     unsigned* fault_tc = reinterpret_cast<unsigned*>(res + 28);  // the tensor-core stage's fault word
     if (dft_pieces_ && !cuda_ok(cudaMemsetAsync(fault_tc, 0, 4, st), "shift_map")) return false;
-    auto cols_of = [&](int s) {
-        float2* half = (s == 0 ? half_a_ : half_b_).as<float2>();
+    auto cols_of = [&](int s, int p0, int p1) {
+        const CorrPlanDev plan = job.planes(p0, p1);
+        counts[0] += 1;
         if (dft_pieces_) {
             if (job.col.radix[0] != 16 || (g.ny / 16) % 4 != 0)
                 return fail("dft stage: the column length " + std::to_string(g.ny) + " does not start with radix 16");
-            return cuda_ok(dft_scratch_.ensure(hs), "dft stage") &&
-                   cuda_ok(forward_cols_tc(half, dft_scratch_.as<float2>(), g, job.plan, job.col, dft_pieces_, fault_tc,
-                                           st),
+            return cuda_ok(forward_cols_tc(half_of(s, p0), dft_scratch_.as<float2>(), g, plan, job.col, dft_pieces_,
+                                           fault_tc, st),
                            "forward columns (tensor-core stage)");
         }
-        return cuda_ok(forward_cols(half, g, job.plan, job.col, st), "forward columns");
+        return cuda_ok(forward_cols(half_of(s, p0), g, plan, job.col, st), "forward columns");
     };
     // Each side's canvas, grid and half spectra depend on its feature build, the canvas frame and
     // plan, the buffers they live in and, for the moving side, the canvas pose: with the same key
-    // as the last map that built them, they are still in the buffers and are reused.
+    // as the last map that built them, they are still in the buffers and are reused. A map that needs
+    // more of the side's planes, or its moment table, adds what is missing.
     auto side_key = [&](int s) {
         std::vector<uint64_t> k;
         const DevBuf &cv = s == 0 ? canvas_a_ : canvas_b_, &gd = s == 0 ? grid_a_ : grid_b_,
                      &hf = s == 0 ? half_a_ : half_b_;
         for (const DevBuf* b : {&cv, &gd, &hf}) k.push_back((uint64_t)(uintptr_t)b->p), k.push_back(b->gen);
         for (int v : {s, side[s].mode, (int)side[s].half, g.W, g.Hh, g.ox, g.oy, g.cw, g.ch, g.nx, g.ny, g.WP,
-                      (int)job.identity_grid, job.plan.n_real})
+                      (int)job.identity_grid, (int)(job.box.mode >= 1), job.plan.n_real})
             k.push_back((uint64_t)(int64_t)v);
         k.push_back(side[s].ver);
         for (int i = 0; i < job.plan.n_real; ++i) k.push_back((uint64_t)job.plan.planes[i]);
@@ -614,23 +686,44 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
         if (!job.identity_grid) grid = (s == 0 ? grid_a_ : grid_b_).as<float>();
         return true;
     };
-    auto side_canvas = [&](int s, const float*& grid) { return have[s] ? kept_grid(s, grid) : canvas_side(s, grid); };
-    auto side_rows = [&](int s, const float* grid) { return have[s] || rows_of(s, grid); };
-    auto side_cols = [&](int s) {
-        if (have[s]) return true;
-        if (!cols_of(s)) return false;
-        spec_key_[s] = key[s];
+    auto side_canvas = [&](int s, const float*& grid) {
+        if (have[s]) {
+            kept_grid(s, grid);
+        } else {
+            spec_key_[s].clear();  // until this side's passes are queued
+            if (!canvas_side(s, grid)) return false;
+            counts[0] += job.identity_grid ? 1 : 2;
+        }
+        if (job.box.mode <= s) return true;
+        const DevBuf& bt = s == 0 ? box_a_ : box_b_;
+        std::vector<uint64_t> bk = key[s];
+        bk.push_back((uint64_t)(uintptr_t)bt.p), bk.push_back(bt.gen);
+        if (have[s] && bk == box_key_[s]) return true;
+        if (!aux_after_st() ||
+            !cuda_ok(box_table(grid, g.cw, g.ch, job.cp.nf, bt.as<float>(), box_tmp_.p, aux_st_), "moment tables"))
+            return false;
+        counts[0] += 3;
+        box_key_[s] = bk;
         return true;
     };
-    for (int s = 0; s < 2; ++s)
-        if (!have[s]) spec_key_[s].clear();  // until this side's passes are queued
+    auto side_rows = [&](int s, const float* grid) {
+        return rows_of(s, grid, have[s] ? std::min(spec_planes_[s], job.n_side[s]) : 0, job.n_side[s]);
+    };
+    auto side_cols = [&](int s) {
+        const int p0 = have[s] ? spec_planes_[s] : 0;
+        if (p0 >= job.n_side[s]) return true;
+        if (!cols_of(s, p0, job.n_side[s])) return false;
+        spec_key_[s] = key[s];
+        spec_planes_[s] = job.n_side[s];
+        return true;
+    };
     const float *ga = nullptr, *gb = nullptr;
     if (!join_side(0)) return false;
     if (ev) {
         // in stage order, so each stage's events bracket its own passes
         if (!join_side(1)) return false;
         rec(0);
-        if (!side_canvas(0, ga) || !side_canvas(1, gb) || !lag0(ga, gb)) return false;
+        if (!side_canvas(0, ga) || !side_canvas(1, gb) || !lag0(ga, gb) || !st_after_aux()) return false;
         rec(1);
         if (!side_rows(0, ga) || !side_rows(1, gb)) return false;
         rec(2);
@@ -648,10 +741,20 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
                  "inverse columns"))
         return false;
     rec(4);
-    // the correlation area (from both sides' autocorrelations) enters the row pass's score
-    if (!finish_acf()) return false;
-    job.cp.area = std::max(1.0, pair_area() * (1.0 / (job.gcell * job.gcell)));
-    const bool tmem = rows_tmem_supported(g.nx, job.plan.n_corr);
+    // the calibrated score reads the correlation area, computed on the device once both sides'
+    // autocorrelations are there, so the host does not wait for them here
+    if (job.calibrated) {
+        for (int i = 0; i < 2; ++i)
+            if (side[i].acf_pending && !cuda_ok(cudaStreamWaitEvent(st, side[i].acf_ev, 0), "area")) return false;
+        double* area = reinterpret_cast<double*>(res + 32);
+        if (!cuda_ok(pair_area_cells(A.acf_dev.as<double>(), B.acf_dev.as<double>(), job.gcell, area, st), "area"))
+            return false;
+        job.cp.area_dev = area;
+        counts[0] += 1;
+    }
+    if (!ev && !st_after_aux()) return false;
+    const bool tmem = job.box.mode == 0 && rows_tmem_supported(g.nx, job.plan.n_corr);
+    job.box.ta = box_a_.as<float>(), job.box.tb = box_b_.as<float>();
     if (!tmem &&
         !cuda_ok(inverse_rows(q_.as<float2>(), g, job.plan, job.line, job.S, twiddles(g.nx), st), "inverse rows"))
         return false;
@@ -660,7 +763,8 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
             return cuda_ok(inverse_rows_score_tmem(q_.as<float2>(), g, job.plan, twiddles(g.nx), job.cp, n00,
                                                    map_.as<float>(), best, zero, st, y0, rows),
                            "inverse rows (tensor memory)");
-        return cuda_ok(map_scores(q_.as<float2>(), g, job.cp, n00, map_.as<float>(), best, zero, st, 1, 0, 0, y0, rows),
+        return cuda_ok(map_scores(q_.as<float2>(), g, job.cp, n00, map_.as<float>(), best, zero, st, 1, 0, 0, y0, rows,
+                                  job.box),
                        "scores");
     };
     if (host_map) {
@@ -690,8 +794,7 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
         return false;
     }
     rec(5);
-    counts[0] += (job.identity_grid ? 11 : 13) - (have[0] ? (job.identity_grid ? 3 : 4) : 0) -
-                 (have[1] ? (job.identity_grid ? 3 : 4) : 0);
+    counts[0] += 5;  // zero lag, inverse columns, rows, scores, result
     return true;
 }
 
@@ -735,6 +838,7 @@ bool Engine::shift_map(const Mat3& Hm, bool exact, bool calibrated, unsigned cap
     memcpy(&fault, host + 28, 4);
     if (dft_pieces_ && fault)
         return fail("shift_map: the tensor-core column stage gave up waiting for its products; the map is not valid");
+    if (!finish_acf()) return false;
     map_result(job, best, zero, pair_area(), out);
     return true;
 }
@@ -878,7 +982,7 @@ bool Engine::bench_maps(const Mat3& Hm, unsigned flags, unsigned cap, unsigned w
     out[9] = job.g.ny;
     out[10] = job.g.cw;
     out[11] = job.g.ch;
-    out[12] = job.plan.n_real;
+    out[12] = job.n_side[0] + job.n_side[1];
     out[13] = job.plan.n_corr;
     out[14] = job.S;
     out[7] = job.g.Hh;

@@ -97,10 +97,21 @@ struct MapJob {
     CorrPlanDev plan;
     LinePlan row, col, line;
     int S;
-    CombineParams cp;  // cp.area set when the row pass is launched
+    CombineParams cp;  // cp.area_dev set by run_map
     double gcell = 1.0;  // canvas pixels per grid cell
     bool identity_grid;
     bool exact, calibrated;
+    // moments read from summed-area tables in place of transformed correlations (box.cu): the mode,
+    // each side's box of weight 1 on the grid, the real planes each side transforms
+    BoxSums box;
+    int n_side[2];
+    // the plan's real planes [p0, p1) alone, for the forward passes
+    CorrPlanDev planes(int p0, int p1) const {
+        CorrPlanDev p = plan;
+        p.n_real = p1 - p0;
+        for (int i = 0; i < p.n_real; ++i) p.planes[i] = plan.planes[p0 + i];
+        return p;
+    }
 };
 
 // One candidate of the sweep with its window on the sweep canvas (src/search.zig:340-366).
@@ -137,8 +148,9 @@ struct ScoredPose {
 };
 
 // The correlation plan for exact (15 planes) or global (5) scores, without the fourth feature's
-// planes when `three` (src/smi.zig:90-158).
-CorrPlanDev corr_plan_dev(bool exact, bool three);
+// planes when `three` (src/smi.zig:90-158); box_mode: without the correlations whose sums come from
+// summed-area tables (combine.cuh corr_fft).
+CorrPlanDev corr_plan_dev(bool exact, bool three, int box_mode = 0);
 
 // One direction's roto-scale map plan (src/smi.zig RsPlan).
 struct RsPlan {
@@ -181,6 +193,8 @@ class Engine {
     cudaEvent_t up_ev_ = nullptr;     // an image upload done
     static constexpr int kChunkEvents = 16;
     cudaEvent_t chunk_ev_[kChunkEvents] = {};
+    cudaStream_t aux_st_ = nullptr;  // a map's zero-lag overlap and moment tables, beside its transforms
+    cudaEvent_t aux_ev_[2] = {};     // its hand-offs: from the engine stream, back to it
 
     // counters since the last zc_gpu_counts: launches, submits, reads, waits
     uint32_t counts[4] = {0, 0, 0, 0};
@@ -210,6 +224,7 @@ class Engine {
     double pair_area() const;
 
     // maps
+    BoxSums box_sums(const MapJob& job) const;
     bool plan_map(const Mat3& H, bool exact, bool calibrated, unsigned cap, double min_overlap, MapJob& job);
     // host_map (nullable): with the tensor-memory row pass, the map is copied there in row
     // chunks on the copy stream during the pass (the caller synchronises copy_st_)
@@ -320,6 +335,8 @@ class Engine {
     // known): a map whose side has the same key reuses them instead of rebuilding that side's
     // canvas and forward transforms. Cleared by every other user of those buffers.
     std::array<std::vector<uint64_t>, 2> spec_key_;
+    int spec_planes_[2] = {0, 0};                  // leading planes of the side whose spectra are kept
+    std::array<std::vector<uint64_t>, 2> box_key_;  // what the sides' moment tables were built from
     bool spectra_cache_ = true;     // ZCMIR_B200_SPECTRA_CACHE=0 at creation: always rebuild
     bool spectra_cache_off_ = false;  // set while a benchmark times whole maps
     uint64_t build_counter_ = 0;
@@ -384,6 +401,7 @@ class Engine {
     cudaStream_t acf_st_ = nullptr;     // the features' autocorrelations, lowest priority
     int prio_lo_ = 0, prio_hi_ = 0;     // the device's stream priority range
     DevBuf canvas_a_, canvas_b_, grid_a_, grid_b_, half_a_, half_b_, q_, map_, res_, flush_;
+    DevBuf box_a_, box_b_, box_tmp_;  // the sides' summed-area tables; the build's scratch
     DevBuf pose_hinv_, pose_sums_, pose_coef_, pose_score_, pose_tsum_, pose_gens_;
     // the pose kernels' per-block totals and per-pose tickets (their sums added in block order)
     DevBuf pose_part_, pose_ticket_;

@@ -293,7 +293,7 @@ bool Engine::sweep_maps(const Mat3& H0, const SweepGrid& gv, int G, bool exact, 
         // with the stack's branch: the loaded stack and every buffer its maps use
         put(sweep_with_stack_ ? stack_gen_ : 0);
         if (sweep_with_stack_)
-            for (const DevBuf* b : {&canvas_a_, &canvas_b_, &grid_a_, &grid_b_, &half_a_, &half_b_, &q_, &map_, &res_,
+            for (const DevBuf* b : {&canvas_a_, &canvas_b_, &grid_a_, &grid_b_, &half_a_, &half_b_, &box_a_, &box_b_, &box_tmp_, &q_, &map_, &res_,
                                     &stack_res_, &dft_scratch_})
                 put((uint64_t)(uintptr_t)b->p), put(b->gen);
     }

@@ -18,6 +18,7 @@
 // N = 1024 → 16 · 8 · 8 with 64 threads per line (TX = 8). The first stage's butterfly of
 // thread t takes rows t + r·N/16; the middle stages pass through a padded line buffer; the last
 // stage stores straight to Q.
+#include <algorithm>
 #include <mutex>
 
 #include "fft.cuh"
@@ -365,8 +366,10 @@ cudaError_t launch_tma(const float2* ha, const float2* hb, const MapGeom& g, con
     const int ncols = g.nx / 2 + 1;
     const size_t pstride = (size_t)g.ny * g.WP;
     CUtensorMap ma, mb;
-    if (!encode_cplx_map(&ma, ha, ncols, g.ny, plan.n_real, g.WP, pstride, SH::TX, kBoxRows) ||
-        !encode_cplx_map(&mb, hb, ncols, g.ny, plan.n_real, g.WP, pstride, SH::TX, kBoxRows))
+    // each side's planes up to the last one a correlation reads (a side may hold fewer than the plan)
+    const int na = 1 + *std::max_element(plan.ca, plan.ca + plan.n_corr), nb = 1 + *std::max_element(plan.cb, plan.cb + plan.n_corr);
+    if (!encode_cplx_map(&ma, ha, ncols, g.ny, na, g.WP, pstride, SH::TX, kBoxRows) ||
+        !encode_cplx_map(&mb, hb, ncols, g.ny, nb, g.WP, pstride, SH::TX, kBoxRows))
         return cudaErrorInvalidValue;
     cudaError_t e = cudaSuccess;
     if (!fault && (e = fault_word(&fault)) != cudaSuccess) return e;

@@ -4,17 +4,19 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "box.cuh"
 #include "fft.cuh"
 
 namespace zc {
 
 // ── per-image features (features.cu) ──
+constexpr int kAcfSums = 153 * 4;  // lags dy = 0..8, dx = −8..8, of 4 planes
 // Scratch the feature build needs on the device (sizes in bytes are fixed; see features.cu).
 struct FeatScratch {
     double* stats = nullptr;     // [0] Σg, [1] Σ(g − mean)², [2..21] whitening moments
     unsigned* hist = nullptr;    // 256 bins
     float* wt = nullptr;         // L⁻¹ (16) and μ (4) of the whitening
-    float* acf_part = nullptr;   // per-tile autocorrelation partial sums
+    float* acf_part = nullptr;   // per-tile autocorrelation partial sums, kAcfSums per 32 × 32 tile
     size_t acf_part_cap = 0;     // floats
     double* acf = nullptr;       // 289 × 4 normalised autocorrelation
 };
@@ -26,6 +28,9 @@ cudaError_t build_features(float* gray, int w, int h, int mode, bool half, float
 // the features' autocorrelation sums at |τ| ≤ 8 (289 lags × 4 planes, device doubles in s.acf;
 // per-tile partials in s.acf_part)
 cudaError_t autocorrelation(const float* feat, int w, int h, FeatScratch& s, cudaStream_t st);
+// a pair's feature correlation area in cells of gcell pixels a side, from both images' sums (at
+// least 1 pixel and 1 cell), into *area
+cudaError_t pair_area_cells(const double* acf_a, const double* acf_b, double gcell, double* area, cudaStream_t st);
 
 // ── shift maps (shiftmap.cu) ──
 struct MapGeom {
@@ -43,6 +48,7 @@ struct CombineParams {
                      // over the norm product, which the n00 slot carries)
     float min_n;     // overlap floor (cells)
     double area;     // feature correlation area in cells (calibrated z)
+    const double* area_dev = nullptr;  // read in place of area where set (device memory)
     double ridge;
     double inv_nn;   // 1/(nx·ny): the inverse FFT's scale
     // log-polar maps: each correlation at log-radius lag k (row k, wrapped) is scaled by
@@ -107,10 +113,15 @@ cudaError_t inverse_rows(float2* Q, const MapGeom& g, const CorrPlanDev& plan, c
 // the per-shift score and the argmax from those real rows: map (ny × nx f32), best key (u64),
 // zero-lag score (best and zero may be null); n00: one zero-lag overlap per item. Rows y0 ..
 // y0 + rows − 1 (rows < 0: to the last), so a caller can copy the map out in row chunks while the
-// later rows run
+// later rows run. bx: moment sums read from tables in place of transformed correlations
 cudaError_t map_scores(const float2* Q, const MapGeom& g, const CombineParams& cp, const double* n00, float* map,
                        unsigned long long* best, float* zero, cudaStream_t st, int batch = 1, size_t q_stride = 0,
-                       size_t map_stride = 0, int y0 = 0, int rows = -1);
+                       size_t map_stride = 0, int y0 = 0, int rows = -1, const BoxSums& bx = {});
+// the summed-area table of a side's moment planes (box.cuh) from its 1 + nf sample planes of ch × cw
+// cells; t and tmp: box_table_bytes / box_scratch_bytes
+size_t box_table_bytes(int nf, int cw, int ch);
+size_t box_scratch_bytes(int nf, int cw, int ch);
+cudaError_t box_table(const float* grid, int cw, int ch, int nf, float* t, void* tmp, cudaStream_t st);
 // both passes in one with the sums in tensor memory, a whole row per block (nx = 2048)
 bool rows_tmem_supported(int nx, int n_corr);
 cudaError_t inverse_rows_score_tmem(const float2* Q, const MapGeom& g, const CorrPlanDev& plan, const float2* tw_nx,

@@ -75,8 +75,9 @@ struct RealPlane {
 // LO: cw ≤ nx/2, so the first butterflies read only the row's lower half.
 template <class F, bool LO>
 __global__ void __launch_bounds__(512, 1) k_fwd_rows(const float* __restrict__ grid, int cw, int ch, int WP,
-                                                     CorrPlanDev plan, F f, int lpb, float2* __restrict__ half,
-                                                     size_t pstride, size_t gbs, size_t hbs) {
+                                                     CorrPlanDev plan, F f, int lpb, int products,
+                                                     float2* __restrict__ half, size_t pstride, size_t gbs,
+                                                     size_t hbs) {
     extern __shared__ float2 smem[];
     const int nx = f.n(), tl = f.tl();
     const int y = blockIdx.x;
@@ -94,9 +95,11 @@ __global__ void __launch_bounds__(512, 1) k_fwd_rows(const float* __restrict__ g
         float v[5];
 #pragma unroll
         for (int p = 0; p < 5; ++p) row[p * cw + x] = v[p] = __ldg(&grid[p * gn + (size_t)y * cw + x]);
-        const float inv = v[0] <= 1e-6f ? 0.f : 1.f / v[0];
+        if (products) {
+            const float inv = v[0] <= 1e-6f ? 0.f : 1.f / v[0];
 #pragma unroll
-        for (int p = 1; p < 5; ++p) row[(4 + p) * cw + x] = v[p] * inv;
+            for (int p = 1; p < 5; ++p) row[(4 + p) * cw + x] = v[p] * inv;
+        }
     }
     __syncthreads();
     const int n_cplx = (plan.n_real + 1) / 2;
@@ -271,13 +274,15 @@ cudaError_t run_pass(Pass p, F f, const PassArgs& a, cudaStream_t st) {
     cudaError_t e;
     if (p == Pass::FwdRows) {
         const int n_cplx = (plan.n_real + 1) / 2;
-        // up to 256 threads of lines (one line of more for the longest rows: 8192 points, 512 threads)
-        const int lines = std::min(lines_per_block(tl, 256), n_cplx);
-        const size_t sm = (size_t)lines * padded_len(g.nx) * sizeof(float2) + (size_t)9 * g.cw * sizeof(float);
+        // the row's lines at once where 512 threads hold them (5 planes: 3 lines), else up to 256
+        // threads of lines (one line of more for the longest rows: 8192 points, 512 threads)
+        const int lines = std::min(n_cplx, n_cplx <= 3 && n_cplx * tl <= 512 ? n_cplx : lines_per_block(tl, 256));
+        const int products = plan.planes[plan.n_real - 1] >= 5;
+        const size_t sm = (size_t)lines * padded_len(g.nx) * sizeof(float2) + (size_t)(products ? 9 : 5) * g.cw * sizeof(float);
         auto k = 2 * g.cw <= g.nx ? k_fwd_rows<F, true> : k_fwd_rows<F, false>;
         if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
-        k<<<dim3(g.ch, a.batch), lines * tl, sm, st>>>(a.grid, g.cw, g.ch, g.WP, plan, f, lines, a.half, pstride,
-                                                       a.grid_stride, a.half_stride);
+        k<<<dim3(g.ch, a.batch), lines * tl, sm, st>>>(a.grid, g.cw, g.ch, g.WP, plan, f, lines, products, a.half,
+                                                       pstride, a.grid_stride, a.half_stride);
         return cudaGetLastError();
     }
     if (p == Pass::FwdCols || p == Pass::InvCols)

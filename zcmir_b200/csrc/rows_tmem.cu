@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(512, 1) k_rows_tmem(const float2* __restrict__
     __syncthreads();
     tc_fence_after();
 
+    if (CALIB) read_area(cp);
     const double n00 = *n00p;
     float bv = -3.4e38f;
     uint32_t bi = 0xffffffffu;
@@ -154,7 +155,12 @@ __global__ void __launch_bounds__(512, 1) k_rows_tmem(const float2* __restrict__
         tmem_ld32(tq + (uint32_t)(j * kTmemSlots), r);
         tmem_wait_ld();
         const float sc = combine_t<NF, EXACT, CALIB>(
-            [&](int k) { return k < kTmemSlots ? __uint_as_float(r[k]) : cs[(size_t)(k - kTmemSlots) * N + m]; }, cp, n00);
+            [&](int c) {
+                constexpr CorrSource from = corr_source<NF, 0>();
+                const int k = from.at[c];
+                return k < kTmemSlots ? __uint_as_float(r[k]) : cs[(size_t)(k - kTmemSlots) * N + m];
+            },
+            cp, n00);
         const uint32_t idx = (uint32_t)y * (uint32_t)N + (uint32_t)m;
         map[idx] = sc;
         if (sc > bv || (sc == bv && idx < bi)) {
