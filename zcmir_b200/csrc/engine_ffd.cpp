@@ -111,13 +111,15 @@ bool Engine::ffd_gradient(const Mat3& H, double* score, double* grad, size_t len
     ok = cuda_ok(cudaMemcpyAsync(ffd_dev_.p, h.data(), h.size() * 4, cudaMemcpyHostToDevice, st), "ffd_gradient") &&
          cuda_ok(cudaMemcpyAsync(dh, hinv, sizeof hinv, cudaMemcpyHostToDevice, st), "ffd_gradient");
     PoseRed rd;
-    ok = ok && pose_red(1, rd);
+    ok = ok && pose_red(nd, rd);
+    PoseCall pc;
+    pc.a = pa, pc.b = pb, pc.sym = sym, pc.hinv = dh, pc.n = 1, pc.ffd[0] = ff, pc.ffd[1] = fi, pc.red = rd;
+    PoseScores ps;
+    ps.exact = exact, ps.coef = coef, ps.score = pose_score_.as<double>();
+    ok = ok && cuda_ok(pose_moments(pc, sums, ps, st), "ffd_gradient");
     for (int d = 0; ok && d < nd; ++d) {
         const PoseSide &a = d ? pb : pa, &b = d ? pa : pb;
         const PoseFfd& f = d ? fi : ff;
-        ok = cuda_ok(pose_moments(a, b, dh + 9 * d, 1, sums + kMom * d, st, f, nullptr, rd), "ffd_gradient") &&
-             cuda_ok(pose_coefs(sums + kMom * d, 1, exact, coef + kCoef * d, pose_score_.as<double>() + d, st),
-                     "ffd_gradient");
         for (int c = 0; ok && c < nchunk; ++c)
             ok = cuda_ok(pose_ffd_grad(a, b, dh + 9 * d, coef + kCoef * d, f, 16 * c, out + ((size_t)d * nchunk + c) * 32, st,
                                        rd),

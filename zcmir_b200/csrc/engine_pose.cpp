@@ -71,18 +71,16 @@ bool Engine::eval_poses(const std::vector<Mat3>& Hs, bool grad, bool hess, std::
     const int n = (int)Hs.size(), nd = sym ? 2 : 1, nk = n_keys(homog);
     if (n == 0) return true;
     const size_t m = (size_t)nd * n;
-    bool ok = cuda_ok(pose_hinv_.ensure(m * 9 * 4), "score") && cuda_ok(pose_sums_.ensure(m * kMom * 8), "score") &&
-              cuda_ok(pose_coef_.ensure(m * kCoef * 4), "score") && cuda_ok(pose_score_.ensure(m * 8), "score") &&
-              cuda_ok(pose_tsum_.ensure(m * kGrad * 8), "score") && cuda_ok(pose_gens_.ensure(2 * 72 * 4), "score");
+    bool ok = cuda_ok(pose_sums_.ensure(m * kMom * 8), "score") && cuda_ok(pose_coef_.ensure(m * kCoef * 4), "score") &&
+              cuda_ok(pose_score_.ensure(m * 8), "score") && cuda_ok(pose_tsum_.ensure(m * kGrad * 8), "score");
     if (!ok) return false;
     // inverse poses: forward direction H⁻¹; inverse direction (pose H⁻¹) its inverse; written to
-    // page-locked memory, as the sums come back into it, so neither copy is staged
-    const size_t n_in = m * 9 + 2 * 72, n_out = m * kMom + m + (grad ? m * kGrad : 0);
+    // page-locked memory, as the kernels write the sums back into it, so no copy is staged
+    const size_t n_in = m * 9, n_out = m * kMom + m + (grad ? m * kGrad : 0);
     if (!cuda_ok(pose_in_pin_.ensure(n_in * sizeof(float)), "score") ||
         !cuda_ok(pose_out_pin_.ensure(n_out * sizeof(double)), "score"))
         return false;
     float* pose_host = pose_in_pin_.as<float>();
-    std::fill(pose_host, pose_host + n_in, 0.f);
     for (int i = 0; i < n; ++i) {
         const Mat3 Hi = inv3(Hs[i]);
         for (int k = 0; k < 9; ++k) pose_host[(size_t)i * 9 + k] = (float)Hi[k];
@@ -92,50 +90,35 @@ bool Engine::eval_poses(const std::vector<Mat3>& Hs, bool grad, bool hess, std::
         }
     }
     const Side &A = side[0], &B = side[1];
-    // generators in the destination's pixels: the fixed image forward, the moving one inverse
-    const auto gf = generators(homog, B.w, B.h), gi = generators(homog, A.w, A.h);
-    float* gens = pose_host + m * 9;
-    for (int k = 0; k < 8; ++k)
-        for (int e = 0; e < 9; ++e) {
-            gens[k * 9 + e] = (float)gf[k][e];
-            gens[72 + k * 9 + e] = (float)gi[k][e];
-        }
-    float* dh = pose_hinv_.as<float>();
-    float* dg = pose_gens_.as<float>();
-    if (!cuda_ok(cudaMemcpyAsync(dh, pose_host, m * 9 * 4, cudaMemcpyHostToDevice, st), "score") ||
-        !cuda_ok(cudaMemcpyAsync(dg, gens, 2 * 72 * 4, cudaMemcpyHostToDevice, st), "score"))
-        return false;
-    const PoseSide pa{A.feat.as<float>(), A.feat4.as<float4>(), A.w, A.h},
-        pb{B.feat.as<float>(), B.feat4.as<float4>(), B.w, B.h};
-    double* sums = pose_sums_.as<double>();
-    double* tsum = pose_tsum_.as<double>();
-    float* coef = pose_coef_.as<float>();
-    // a live spline moves the samples of both directions (src/pair.zig:127-150)
-    PoseFfd ff, fi;
-    if (!(pose_cps ? ffd_pose_dirs(pose_cps, n, ff, fi) : ffd_dirs(ff, fi))) return false;
-    PoseRed rd;
-    if (!pose_red(n, rd)) return false;
-    if (!cuda_ok(pose_moments(pa, pb, dh, n, sums, st, ff, nullptr, rd), "moments")) return false;
-    if (sym &&
-        !cuda_ok(pose_moments(pb, pa, dh + (size_t)n * 9, n, sums + (size_t)n * kMom, st, fi, nullptr, rd), "moments"))
-        return false;
-    if (!cuda_ok(pose_coefs(sums, (int)m, exact, coef, pose_score_.as<double>(), st), "score")) return false;
-    counts[0] += nd + 1;
-    if (grad) {
-        if (!cuda_ok(pose_tangent(pa, pb, dh, coef, dg, n, hess, tsum, st, ff, nullptr, rd), "gradient")) return false;
-        if (sym && !cuda_ok(pose_tangent(pb, pa, dh + (size_t)n * 9, coef + (size_t)n * kCoef, dg + 72, n, hess,
-                                         tsum + (size_t)n * kGrad, st, fi, nullptr, rd),
-                            "gradient"))
+    PoseCall pc;
+    pc.a = PoseSide{A.feat.as<float>(), A.feat4.as<float4>(), A.w, A.h};
+    pc.b = PoseSide{B.feat.as<float>(), B.feat4.as<float4>(), B.w, B.h};
+    pc.sym = sym, pc.n = n, pc.hinv_host = pose_host;
+    if (m > (size_t)kPoseInline) {
+        if (!cuda_ok(pose_hinv_.ensure(n_in * 4), "score") ||
+            !cuda_ok(cudaMemcpyAsync(pose_hinv_.p, pose_host, n_in * 4, cudaMemcpyHostToDevice, st), "score"))
             return false;
-        counts[0] += nd;
+        pc.hinv = pose_hinv_.as<float>();
     }
     double* hs = pose_out_pin_.as<double>();
     double* hsc = hs + m * kMom;
     double* ht = hsc + m;
-    if (!cuda_ok(cudaMemcpyAsync(hs, sums, m * kMom * 8, cudaMemcpyDeviceToHost, st), "score") ||
-        !cuda_ok(cudaMemcpyAsync(hsc, pose_score_.p, m * 8, cudaMemcpyDeviceToHost, st), "score"))
-        return false;
-    if (grad && !cuda_ok(cudaMemcpyAsync(ht, tsum, m * kGrad * 8, cudaMemcpyDeviceToHost, st), "score")) return false;
+    float* coef = pose_coef_.as<float>();
+    // a live spline moves the samples of both directions (src/pair.zig:127-150)
+    if (!(pose_cps ? ffd_pose_dirs(pose_cps, n, pc.ffd[0], pc.ffd[1]) : ffd_dirs(pc.ffd[0], pc.ffd[1]))) return false;
+    if (!pose_red((int)m, pc.red)) return false;
+    const PoseScores ps{exact, coef, pose_score_.as<double>(), hs, hsc};
+    if (!cuda_ok(pose_moments(pc, pose_sums_.as<double>(), ps, st), "moments")) return false;
+    counts[0] += 1;
+    if (grad) {
+        // generators in the destination's pixels: the fixed image forward, the moving one inverse
+        const auto gf = generators(homog, B.w, B.h), gi = generators(homog, A.w, A.h);
+        float gens[144];
+        for (int k = 0; k < 8; ++k)
+            for (int e = 0; e < 9; ++e) gens[k * 9 + e] = (float)gf[k][e], gens[72 + k * 9 + e] = (float)gi[k][e];
+        if (!cuda_ok(pose_tangent(pc, coef, gens, hess, pose_tsum_.as<double>(), ht, st), "gradient")) return false;
+        counts[0] += 1;
+    }
     if (!cuda_ok(cudaStreamSynchronize(st), "score")) return false;
     counts[1]++;
     counts[2] += grad ? 3 : 2;

@@ -457,14 +457,14 @@ bool Engine::gn_batch_dev(const std::vector<Mat3>& Hs, unsigned iters, const std
               cuda_ok(gn_cur_.ensure((size_t)n * 8), "refine") && cuda_ok(pose_hinv_.ensure(mt * 9 * 4), "refine") &&
               cuda_ok(pose_sums_.ensure(mt * kMom * 8), "refine") &&
               cuda_ok(pose_coef_.ensure(mt * kCoef * 4), "refine") && cuda_ok(pose_score_.ensure(mt * 8), "refine") &&
-              cuda_ok(pose_tsum_.ensure(m * kGrad * 8), "refine") && cuda_ok(pose_gens_.ensure(2 * 72 * 4), "refine") &&
-              cuda_ok(gn_pin_.ensure((size_t)n * 9 * 8 + (size_t)n * 8 + act_b + 2 * 72 * 4), "refine");
+              cuda_ok(pose_tsum_.ensure(m * kGrad * 8), "refine") &&
+              cuda_ok(gn_pin_.ensure((size_t)n * 9 * 8 + (size_t)n * 8 + act_b), "refine");
     if (!ok) return false;
-    // page-locked staging: poses (f64), scores (f64), moved flags, generators (f32)
+    // page-locked staging: poses (f64), scores (f64), moved flags
     double* hH = gn_pin_.as<double>();
     double* hcur = hH + (size_t)n * 9;
     unsigned char* hact = reinterpret_cast<unsigned char*>(hcur + n);
-    float* hgens = reinterpret_cast<float*>(hact + act_b);
+    float hgens[144];
     for (int i = 0; i < n; ++i)
         for (int k = 0; k < 9; ++k) hH[(size_t)i * 9 + k] = Hs[i][k];
     const auto gf = generators(homog, B.w, B.h), gi = generators(homog, A.w, A.h);
@@ -479,44 +479,39 @@ bool Engine::gn_batch_dev(const std::vector<Mat3>& Hs, unsigned iters, const std
     unsigned char* act = gn_active_.as<unsigned char>();
     unsigned char* valid = gn_valid_.as<unsigned char>();
     float* dh = pose_hinv_.as<float>();
-    float* dg = pose_gens_.as<float>();
     double* sums = pose_sums_.as<double>();
     double* tsum = pose_tsum_.as<double>();
     double* score = pose_score_.as<double>();
     float* coef = pose_coef_.as<float>();
     std::vector<double> ninf((size_t)n, -INFINITY);
     if (!cuda_ok(cudaMemcpyAsync(H, hH, (size_t)n * 9 * 8, cudaMemcpyHostToDevice, st), "refine") ||
-        !cuda_ok(cudaMemcpyAsync(dg, hgens, 2 * 72 * 4, cudaMemcpyHostToDevice, st), "refine") ||
         !cuda_ok(cudaMemsetAsync(act, 1, (size_t)n, st), "refine"))
         return false;
     std::copy(ninf.begin(), ninf.end(), hcur);
     if (!cuda_ok(cudaMemcpyAsync(cur, hcur, (size_t)n * 8, cudaMemcpyHostToDevice, st), "refine")) return false;
     counts[2] += 3;
-    const PoseSide pa{A.feat.as<float>(), A.feat4.as<float4>(), A.w, A.h},
-        pb{B.feat.as<float>(), B.feat4.as<float4>(), B.w, B.h};
-    PoseRed rd;
-    if (!pose_red((int)nt, rd)) return false;
+    PoseCall at, tries;  // the poses; their candidates
+    at.a = PoseSide{A.feat.as<float>(), A.feat4.as<float4>(), A.w, A.h};
+    at.b = PoseSide{B.feat.as<float>(), B.feat4.as<float4>(), B.w, B.h};
+    at.sym = sym, at.hinv = dh;
+    if (!pose_red((int)mt, at.red)) return false;
+    tries = at;
+    at.n = n, at.mask = act;
+    tries.n = (int)nt, tries.mask = valid;
+    PoseScores ps;
+    ps.exact = exact, ps.coef = coef, ps.score = score;
     constexpr unsigned kGnBatch = 4;
     for (unsigned it = 0; it < iters && !cancel; ++it) {
         // the poses: moments, coefficients, gradient and Gauss–Newton sums
-        ok = cuda_ok(gn_hinv(H, n, d.sym, dh, st), "refine") &&
-             cuda_ok(pose_moments(pa, pb, dh, n, sums, st, {}, act, rd), "refine") &&
-             (!sym || cuda_ok(pose_moments(pb, pa, dh + (size_t)n * 9, n, sums + (size_t)n * kMom, st, {}, act, rd), "refine")) &&
-             cuda_ok(pose_coefs(sums, (int)m, exact, coef, score, st), "refine") &&
-             cuda_ok(pose_tangent(pa, pb, dh, coef, dg, n, true, tsum, st, {}, act, rd), "refine") &&
-             (!sym || cuda_ok(pose_tangent(pb, pa, dh + (size_t)n * 9, coef + (size_t)n * kCoef, dg + 72, n, true,
-                                           tsum + (size_t)n * kGrad, st, {}, act, rd),
-                              "refine")) &&
+        ok = cuda_ok(gn_hinv(H, n, d.sym, dh, st), "refine") && cuda_ok(pose_moments(at, sums, ps, st), "refine") &&
+             cuda_ok(pose_tangent(at, coef, hgens, true, tsum, nullptr, st), "refine") &&
              // the candidates, then their scores
              cuda_ok(gn_propose(d, ga, H, sums, score, tsum, act, cur, Ht, valid, st), "refine") &&
              cuda_ok(gn_hinv(Ht, (int)nt, d.sym, dh, st), "refine") &&
-             cuda_ok(pose_moments(pa, pb, dh, (int)nt, sums, st, {}, valid, rd), "refine") &&
-             (!sym ||
-              cuda_ok(pose_moments(pb, pa, dh + nt * 9, (int)nt, sums + nt * kMom, st, {}, valid, rd), "refine")) &&
-             cuda_ok(pose_coefs(sums, (int)mt, exact, coef, score, st), "refine") &&
+             cuda_ok(pose_moments(tries, sums, ps, st), "refine") &&
              cuda_ok(gn_select(d, score, valid, Ht, H, cur, act, st), "refine");
         if (!ok) return false;
-        counts[0] += 5 + 2 * nd + 2 + nd + 2;
+        counts[0] += 7;
         if ((it + 1) % kGnBatch != 0 || it + 1 == iters) continue;
         // stop once no pose moved in the last iteration
         if (!cuda_ok(cudaMemcpyAsync(hact, act, (size_t)n, cudaMemcpyDeviceToHost, st), "refine") ||

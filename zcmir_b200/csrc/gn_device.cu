@@ -3,7 +3,7 @@
 //
 // Each iteration is, for n poses at once: the poses' inverse maps, their overlap moments,
 // scores, tangent gradients and Gauss–Newton matrices (the pose kernels of pose.cu); then, one
-// warp per pose, the symmetric pair's gradient and matrix, the unit-ascent candidates (the step
+// block per pose, the symmetric pair's gradient and matrix, the unit-ascent candidates (the step
 // ladder `amps`) and the Gauss–Newton candidates (the solved step at 0.5, 1, 2, 4, 8 times, each
 // capped at a tangent norm of 0.25), each composed onto the pose in normalised fixed
 // coordinates; their scores; and, per pose, the first candidate in order that beats the score so
@@ -20,7 +20,7 @@ namespace zc {
 namespace {
 
 // sums per pose row, tangent sums per pose row; candidates per pose: at most 16 ascent steps and
-// the 5 Gauss–Newton multiples, one lane each
+// the 5 Gauss–Newton multiples
 constexpr int kMomN = 45, kGradN = 44, kMaxTry = 21;
 
 __device__ void d_mul3(const double* a, const double* b, double* o) {
@@ -82,107 +82,6 @@ __device__ void d_vee(const double* A0, bool homog, double* out) {
     for (int k = 0; k < 8; ++k) out[k] = v[k];
 }
 
-// scaling and squaring of a 13-term Taylor series (lie.hpp expm3)
-__device__ void d_expm3(const double* A, double* T) {
-    double nrm = 0;
-    for (int i = 0; i < 9; ++i) nrm = fmax(nrm, fabs(A[i]));
-    int s = 0;
-    for (double v = nrm; v > 0.5 && s < 10; v *= 0.5) ++s;
-    const double sc = ldexp(1.0, -s);
-    double B[9], P[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-    for (int i = 0; i < 9; ++i) B[i] = A[i] * sc;
-    for (int i = 0; i < 9; ++i) T[i] = P[i];
-    for (int k = 1; k < 14; ++k) {
-        d_mul3(P, B, P);
-        for (int i = 0; i < 9; ++i) P[i] /= (double)k;
-        for (int i = 0; i < 9; ++i) T[i] += P[i];
-    }
-    for (int i = 0; i < s; ++i) d_mul3(T, T, T);
-}
-
-__device__ void d_project_group(const double* H, bool homog, double* o) {
-    const double s = fabs(H[8]) > 1e-12 ? H[8] : 1;
-    for (int i = 0; i < 9; ++i) o[i] = H[i] / s;
-    if (!homog) {
-        o[6] = 0;
-        o[7] = 0;
-        o[8] = 1;
-    }
-}
-
-// exp(ξ̂) applied in normalised coordinates of a dw×dh destination (lie.hpp composeN)
-__device__ void d_composeN(const double* H0, const double* x, bool homog, double dw, double dh, double* o) {
-    double N[9], Ni[9], X[9], E[9], t[9];
-    d_destN(dw, dh, N);
-    d_inv3(N, Ni);
-    d_hat(x, homog, X);
-    d_expm3(X, E);
-    d_mul3(Ni, E, t);
-    d_mul3(t, N, t);
-    d_mul3(t, H0, t);
-    d_project_group(t, homog, o);
-}
-
-// dS/dξ on H given dS/dη on H⁻¹ (lie.hpp adjoint_grad)
-__device__ void d_adjoint_grad(const double* g_eta, const double* H, bool homog, double mw, double mh, double fw,
-                               double fh, double* out) {
-    double Hi[9], Nm[9], Nf[9], Nfi[9], M[9], Mi[9], t[9];
-    d_inv3(H, Hi);
-    d_destN(mw, mh, Nm);
-    d_destN(fw, fh, Nf);
-    d_inv3(Nf, Nfi);
-    d_mul3(Nm, Hi, t);
-    d_mul3(t, Nfi, M);
-    d_inv3(M, Mi);
-    const int nk = homog ? 8 : 6;
-    for (int k = 0; k < 8; ++k) out[k] = 0;
-    for (int i = 0; i < nk; ++i) {
-        double e[8] = {0, 0, 0, 0, 0, 0, 0, 0}, X[9], cc[8];
-        e[i] = 1;
-        d_hat(e, homog, X);
-        d_mul3(M, X, t);
-        d_mul3(t, Mi, t);
-        d_vee(t, homog, cc);
-        for (int j = 0; j < nk; ++j) out[i] -= g_eta[j] * cc[j];
-    }
-}
-
-// A·x = b by Gauss–Jordan with partial pivoting (lie.hpp solve_linear)
-__device__ bool d_solve_linear(const double* A, const double* b, int n, double* x) {
-    double M[64];
-    for (int i = 0; i < n * n; ++i) M[i] = A[i];
-    for (int i = 0; i < n; ++i) x[i] = b[i];
-    for (int i = 0; i < n; ++i) {
-        int piv = i;
-        for (int r = i + 1; r < n; ++r)
-            if (fabs(M[r * n + i]) > fabs(M[piv * n + i])) piv = r;
-        if (piv != i) {
-            for (int j = 0; j < n; ++j) {
-                const double tmp = M[i * n + j];
-                M[i * n + j] = M[piv * n + j];
-                M[piv * n + j] = tmp;
-            }
-            const double tmp = x[i];
-            x[i] = x[piv];
-            x[piv] = tmp;
-        }
-        const double d = M[i * n + i];
-        if (!isfinite(d) || fabs(d) < 1e-300) return false;
-        for (int r = 0; r < n; ++r) {
-            if (r == i) continue;
-            const double f = M[r * n + i] / d;
-            if (f == 0) continue;
-            for (int j = i; j < n; ++j) M[r * n + j] -= f * M[i * n + j];
-            x[r] -= f * x[i];
-        }
-    }
-    for (int i = 0; i < n; ++i) {
-        x[i] /= M[i * n + i];
-        if (!isfinite(x[i])) return false;
-    }
-    return true;
-}
-
 __device__ __forceinline__ double fin(double v) { return isfinite(v) ? v : 0.0; }
 
 // one direction's gradient and Gauss–Newton matrix from its tangent sums (zero below 12 overlap)
@@ -211,59 +110,94 @@ __global__ void k_gn_hinv(const double* __restrict__ H, int n, int sym, float* _
     }
 }
 
-// one warp per pose: the lanes share the pull-back's columns, the matrix entries and the
-// candidates; each value is still computed by one lane in the host loop's order
-__global__ void __launch_bounds__(32) k_gn_propose(GnDims d, GnAmps amps, const double* __restrict__ H,
-                                                   const double* __restrict__ sums, const double* __restrict__ score,
-                                                   const double* __restrict__ tsum,
-                                                   const unsigned char* __restrict__ active, double* __restrict__ cur,
-                                                   double* __restrict__ Htry, unsigned char* __restrict__ valid) {
-    const int i = blockIdx.x, lane = threadIdx.x;
+// One element of a 3 × 3 product, in d_mul3's order.
+__device__ __forceinline__ double mul3_at(const double* a, const double* b, int e) {
+    const int r = 3 * (e / 3), c = e % 3;
+    return a[r] * b[c] + a[r + 1] * b[3 + c] + a[r + 2] * b[6 + c];
+}
+
+// A block per pose. Each value is computed in the host loop's order by one thread, and values that do
+// not depend on one another by threads of their own: the pull-back's 8 columns, the matrix's 64
+// entries, the rows of the elimination, and the 9 entries of each candidate's 3 × 3 products (the
+// exponential's series divides 117 entries a candidate). With a warp per pose and a lane per
+// candidate the chains took 61 µs.
+constexpr int kProposeThreads = 192;  // ≥ 9 · kMaxTry
+static_assert(kProposeThreads >= 9 * kMaxTry, "nine threads per candidate");
+
+__global__ void __launch_bounds__(kProposeThreads) k_gn_propose(GnDims d, GnAmps amps, const double* __restrict__ H,
+                                                                const double* __restrict__ sums,
+                                                                const double* __restrict__ score,
+                                                                const double* __restrict__ tsum,
+                                                                const unsigned char* __restrict__ active,
+                                                                double* __restrict__ cur, double* __restrict__ Htry,
+                                                                unsigned char* __restrict__ valid) {
+    const int i = blockIdx.x, tid = threadIdx.x;
     const int T = d.T, nk = d.nk, n = d.n;
     const bool homog = d.homog != 0, sym = d.sym != 0;
-    __shared__ double g[8], A[64], gf[8], Af[64], gb[8], Ab[64], PT[64], step[8], dv[8];
-    __shared__ int use_ascent, use_step;
+    __shared__ double g[8], A[64], gf[8], Af[64], gb[8], Ab[64], PT[64], step[8], dv[8], cc[8][8], Mw[9], Mwi[9], N[9], Ni[9];
+    __shared__ double M[64], rhs[8], fac[8], E[kMaxTry][9], P[kMaxTry][9], B[kMaxTry][9];
+    __shared__ int use_ascent, use_step, piv, sq[kMaxTry];
     unsigned char* ok = valid + (size_t)i * T;
-    if (lane < T) ok[lane] = 0;
+    if (tid < T) ok[tid] = 0;
     if (!active[i]) return;  // uniform over the block
     const double* Hp = H + (size_t)i * 9;
-    if (lane == 0) {
+    // independent starts, a warp each: both directions' sums, the pull-back's map, the fixed frame
+    if (tid == 0) {
         const double fwd = fin(score[i]), inv = sym ? fin(score[n + i]) : 0.0;
         cur[i] = sym ? 0.5 * (fwd + inv) : fwd;
         unpack(tsum + (size_t)i * kGradN, sums[(size_t)i * kMomN], nk, gf, Af);
-        if (sym) unpack(tsum + ((size_t)n + i) * kGradN, sums[((size_t)n + i) * kMomN], nk, gb, Ab);
+    } else if (tid == 32 && sym) {
+        unpack(tsum + ((size_t)n + i) * kGradN, sums[((size_t)n + i) * kMomN], nk, gb, Ab);
+    } else if (tid == 64 && sym) {
+        // M = N_moving H⁻¹ N_fixed⁻¹ and its inverse (lie.hpp adjoint_grad)
+        double Hi[9], Nm[9], Nf[9], Nfi[9], t[9];
+        d_inv3(Hp, Hi);
+        d_destN(d.mw, d.mh, Nm);
+        d_destN(d.fw, d.fh, Nf);
+        d_inv3(Nf, Nfi);
+        d_mul3(Nm, Hi, t);
+        d_mul3(t, Nfi, Mw);
+        d_inv3(Mw, Mwi);
+    } else if (tid == 96) {
+        d_destN(d.fw, d.fh, N);
+        d_inv3(N, Ni);
     }
-    for (int q = lane; q < 64; q += 32) PT[q] = 0;
-    __syncwarp();
+    __syncthreads();
     if (!sym) {
-        for (int q = lane; q < 64; q += 32) A[q] = Af[q];
-        if (lane < 8) g[lane] = gf[lane];
+        if (tid < 64) A[tid] = Af[tid];
+        if (tid < 8) g[tid] = gf[tid];
     } else {
-        // the pull-back's columns (lanes 0..nk−1) and the pulled inverse-direction gradient (lane 8)
-        double col[8];
-        if (lane < nk) {
-            double e[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            e[lane] = 1;
-            d_adjoint_grad(e, Hp, homog, d.mw, d.mh, d.fw, d.fh, col);
-            for (int q = 0; q < nk; ++q) PT[q * nk + lane] = col[q];
-        } else if (lane == 8) {
-            d_adjoint_grad(gb, Hp, homog, d.mw, d.mh, d.fw, d.fh, col);
-            for (int q = 0; q < 8; ++q) g[q] = 0;
-            for (int q = 0; q < nk; ++q) g[q] = 0.5 * (gf[q] + col[q]);
+        // tangent i through the pull-back: vee(M hat(e_i) M⁻¹)
+        if (tid < nk) {
+            double e[8] = {0, 0, 0, 0, 0, 0, 0, 0}, X[9], t[9];
+            e[tid] = 1;
+            d_hat(e, homog, X);
+            d_mul3(Mw, X, t);
+            d_mul3(t, Mwi, t);
+            d_vee(t, homog, cc[tid]);
         }
-        for (int q = lane; q < 64; q += 32) A[q] = 0;
-        __syncwarp();
-        for (int e = lane; e < nk * nk; e += 32) {
-            const int p = e / nk, q = e % nk;
+        __syncthreads();
+        if (tid < nk * nk) PT[tid] = 0.0 - cc[tid / nk][tid % nk];
+        if (tid >= 64 && tid < 72) {
+            const int q = tid - 64;
+            double o = 0.0;
+            if (q < nk)
+                for (int j = 0; j < nk; ++j) o -= gb[j] * cc[q][j];
+            g[q] = q < nk ? 0.5 * (gf[q] + o) : 0.0;
+        }
+        __syncthreads();
+        if (tid < 64) A[tid] = 0;
+        if (tid < nk * nk) {
+            const int p = tid / nk, q = tid % nk;
             double s2 = 0;
             for (int x = 0; x < nk; ++x)
                 for (int y = 0; y < nk; ++y) s2 += PT[p * nk + x] * Ab[x * nk + y] * PT[q * nk + y];
-            A[p * nk + q] = 0.5 * (Af[p * nk + q] + s2);
+            A[tid] = 0.5 * (Af[tid] + s2);
         }
     }
-    __syncwarp();
-    if (lane == 0) {
-        // the unit ascent direction (src/lie.zig unitAscent)
+    __syncthreads();
+    // the unit ascent direction (src/lie.zig unitAscent); the Gauss–Newton system
+    if (tid == 32) {
         use_ascent = 0;
         for (int q = 0; q < 8; ++q) dv[q] = 0;
         if (amps.n > 0) {
@@ -276,23 +210,63 @@ __global__ void __launch_bounds__(32) k_gn_propose(GnDims d, GnAmps amps, const 
             for (int q = 0; q < nk; ++q) dn += dv[q] * dv[q];
             use_ascent = sqrt(dn) > 1e-12;
         }
-        // the Gauss–Newton step
-        double Am[64], half[8], st8[8];
-        for (int q = 0; q < nk * nk; ++q) Am[q] = A[q];
-        for (int q = 0; q < nk; ++q) Am[q * nk + q] += 1e-4 * fmax(Am[q * nk + q], 1e-12);
-        for (int q = 0; q < nk; ++q) half[q] = 0.5 * g[q];
-        use_step = d_solve_linear(Am, half, nk, st8) ? 1 : 0;
-        for (int q = 0; q < 8; ++q) step[q] = (q < nk && use_step) ? st8[q] : 0;
     }
-    __syncwarp();
-    // the candidates, one lane each: the step ladder along the ascent direction, then the step's
-    // multiples (each capped at a tangent norm of 0.25)
-    if (lane < T) {
+    if (tid < nk * nk) M[tid] = A[tid] + (tid / nk == tid % nk ? 1e-4 * fmax(A[tid], 1e-12) : 0.0);
+    if (tid < nk) rhs[tid] = 0.5 * g[tid];
+    if (tid == 0) use_step = 1;
+    __syncthreads();
+    // M·step = rhs by Gauss–Jordan with partial pivoting (lie.hpp solve_linear); thread (r, c) one entry
+    const int er = tid / nk, ec = tid % nk;
+    for (int k = 0; k < nk; ++k) {
+        if (tid == 0) {
+            int b = k;
+            for (int r = k + 1; r < nk; ++r)
+                if (fabs(M[r * nk + k]) > fabs(M[b * nk + k])) b = r;
+            piv = b;
+        }
+        __syncthreads();
+        const int b = piv;
+        if (b != k) {
+            if (tid < nk) {
+                const double t = M[k * nk + tid];
+                M[k * nk + tid] = M[b * nk + tid];
+                M[b * nk + tid] = t;
+            } else if (tid == 32) {
+                const double t = rhs[k];
+                rhs[k] = rhs[b];
+                rhs[b] = t;
+            }
+            __syncthreads();
+        }
+        const double dk = M[k * nk + k];
+        if (!isfinite(dk) || fabs(dk) < 1e-300) {  // uniform over the block
+            if (tid == 0) use_step = 0;
+            break;
+        }
+        if (tid < nk) fac[tid] = tid == k ? 0.0 : M[tid * nk + k] / dk;
+        __syncthreads();
+        if (tid < nk * nk && er != k && ec >= k && fac[er] != 0) M[er * nk + ec] -= fac[er] * M[k * nk + ec];
+        if (tid >= 64 && tid < 64 + nk && tid - 64 != k && fac[tid - 64] != 0) rhs[tid - 64] -= fac[tid - 64] * rhs[k];
+        __syncthreads();
+    }
+    __syncthreads();
+    if (tid < 8) step[tid] = (tid < nk && use_step) ? rhs[tid] / M[tid * nk + tid] : 0.0;
+    __syncthreads();
+    if (tid == 0 && use_step) {
+        bool fine = true;
+        for (int q = 0; q < nk; ++q) fine = fine && isfinite(step[q]);
+        use_step = fine ? 1 : 0;
+    }
+    __syncthreads();
+    // the candidates: the step ladder along the ascent direction, then the step's multiples (each
+    // capped at a tangent norm of 0.25), as exp(ξ̂) in normalised fixed coordinates (lie.hpp composeN,
+    // expm3: a 13-term Taylor series, scaled and squared)
+    if (tid < T) {
         double x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         bool made = false;
-        if (lane < amps.n) {
+        if (tid < amps.n) {
             if (use_ascent) {
-                for (int k = 0; k < nk; ++k) x[k] = amps.v[lane] * dv[k];
+                for (int k = 0; k < nk; ++k) x[k] = amps.v[tid] * dv[k];
                 made = true;
             }
         } else if (use_step) {
@@ -300,15 +274,56 @@ __global__ void __launch_bounds__(32) k_gn_propose(GnDims d, GnAmps amps, const 
             for (int q = 0; q < nk; ++q) nrm += step[q] * step[q];
             nrm = sqrt(nrm);
             const double mults[5] = {0.5, 1, 2, 4, 8};
-            const double m = mults[lane - amps.n];
+            const double m = mults[tid - amps.n];
             const double sc = m * (nrm * m > 0.25 ? 0.25 / (nrm * m) : 1.0);
             for (int k = 0; k < nk; ++k) x[k] = sc * step[k];
             made = true;
         }
-        if (made) {
-            d_composeN(Hp, x, homog, d.fw, d.fh, Htry + ((size_t)i * T + lane) * 9);
-            ok[lane] = 1;
+        double X[9], nrm = 0;
+        d_hat(x, homog, X);
+        for (int k = 0; k < 9; ++k) nrm = fmax(nrm, fabs(X[k]));
+        int s = 0;
+        for (double v = nrm; v > 0.5 && s < 10; v *= 0.5) ++s;
+        const double sc = ldexp(1.0, -s);
+        for (int k = 0; k < 9; ++k) {
+            B[tid][k] = X[k] * sc;
+            P[tid][k] = E[tid][k] = k % 4 == 0 ? 1.0 : 0.0;
         }
+        sq[tid] = made ? s : -1;
+    }
+    __syncthreads();
+    const int c = tid / 9, e = tid - 9 * c;
+    const bool mine = c < T && sq[c < T ? c : 0] >= 0;
+    for (int k = 1; k < 14; ++k) {
+        const double v = mine ? mul3_at(P[c], B[c], e) / (double)k : 0.0;
+        __syncthreads();
+        if (mine) {
+            P[c][e] = v;
+            E[c][e] += v;
+        }
+        __syncthreads();
+    }
+    for (int k = 0; k < 10; ++k) {
+        const bool go = mine && k < sq[c];
+        if (!__syncthreads_or(go)) break;
+        const double v = go ? mul3_at(E[c], E[c], e) : 0.0;
+        __syncthreads();
+        if (go) E[c][e] = v;
+        __syncthreads();
+    }
+    // Ni E N H, then the group's normal form (projectGroup)
+    if (mine) P[c][e] = mul3_at(Ni, E[c], e);
+    __syncthreads();
+    if (mine) E[c][e] = mul3_at(P[c], N, e);
+    __syncthreads();
+    if (mine) P[c][e] = mul3_at(E[c], Hp, e);
+    __syncthreads();
+    if (mine) {
+        const double w = fabs(P[c][8]) > 1e-12 ? P[c][8] : 1;
+        double v = P[c][e] / w;
+        if (!homog && e >= 6) v = e == 8 ? 1 : 0;
+        Htry[((size_t)i * T + c) * 9 + e] = v;
+        if (e == 0) ok[c] = 1;
     }
 }
 
@@ -351,7 +366,7 @@ cudaError_t gn_propose(const GnDims& d, const GnAmps& amps, const double* H, con
                        unsigned char* valid, cudaStream_t st) {
     if (d.n <= 0) return cudaSuccess;
     if (amps.n < 0 || amps.n > 16 || d.T != amps.n + 5 || d.T > kMaxTry) return cudaErrorInvalidValue;
-    k_gn_propose<<<d.n, 32, 0, st>>>(d, amps, H, sums, score, tsum, active, cur, Htry, valid);
+    k_gn_propose<<<d.n, kProposeThreads, 0, st>>>(d, amps, H, sums, score, tsum, active, cur, Htry, valid);
     return cudaGetLastError();
 }
 

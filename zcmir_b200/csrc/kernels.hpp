@@ -211,22 +211,41 @@ struct PoseRed {
 };
 // doubles of PoseRed::part any pose kernel needs for n poses onto an image of `pixels` pixels
 size_t pose_red_need(size_t pixels, int n);
-// the 45 sums of n poses of one direction (a sampled at H⁻¹x for every b pixel x); hinv: n
-// inverse poses (f32, row-major); sums: n × 45 float64 (zeroed here)
 // The pose kernels' launch shape (zc_tune_parts): pixels per thread, the least and the most
 // blocks per pose (0 keeps the current value). It changes the order of the cross-block sums, so
 // scores move within their float32 rounding.
 void pose_tune(unsigned px_per_thread, unsigned min_blocks, unsigned max_blocks);
-// mask (nullable, n bytes): poses with a zero byte are skipped (their sums stay 0)
-cudaError_t pose_moments(const PoseSide& a, const PoseSide& b, const float* hinv, int n, double* sums, cudaStream_t st,
-                         const PoseFfd& ffd = {}, const unsigned char* mask = nullptr, const PoseRed& red = {});
-// score (float64) and the 102 gradient coefficients (f32) of each pose's sums
+// Poses of a pair scored together: direction 0 samples a at H⁻¹x for every pixel x of b, direction 1
+// (sym) b at Hx for every pixel of a. hinv: n inverse maps (f32, row-major) of direction 0, then n of
+// direction 1, on the device; hinv_host (nullable): the same on the host, which a launch of at most
+// kPoseInline of them carries itself (hinv is then not read). mask (nullable, n bytes): poses with a
+// zero byte are skipped, and what the launch would write of theirs is left as it was.
+constexpr int kPoseInline = 8;
+struct PoseCall {
+    PoseSide a, b;
+    bool sym = false;
+    const float* hinv = nullptr;
+    const float* hinv_host = nullptr;
+    int n = 0;
+    PoseFfd ffd[2] = {};
+    const unsigned char* mask = nullptr;
+    PoseRed red = {};
+};
+// What the launch's last block per row makes of its sums (with PoseRed::part only): score (null: not
+// scored) and coef, and in page-locked memory the sums and the score (each nullable).
+struct PoseScores {
+    bool exact = true;
+    float* coef = nullptr;
+    double *score = nullptr, *host_sums = nullptr, *host_score = nullptr;
+};
+// the 45 sums of each row (n of direction 0, then n of direction 1): rows × 45 float64
+cudaError_t pose_moments(const PoseCall& c, double* sums, const PoseScores& sc, cudaStream_t st);
+// score (float64) and the 102 gradient coefficients (f32) of each row's sums
 cudaError_t pose_coefs(const double* sums, int n, bool exact, float* coef, double* score, cudaStream_t st);
-// tangent sums per pose: 8 gradient + 36 Gauss–Newton (upper triangle) float64 (zeroed here);
-// gens: 8 generators (9 f32 each) in b's pixel coordinates
-cudaError_t pose_tangent(const PoseSide& a, const PoseSide& b, const float* hinv, const float* coef, const float* gens,
-                         int n, bool hess, double* out, cudaStream_t st, const PoseFfd& ffd = {},
-                         const unsigned char* mask = nullptr, const PoseRed& red = {});
+// tangent sums per row: 8 gradient + 36 Gauss–Newton (upper triangle) float64, and in page-locked
+// memory (host, nullable); gens (host): 8 generators of 9 f32 in b's pixels, then 8 in a's
+cudaError_t pose_tangent(const PoseCall& c, const float* coef, const float* gens, bool hess, double* out, double* host,
+                         cudaStream_t st);
 // ── the batched Gauss–Newton refine on the device (gn_device.cu) ──
 struct GnDims {
     int n;        // poses

@@ -7,7 +7,11 @@
 // One direction warps image a (moving) onto image b (fixed): every b pixel x samples a's
 // features bilinearly at H⁻¹(x + 1) − 1, weighted by a 2-px ramp inside a's valid border. Blocks
 // of pose p sum their pixels in float32 per thread, then float64 across the block; the pose's
-// blocks' totals are added in block order by the last of them to finish (block_add).
+// blocks' totals are added in block order by the last of them to finish (block_add). One launch
+// takes both directions of every pose; its last block per pose and direction also scores it, so a
+// pose score is one kernel and its result (with out.host) is written to the caller's page-locked
+// memory by that block: a score of a 256² pair took 88 µs as two moment launches, a one-thread
+// score kernel and four copies.
 #include <array>
 #include <atomic>
 #include <algorithm>
@@ -27,30 +31,32 @@ __device__ __forceinline__ int tri4(int i, int j) {
 }
 
 // The block's k ≤ 48 float64 totals (thread t < k holds total t; the others pass anything) added
-// into out[0 .. k) of this pose. With r.part: every block stores its totals at
-// part[(pose · blocks + block) · k], then the pose's last block to finish (the old value of its
-// ticket is blocks − 1) adds them in a fixed order — group g of ⌊256 / k⌋ threads takes blocks
-// g, g + groups, …, and thread t adds the groups' totals 0, 1, … — and puts the ticket back to
-// 0. Every thread of the block calls it. Without r.part: float64 atomics.
-__device__ void block_add(double s, int k, double* __restrict__ out, const PoseRed& r, int pose) {
-    const int t = threadIdx.x, nblk = gridDim.x;
+// into out[0 .. k) of row `row` (a pose in one direction) of nblk blocks. With r.part: every block
+// stores its totals at part[(row · cap + block) · k], cap the grid's blocks per row, then the row's
+// last block to finish (the old value of its ticket is nblk − 1) adds them in a fixed order — group
+// g of ⌊256 / k⌋ threads takes blocks g, g + groups, …, and thread t adds the groups' totals 0, 1, …
+// — puts the ticket back to 0 and returns true with the totals in tot. Every thread of the block
+// calls it. Without r.part: float64 atomics, and false.
+__device__ bool block_add(double s, int k, double* __restrict__ out, const PoseRed& r, int row, int nblk, double* tot) {
+    const int t = threadIdx.x;
     if (!r.part) {
         if (t < k) atomicAdd(&out[t], s);
-        return;
+        return false;
     }
     __shared__ int last;
     __shared__ double grp[8][48];
-    double* part = r.part + (size_t)pose * nblk * k;
+    double* part = r.part + (size_t)row * gridDim.x * k;
     if (t < k) part[(size_t)blockIdx.x * k + t] = s;
     __threadfence();
     __syncthreads();
-    if (t == 0) last = atomicAdd(&r.ticket[pose], 1u) == (unsigned)(nblk - 1);
+    if (t == 0) last = atomicAdd(&r.ticket[row], 1u) == (unsigned)(nblk - 1);
     __syncthreads();
-    if (!last) return;  // uniform over the block
+    if (!last) return false;  // uniform over the block
     __threadfence();
     const int ng = min((int)blockDim.x / k, 8), g = t / k, e = t - g * k;
     if (g < ng) {
         double a = 0.0;
+#pragma unroll 8
         for (int b = g; b < nblk; b += ng) a += __ldcg(&part[(size_t)b * k + e]);
         grp[g][e] = a;
     }
@@ -58,9 +64,84 @@ __device__ void block_add(double s, int k, double* __restrict__ out, const PoseR
     if (t < k) {
         double a = 0.0;
         for (int q = 0; q < ng; ++q) a += grp[q][t];
-        out[t] = a;
+        out[t] = tot[t] = a;
     }
-    if (t == 0) r.ticket[pose] = 0;
+    if (t == 0) r.ticket[row] = 0;
+    __syncthreads();
+    return true;
+}
+
+// ── pairs of float32 in one 64-bit register: two operations an instruction, each rounded as the
+// scalar one ──
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// The warp's sums of 48 values per lane: each step adds and halves the values a lane still carries
+// (48 shuffles, not 240). Lane l is left with values warp_first(l) .. + 2 in v[0..2] (lanes l and
+// l ^ 1 hold the same).
+__device__ __forceinline__ void warp_sums48(float (&v)[48]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int n = 24, bit = 16; n >= 3; n >>= 1, bit >>= 1)
+#pragma unroll
+        for (int i = 0; i < 24; ++i) {
+            if (i >= n) continue;
+            const bool up = (lane & bit) != 0;
+            const float other = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[n + i], bit);
+            v[i] = (up ? v[n + i] : v[i]) + other;
+        }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 1);
+}
+__device__ __forceinline__ int warp_first(int lane) {
+    return ((lane >> 4) & 1) * 24 + ((lane >> 3) & 1) * 12 + ((lane >> 2) & 1) * 6 + ((lane >> 1) & 1) * 3;
+}
+
+// what a pose launch reads and writes; direction d samples image d at every pixel of image 1 − d
+struct PoseLaunch {
+    const float4* f[2];
+    int w[2], h[2];
+    int n;                 // poses
+    int nblk[2];           // blocks per pose of each direction
+    const float* hinv;     // inverse poses: direction 0's n, then direction 1's
+    PoseFfd ffd[2];
+    const unsigned char* mask;
+    PoseRed rd;
+    double* out;           // rows of totals, direction 0's n then direction 1's
+    double* host;          // the same in page-locked memory (nullable)
+    // moments: the score of each row (scored), its coefficients; tangent: coefficients, generators
+    int scored, exact, hess;
+    float* coef;
+    double *score, *host_score;
+    float gens[144];
+    int n_inl;             // rows of inl in place of hinv (0: none)
+    float inl[9 * kPoseInline];
+};
+
+__device__ __forceinline__ float hinv_at(const PoseLaunch& L, int row, int e) {
+    return L.n_inl ? L.inl[row * 9 + e] : L.hinv[(size_t)row * 9 + e];
 }
 
 // (w, ∂w/∂fx, ∂w/∂fy) of the border taper at (fx, fy) in a w×h image
@@ -142,20 +223,20 @@ __device__ __forceinline__ float2 ffd_disp(const FfdView& f, float xf, float yf,
     return make_float2(dx, dy);
 }
 
-// A grid-stride walk over a w × h image in tiles of 8 × 4 pixels, one tile per warp and step
-// (lane → (lane mod 8, lane / 8)): a warp's 32 pixels are a compact patch, so the bilinear taps
+// A walk of a row's nblk blocks over a w × h image in tiles of 8 × 4 pixels, one tile per warp and
+// step (lane → (lane mod 8, lane / 8)): a warp's 32 pixels are a compact patch, so the bilinear taps
 // they gather on the other image under any rotation fall on few rows (few sectors per load).
 // Tile coordinates are stepped along, not divided out per tile.
 struct TileWalk {
     int T, nt, step, tx, ty, sx, sy, ntx, lx, ly, w, h;
-    __device__ __forceinline__ TileWalk(int w_, int h_) : w(w_), h(h_) {
+    __device__ __forceinline__ TileWalk(int w_, int h_, int nblk) : w(w_), h(h_) {
         ntx = (w + 7) >> 3;
         nt = ntx * ((h + 3) >> 2);
         const int lane = threadIdx.x & 31;
         lx = lane & 7;
         ly = lane >> 3;
         T = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-        step = (int)((gridDim.x * blockDim.x) >> 5);
+        step = (int)((nblk * blockDim.x) >> 5);
         ty = T / ntx;
         tx = T - ty * ntx;
         sy = step / ntx;
@@ -208,221 +289,250 @@ __device__ __forceinline__ bool sample_pos(const float* Hi, const FfdView& f, in
     return !(fx < 2.f || fy < 2.f || fx > (float)aw - 3.f || fy > (float)ah - 3.f);
 }
 
+// scoreFromMoments (src/moments.zig:91-172) in float64 by one warp: the score of the 45 sums st
+// (shared memory) and the 102 coefficients [W 0–15, μ_B 16–19, M̂ 20–35, μ_A 36–39, g = ∂S/∂sums
+// 40–84, Q 85–100, flag] the tangent pass reads (zero when the overlap is under 12 or a whitening
+// fails). Lane 16·h + 4·i + j holds entry (i, j) of the 4 × 4 matrices, half h side A's or B's
+// Gram matrix: a thread of its own took 14 µs over the same steps.
+__device__ __forceinline__ double lane_get(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+
+__device__ void score_warp(const double* st, int exact, double ridge, float* __restrict__ out, double* score,
+                           double* host_score) {
+    const int lane = threadIdx.x & 31, h = lane >> 4, base = h * 16, i = (lane >> 2) & 3, j = lane & 3;
+    auto fail = [&] {
+        for (int k = lane; k < kCoef; k += 32) out[k] = 0.f;
+        if (lane == 0) {
+            *score = 0.0;
+            if (host_score) *host_score = 0.0;
+        }
+    };
+    const double nn = st[0];
+    if (!(nn >= 12.0)) return fail();
+    const double mai = st[1 + i] / nn, maj = st[1 + j] / nn, mbi = st[5 + i] / nn, mbj = st[5 + j] / nn;
+    const double C = st[9 + 4 * i + j] / nn - mai * mbj;
+    // Σ_k a(i, k)·b(k, j), a in half ha and b in half hb; ta, tb: the factor transposed
+    auto mm = [&](double a, int ha, bool ta, double b, int hb, bool tb) {
+        double r = 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            r += lane_get(a, 16 * ha + (ta ? 4 * k + i : 4 * i + k)) * lane_get(b, 16 * hb + (tb ? 4 * j + k : 4 * k + j));
+        return r;
+    };
+    double W = C, MN = 0.0, phi;  // MN: M̂ in half 0, N̂ in half 1
+    if (!exact) {
+        phi = h == 0 ? C * C : 0.0;
+    } else {
+        const int t0 = h ? 35 : 25;
+        double g = st[t0 + tri4(i, j)] / nn - (h ? mbi * mbj : mai * maj);
+        double tr = 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) tr += lane_get(g, base + 5 * k);
+        if (i == j) g += ridge * fmax(tr / 4, 1e-12);
+        // Cholesky by columns; il: the inverse diagonal
+        double L = 0.0, il[4];
+        bool ok = true;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const double piv = lane_get(g, base + 5 * k);
+            ok = ok && piv > 0.0;
+            const double d = sqrt(piv);
+            il[k] = 1.0 / d;
+            const double lik = lane_get(g, base + 4 * i + k) * il[k], ljk = lane_get(g, base + 4 * j + k) * il[k];
+            if (j == k) L = i == k ? d : (i > k ? lik : 0.0);
+            if (i > k && j > k) g -= lik * ljk;
+        }
+        if (!__all_sync(0xffffffffu, ok)) return fail();
+        // column j of the inverse: L y = e_j, Lᵀ x = y
+        double y[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            double v = r == j ? 1.0 : 0.0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const double l = lane_get(L, base + 4 * r + k);
+                if (k < r) v -= l * y[k];
+            }
+            y[r] = v * il[r];
+        }
+#pragma unroll
+        for (int r = 3; r >= 0; --r) {
+            double v = y[r];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const double l = lane_get(L, base + 4 * k + r);
+                if (k > r) v -= l * y[k];
+            }
+            y[r] = v * il[r];
+        }
+        const double Gi = i == 0 ? y[0] : i == 1 ? y[1] : i == 2 ? y[2] : y[3];
+        W = mm(mm(Gi, 0, false, C, 0, false), 0, false, Gi, 1, false);
+        phi = h == 0 ? W * C : 0.0;
+        // M̂ = W Cᵀ G_A⁻¹ (half 0), N̂ = Wᵀ C G_B⁻¹ (half 1)
+        const double u = mm(W, 0, false, C, 0, true), v = mm(W, 0, true, C, 0, false), x = h ? v : u;
+        MN = mm(x, h, false, Gi, h, false);
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) t += lane_get(MN, base + 5 * k);
+        if (i == j) MN += t * ridge / 4;
+    }
+    const double sc = nn * warp_sum(phi);
+    if (!isfinite(sc)) return fail();
+    // g: the feature sums' entries ga (half 0), gb (half 1), and the products'
+    const double wt = lane_get(W, 16 * h + 4 * j + i);  // W(j, i)
+    double gm = h ? -2 * wt * maj + 2 * MN * mbj : -2 * W * mbj + 2 * MN * maj;
+    gm += __shfl_xor_sync(0xffffffffu, gm, 1);
+    gm += __shfl_xor_sync(0xffffffffu, gm, 2);
+    const double gp = -(i == j ? 1.0 : 2.0) * MN;
+    double rest = 0.0;
+    if (j == 0) rest += gm * st[(h ? 5 : 1) + i];
+    if (h == 0) rest += 2 * W * st[9 + 4 * i + j];
+    if (j >= i) rest += gp * st[(h ? 35 : 25) + tri4(i, j)];
+    rest = warp_sum(rest);
+    const double Q = exact ? MN : mm(C, 0, false, C, 0, true);
+    if (h == 0) {
+        out[4 * i + j] = (float)W;
+        out[20 + 4 * i + j] = (float)MN;
+        out[kG0 + 9 + 4 * i + j] = (float)(2 * W);
+        out[kQ0 + 4 * i + j] = (float)Q;
+    }
+    if (j == 0) {
+        out[h ? 16 + i : 36 + i] = (float)(h ? mbi : mai);
+        out[kG0 + (h ? 5 : 1) + i] = (float)gm;
+    }
+    if (j >= i) out[kG0 + (h ? 35 : 25) + tri4(i, j)] = (float)gp;
+    if (lane == 0) {
+        out[kG0] = (float)((sc - rest) / nn);
+        out[kCoef - 1] = 0.f;
+        *score = sc;
+        if (host_score) *host_score = sc;
+    }
+}
+
+// A pixel's sample: its weight, the 2 × 2 taps' features and its own, two features to a register
+// pair as they are loaded.
+struct PoseSample {
+    bool ok;
+    float wt, ax, ay;
+    ulonglong2 v00, v10, v01, v11, vb;
+};
+
 // The 45 sums: 0 Σw, 1–4 Σw a, 5–8 Σw b, 9–24 Σw a_i b_j, 25–34 / 35–44 upper triangles of
-// Σw a aᵀ and Σw b bᵀ.
-template <bool FFD>
-__global__ void __launch_bounds__(256, FFD ? 2 : 3) k_pose_moments(const float4* __restrict__ fa, int aw, int ah,
-                                                      const float4* __restrict__ fb, int bw, int bh,
-                                                      const float* __restrict__ hinv, double* __restrict__ sums,
-                                                      PoseFfd ffd, const unsigned char* __restrict__ mask, PoseRed rd) {
-    __shared__ float Hs[9];
-    __shared__ float red[8][kMom];
+// Σw a aᵀ and Σw b bᵀ. grid: (blocks, poses, directions). Features (0, 1) and (2, 3) go through
+// the interpolation and the products they meet in as pairs (f32x2), the others alone: 39
+// multiply-add instructions a pixel, not 73. U pixels' taps are loaded before the first is added:
+// 1 where the launch fills the GPU (bound by instructions, 60 % of the issue slots at 24 warps an
+// SM), 4 where few blocks are in flight and each waits on its loads. The order of every sum, and so
+// its bits, is the same for any U.
+template <bool FFD, int U>
+__global__ void __launch_bounds__(256, FFD ? 2 : U == 1 ? 3 : 1) k_pose_moments(const __grid_constant__ PoseLaunch L) {
+    __shared__ float red[8][48];
     __shared__ float cps[2 * kFfdMax * kFfdMax];
-    const int pose = blockIdx.y;
-    if (mask && !mask[pose]) return;  // a pose nobody reads (its sums stay 0)
-    if (threadIdx.x < 9) Hs[threadIdx.x] = hinv[pose * 9 + threadIdx.x];
-    const FfdView fv = ffd_view(ffd, cps, pose);
-    __syncthreads();
+    __shared__ double tot[48];
+    const int pose = blockIdx.y, d = blockIdx.z, row = d * L.n + pose, nblk = L.nblk[d];
+    if ((int)blockIdx.x >= nblk || (L.mask && !L.mask[pose])) return;  // a masked pose's sums are read by nobody
+    const float4 *__restrict__ fa = L.f[d], *__restrict__ fb = L.f[1 - d];
+    const int aw = L.w[d], ah = L.h[d], bw = L.w[1 - d], bh = L.h[1 - d];
+    const FfdView fv = ffd_view(L.ffd[d], cps, pose);
     float Hi[9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) Hi[i] = Hs[i];
-    float acc[kMom];
+    for (int i = 0; i < 9; ++i) Hi[i] = hinv_at(L, row, i);
+    if (FFD) __syncthreads();
+    const float xhi = (float)aw - 3.f, yhi = (float)ah - 3.f;
+    float n = 0.f;
+    // a_i b_j as pairs (00,11) (02,13) (20,31) (22,33) and 01 10 03 12 21 30 23 32; a aᵀ and b bᵀ as
+    // (00,11) (02,13) (22,33) and 01 03 12 23
+    f32x2 sa[2] = {0, 0}, sb[2] = {0, 0}, ab[4] = {0, 0, 0, 0}, aa[3] = {0, 0, 0}, bb[3] = {0, 0, 0};
+    float ab1[8] = {0, 0, 0, 0, 0, 0, 0, 0}, aa1[4] = {0, 0, 0, 0}, bb1[4] = {0, 0, 0, 0};
+    TileWalk pw(bw, bh, nblk);
+    while (pw.ok()) {
+        PoseSample q[U];
 #pragma unroll
-    for (int k = 0; k < kMom; ++k) acc[k] = 0.f;
-    for (TileWalk pw(bw, bh); pw.ok(); pw.next()) {
-        if (!pw.in()) continue;
-        const int y = pw.y(), x = pw.x();
-        const size_t t = (size_t)y * bw + x;
-        float fx, fy, Xx, Xy;
-        float3 ph;
-        if (!sample_pos<FFD>(Hi, fv, x, y, aw, ah, bw, bh, fx, fy, ph, Xx, Xy)) continue;
-        float wt, d1, d2;
-        taper(fx, fy, (float)aw, (float)ah, wt, d1, d2);
-        if (wt <= 0.f) continue;
-        const float flx = floorf(fx), fly = floorf(fy);
-        const float ax = fx - flx, ay = fy - fly;
-        const size_t i00 = (size_t)(int)fly * aw + (int)flx;  // fx, fy ≥ 2 here
-        float va[4], vb[4];
-        const Taps4 tp = taps4(fa, i00, aw);
-        const float4 b4 = __ldg(&fb[t]);
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            const float v00 = comp4(tp.v00, p), v10 = comp4(tp.v10, p);
-            const float v01 = comp4(tp.v01, p), v11 = comp4(tp.v11, p);
-            va[p] = (v00 * (1.f - ax) + v10 * ax) * (1.f - ay) + (v01 * (1.f - ax) + v11 * ax) * ay;
-            vb[p] = comp4(b4, p);
-        }
-        acc[0] += wt;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float wa = wt * va[i], wb = wt * vb[i];
-            acc[1 + i] += wa;
-            acc[5 + i] += wb;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[9 + i * 4 + j] += wa * vb[j];
-#pragma unroll
-            for (int j = i; j < 4; ++j) {
-                acc[25 + tri4(i, j)] += wa * va[j];
-                acc[35 + tri4(i, j)] += wb * vb[j];
+        for (int u = 0; u < U; ++u) {
+            q[u].ok = false;
+            if (pw.ok() && pw.in()) {
+                const int y = pw.y(), x = pw.x();
+                float fx, fy, Xx, Xy;
+                float3 ph;
+                if (sample_pos<FFD>(Hi, fv, x, y, aw, ah, bw, bh, fx, fy, ph, Xx, Xy)) {
+                    // the 2-px ramps: (v − 2) / 2 and (hi − v) / 2 clamped to [0, 1]
+                    const float wt = __saturatef(fmaf(fx, 0.5f, -1.f)) * __saturatef((xhi - fx) * 0.5f) *
+                                     (__saturatef(fmaf(fy, 0.5f, -1.f)) * __saturatef((yhi - fy) * 0.5f));
+                    if (wt > 0.f) {
+                        const float flx = floorf(fx), fly = floorf(fy);
+                        q[u].ok = true, q[u].wt = wt, q[u].ax = fx - flx, q[u].ay = fy - fly;
+                        const ulonglong2* p = reinterpret_cast<const ulonglong2*>(fa) + ((int)fly * aw + (int)flx);  // fx, fy ≥ 2
+                        q[u].v00 = __ldg(p), q[u].v10 = __ldg(p + 1), q[u].v01 = __ldg(p + aw), q[u].v11 = __ldg(p + aw + 1);
+                        q[u].vb = __ldg(reinterpret_cast<const ulonglong2*>(fb) + (y * bw + x));
+                    }
+                }
             }
+            if (U > 1 || u == 0) pw.next();
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (!q[u].ok) continue;
+            const PoseSample& s = q[u];
+            const f32x2 x1 = pack2(s.ax, s.ax), x0 = pack2(1.f - s.ax, 1.f - s.ax);
+            const f32x2 y1 = pack2(s.ay, s.ay), y0 = pack2(1.f - s.ay, 1.f - s.ay), w2 = pack2(s.wt, s.wt);
+            const f32x2 a01 = fma2(fma2(s.v00.x, x0, mul2(s.v10.x, x1)), y0, mul2(fma2(s.v01.x, x0, mul2(s.v11.x, x1)), y1));
+            const f32x2 a23 = fma2(fma2(s.v00.y, x0, mul2(s.v10.y, x1)), y0, mul2(fma2(s.v01.y, x0, mul2(s.v11.y, x1)), y1));
+            const f32x2 b01 = s.vb.x, b23 = s.vb.y;
+            const f32x2 wa01 = mul2(a01, w2), wa23 = mul2(a23, w2), wb01 = mul2(b01, w2), wb23 = mul2(b23, w2);
+            float a0, a1, a2, a3, b0, b1, b2, b3, wa0, wa1, wa2, wa3, wb0, wb1, wb2, wb3;
+            unpack2(a01, a0, a1), unpack2(a23, a2, a3), unpack2(b01, b0, b1), unpack2(b23, b2, b3);
+            unpack2(wa01, wa0, wa1), unpack2(wa23, wa2, wa3), unpack2(wb01, wb0, wb1), unpack2(wb23, wb2, wb3);
+            n += s.wt;
+            sa[0] = add2(sa[0], wa01), sa[1] = add2(sa[1], wa23);
+            sb[0] = add2(sb[0], wb01), sb[1] = add2(sb[1], wb23);
+            ab[0] = fma2(wa01, b01, ab[0]), ab[1] = fma2(wa01, b23, ab[1]);
+            ab[2] = fma2(wa23, b01, ab[2]), ab[3] = fma2(wa23, b23, ab[3]);
+            ab1[0] = fmaf(wa0, b1, ab1[0]), ab1[1] = fmaf(wa1, b0, ab1[1]), ab1[2] = fmaf(wa0, b3, ab1[2]);
+            ab1[3] = fmaf(wa1, b2, ab1[3]), ab1[4] = fmaf(wa2, b1, ab1[4]), ab1[5] = fmaf(wa3, b0, ab1[5]);
+            ab1[6] = fmaf(wa2, b3, ab1[6]), ab1[7] = fmaf(wa3, b2, ab1[7]);
+            aa[0] = fma2(wa01, a01, aa[0]), aa[1] = fma2(wa01, a23, aa[1]), aa[2] = fma2(wa23, a23, aa[2]);
+            aa1[0] = fmaf(wa0, a1, aa1[0]), aa1[1] = fmaf(wa0, a3, aa1[1]), aa1[2] = fmaf(wa1, a2, aa1[2]);
+            aa1[3] = fmaf(wa2, a3, aa1[3]);
+            bb[0] = fma2(wb01, b01, bb[0]), bb[1] = fma2(wb01, b23, bb[1]), bb[2] = fma2(wb23, b23, bb[2]);
+            bb1[0] = fmaf(wb0, b1, bb1[0]), bb1[1] = fmaf(wb0, b3, bb1[1]), bb1[2] = fmaf(wb1, b2, bb1[2]);
+            bb1[3] = fmaf(wb2, b3, bb1[3]);
         }
     }
+    float v[48];
+    v[0] = n, v[45] = v[46] = v[47] = 0.f;
+    unpack2(sa[0], v[1], v[2]), unpack2(sa[1], v[3], v[4]);
+    unpack2(sb[0], v[5], v[6]), unpack2(sb[1], v[7], v[8]);
+    unpack2(ab[0], v[9], v[14]), unpack2(ab[1], v[11], v[16]), unpack2(ab[2], v[17], v[22]), unpack2(ab[3], v[19], v[24]);
+    v[10] = ab1[0], v[13] = ab1[1], v[12] = ab1[2], v[15] = ab1[3];
+    v[18] = ab1[4], v[21] = ab1[5], v[20] = ab1[6], v[23] = ab1[7];
+    auto tri = [&](const f32x2(&q)[3], const float(&r)[4], int o) {
+        unpack2(q[0], v[o], v[o + 4]), unpack2(q[1], v[o + 2], v[o + 6]), unpack2(q[2], v[o + 7], v[o + 9]);
+        v[o + 1] = r[0], v[o + 3] = r[1], v[o + 5] = r[2], v[o + 8] = r[3];
+    };
+    tri(aa, aa1, 25), tri(bb, bb1, 35);
+    warp_sums48(v);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if ((lane & 1) == 0)
 #pragma unroll
-    for (int k = 0; k < kMom; ++k) {
-        const float v = warp_sumf(acc[k]);
-        if (lane == 0) red[w][k] = v;
-    }
+        for (int i = 0; i < 3; ++i) red[w][warp_first(lane) + i] = v[i];
     __syncthreads();
     double s = 0.0;
     if (threadIdx.x < kMom)
         for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += (double)red[i][threadIdx.x];
-    block_add(s, kMom, sums + (size_t)pose * kMom, rd, pose);
+    if (!block_add(s, kMom, L.out + (size_t)row * kMom, L.rd, row, nblk, tot)) return;
+    if (L.host && threadIdx.x < kMom) L.host[(size_t)row * kMom + threadIdx.x] = tot[threadIdx.x];
+    if (L.scored && threadIdx.x < 32)
+        score_warp(tot, L.exact, 1e-4, L.coef + (size_t)row * kCoef, L.score + row, L.host_score ? L.host_score + row : nullptr);
 }
 
-// scoreFromMoments (src/moments.zig:91-172) in float64, one thread per pose: the score and the
-// 102 coefficients [W 0–15, μ_B 16–19, M̂ 20–35, μ_A 36–39, g = ∂S/∂sums 40–84, Q 85–100, flag]
-// the tangent pass reads (zero when the overlap is under 12 or a whitening fails).
-__device__ bool chol4(const double* G, double* L) {
-    for (int i = 0; i < 16; ++i) L[i] = 0.0;
-    for (int i = 0; i < 4; ++i)
-        for (int j = 0; j <= i; ++j) {
-            double s = G[i * 4 + j];
-            for (int k = 0; k < j; ++k) s -= L[i * 4 + k] * L[j * 4 + k];
-            if (i == j) {
-                if (!(s > 0.0)) return false;
-                L[i * 5] = sqrt(s);
-            } else {
-                L[i * 4 + j] = s / L[j * 5];
-            }
-        }
-    return true;
-}
-
-__device__ void chol_inv4(const double* L, double* X) {
-    for (int c = 0; c < 4; ++c) {
-        double y[4];
-        for (int i = 0; i < 4; ++i) {
-            double s = (i == c) ? 1.0 : 0.0;
-            for (int k = 0; k < i; ++k) s -= L[i * 4 + k] * y[k];
-            y[i] = s / L[i * 5];
-        }
-        for (int i = 3; i >= 0; --i) {
-            double s = y[i];
-            for (int k = i + 1; k < 4; ++k) s -= L[k * 4 + i] * X[k * 4 + c];
-            X[i * 4 + c] = s / L[i * 5];
-        }
-    }
-}
-
-__device__ void mm4(const double* A, const double* B, double* o) {
-    for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) {
-            double s = 0.0;
-            for (int k = 0; k < 4; ++k) s += A[i * 4 + k] * B[k * 4 + j];
-            o[i * 4 + j] = s;
-        }
-}
-
-__device__ void tr4(const double* A, double* o) {
-    for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) o[i * 4 + j] = A[j * 4 + i];
-}
-
-__global__ void k_pose_coefs(const double* __restrict__ sums, int n, int exact, double ridge, float* __restrict__ coef,
-                             double* __restrict__ score) {
-    const int pose = blockIdx.x * blockDim.x + threadIdx.x;
+// the scores and coefficients of n poses' sums, a warp each
+__global__ void __launch_bounds__(128) k_pose_coefs(const double* __restrict__ sums, int n, int exact, double ridge,
+                                                    float* __restrict__ coef, double* __restrict__ score) {
+    __shared__ double st[4][kMom];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, pose = blockIdx.x * 4 + w;
     if (pose >= n) return;
-    const double* st = sums + pose * kMom;
-    float* out = coef + pose * kCoef;
-    for (int k = 0; k < kCoef; ++k) out[k] = 0.f;
-    score[pose] = 0.0;
-    const double nn = st[0];
-    if (!(nn >= 12.0)) return;
-    double ma[4], mb[4], C[16], W[16], Mh[16] = {0}, Nh[16] = {0};
-    for (int i = 0; i < 4; ++i) {
-        ma[i] = st[1 + i] / nn;
-        mb[i] = st[5 + i] / nn;
-    }
-    for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) C[i * 4 + j] = st[9 + i * 4 + j] / nn - ma[i] * mb[j];
-    for (int i = 0; i < 16; ++i) W[i] = C[i];
-    double phi = 0.0;
-    if (!exact) {
-        for (int i = 0; i < 16; ++i) phi += C[i] * C[i];
-    } else {
-        double GA[16], GB[16], LA[16], LB[16], GAi[16], GBi[16], T[16], U[16];
-        for (int i = 0; i < 4; ++i)
-            for (int j = 0; j < 4; ++j) {
-                GA[i * 4 + j] = st[25 + tri4(i, j)] / nn - ma[i] * ma[j];
-                GB[i * 4 + j] = st[35 + tri4(i, j)] / nn - mb[i] * mb[j];
-            }
-        const double ra = ridge * fmax((GA[0] + GA[5] + GA[10] + GA[15]) / 4, 1e-12);
-        const double rb = ridge * fmax((GB[0] + GB[5] + GB[10] + GB[15]) / 4, 1e-12);
-        for (int i = 0; i < 4; ++i) {
-            GA[i * 5] += ra;
-            GB[i * 5] += rb;
-        }
-        if (!chol4(GA, LA) || !chol4(GB, LB)) return;
-        chol_inv4(LA, GAi);
-        chol_inv4(LB, GBi);
-        mm4(GAi, C, T);
-        mm4(T, GBi, W);
-        for (int i = 0; i < 16; ++i) phi += W[i] * C[i];
-        tr4(C, U);
-        mm4(W, U, T);
-        mm4(T, GAi, Mh);
-        tr4(W, U);
-        mm4(U, C, T);
-        mm4(T, GBi, Nh);
-        const double tm = (Mh[0] + Mh[5] + Mh[10] + Mh[15]) * ridge / 4;
-        const double tn = (Nh[0] + Nh[5] + Nh[10] + Nh[15]) * ridge / 4;
-        for (int i = 0; i < 4; ++i) {
-            Mh[i * 5] += tm;
-            Nh[i * 5] += tn;
-        }
-    }
-    const double sc = nn * phi;
-    if (!isfinite(sc)) return;
-    score[pose] = sc;
-    for (int i = 0; i < 16; ++i) {
-        out[i] = (float)W[i];
-        out[20 + i] = (float)Mh[i];
-    }
-    for (int i = 0; i < 4; ++i) {
-        out[16 + i] = (float)mb[i];
-        out[36 + i] = (float)ma[i];
-    }
-    double g[kMom];
-    for (int k = 0; k < kMom; ++k) g[k] = 0.0;
-    for (int i = 0; i < 4; ++i) {
-        double ga = 0.0, gb = 0.0;
-        for (int j = 0; j < 4; ++j) {
-            ga += -2 * W[i * 4 + j] * mb[j] + 2 * Mh[i * 4 + j] * ma[j];
-            gb += -2 * W[j * 4 + i] * ma[j] + 2 * Nh[i * 4 + j] * mb[j];
-            g[9 + i * 4 + j] = 2 * W[i * 4 + j];
-        }
-        g[1 + i] = ga;
-        g[5 + i] = gb;
-        for (int j = i; j < 4; ++j) {
-            const double f = (i == j) ? 1.0 : 2.0;
-            g[25 + tri4(i, j)] = -f * Mh[i * 4 + j];
-            g[35 + tri4(i, j)] = -f * Nh[i * 4 + j];
-        }
-    }
-    double rest = 0.0;
-    for (int k = 1; k < kMom; ++k) rest += g[k] * st[k];
-    g[0] = (sc - rest) / nn;
-    for (int k = 0; k < kMom; ++k) out[kG0 + k] = (float)g[k];
-    double Q[16];
-    if (exact) {
-        for (int i = 0; i < 16; ++i) Q[i] = Mh[i];
-    } else {
-        double Ct[16];
-        tr4(C, Ct);
-        mm4(C, Ct, Q);
-    }
-    for (int i = 0; i < 16; ++i) out[kQ0 + i] = (float)Q[i];
+    for (int k = lane; k < kMom; k += 32) st[w][k] = sums[(size_t)pose * kMom + k];
+    __syncwarp();
+    score_warp(st[w], exact, ridge, coef + (size_t)pose * kCoef, score + pose, nullptr);
 }
 
 // The gradient over the tangent coordinates and (hess) the Gauss–Newton matrix Σ wt·J_aᵀ Q J_a:
@@ -430,23 +540,22 @@ __global__ void k_pose_coefs(const double* __restrict__ sums, int n, int exact, 
 // needs the two scalars cx, cy = (∂S/∂v_a)·∇v_a plus the taper's boundary term, times each
 // tangent's flow ∂(sample)/∂ξ_k = ((M_k X)·ph.z − ph·(M_k X).z)/ph.z², M_k = −H⁻¹ G_k.
 template <bool FFD>
-__global__ void __launch_bounds__(256) k_pose_tangent(const float4* __restrict__ fa, int aw, int ah,
-                                                      const float4* __restrict__ fb, int bw, int bh,
-                                                      const float* __restrict__ hinv, const float* __restrict__ coef,
-                                                      const float* __restrict__ gens, int hess, double* __restrict__ out,
-                                                      PoseFfd ffd, const unsigned char* __restrict__ mask, PoseRed rd) {
+__global__ void __launch_bounds__(256) k_pose_tangent(const __grid_constant__ PoseLaunch L) {
     __shared__ float Hs[9], Mk[8][9], cf[kCoef];
-    __shared__ float red[8][kGrad];
+    __shared__ float red[8][48];
     __shared__ float cps[2 * kFfdMax * kFfdMax];
-    const int pose = blockIdx.y;
-    if (mask && !mask[pose]) return;  // a pose nobody reads (its sums stay 0)
-    if (threadIdx.x < 9) Hs[threadIdx.x] = hinv[pose * 9 + threadIdx.x];
-    for (int k = threadIdx.x; k < kCoef; k += blockDim.x) cf[k] = coef[pose * kCoef + k];
-    const FfdView fv = ffd_view(ffd, cps, pose);
+    __shared__ double tot[48];
+    const int pose = blockIdx.y, d = blockIdx.z, row = d * L.n + pose, nblk = L.nblk[d], hess = L.hess;
+    if ((int)blockIdx.x >= nblk || (L.mask && !L.mask[pose])) return;  // a masked pose's sums are read by nobody
+    const float4 *__restrict__ fa = L.f[d], *__restrict__ fb = L.f[1 - d];
+    const int aw = L.w[d], ah = L.h[d], bw = L.w[1 - d], bh = L.h[1 - d];
+    if (threadIdx.x < 9) Hs[threadIdx.x] = hinv_at(L, row, threadIdx.x);
+    for (int k = threadIdx.x; k < kCoef; k += blockDim.x) cf[k] = L.coef[(size_t)row * kCoef + k];
+    const FfdView fv = ffd_view(L.ffd[d], cps, pose);
     __syncthreads();
     if (threadIdx.x < 72) {
         const int k = threadIdx.x / 9, e = threadIdx.x % 9, r = e / 3, c = e % 3;
-        const float* G = gens + k * 9;
+        const float* G = L.gens + 72 * d + k * 9;
         Mk[k][e] = -(Hs[r * 3] * G[c] + Hs[r * 3 + 1] * G[3 + c] + Hs[r * 3 + 2] * G[6 + c]);
     }
     __syncthreads();
@@ -457,7 +566,7 @@ __global__ void __launch_bounds__(256) k_pose_tangent(const float4* __restrict__
     float h36[36];
 #pragma unroll
     for (int k = 0; k < 36; ++k) h36[k] = 0.f;
-    for (TileWalk pw(bw, bh); pw.ok(); pw.next()) {
+    for (TileWalk pw(bw, bh, nblk); pw.ok(); pw.next()) {
         if (!pw.in()) continue;
         const int y = pw.y(), x = pw.x();
         const size_t t = (size_t)y * bw + x;
@@ -555,22 +664,22 @@ __global__ void __launch_bounds__(256) k_pose_tangent(const float4* __restrict__
             }
         }
     }
+    float v[48];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = g8[k];
+#pragma unroll
+    for (int k = 0; k < 40; ++k) v[8 + k] = k < 36 ? h36[k < 36 ? k : 0] : 0.f;
+    warp_sums48(v);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if ((lane & 1) == 0)
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const float v = warp_sumf(g8[k]);
-        if (lane == 0) red[w][k] = v;
-    }
-#pragma unroll
-    for (int k = 0; k < 36; ++k) {
-        const float v = warp_sumf(h36[k]);
-        if (lane == 0) red[w][8 + k] = v;
-    }
+        for (int i = 0; i < 3; ++i) red[w][warp_first(lane) + i] = v[i];
     __syncthreads();
     double s = 0.0;
     if (threadIdx.x < kGrad)
         for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += (double)red[i][threadIdx.x];
-    block_add(s, kGrad, out + (size_t)pose * kGrad, rd, pose);
+    if (!block_add(s, kGrad, L.out + (size_t)row * kGrad, L.rd, row, nblk, tot)) return;
+    if (L.host && threadIdx.x < kGrad) L.host[(size_t)row * kGrad + threadIdx.x] = tot[threadIdx.x];
 }
 
 // ∂score/∂(control points cp0 .. cp0 + 15) of pose 0 (smi.wgsl ffd_grad 1275-1417): per valid
@@ -600,7 +709,7 @@ __global__ void __launch_bounds__(256) k_pose_ffd_grad(const float4* __restrict_
     float acc[32];
 #pragma unroll
     for (int k = 0; k < 32; ++k) acc[k] = 0.f;
-    for (TileWalk pw(bw, bh); pw.ok(); pw.next()) {
+    for (TileWalk pw(bw, bh, gridDim.x); pw.ok(); pw.next()) {
         if (!pw.in()) continue;
         const int y = pw.y(), x = pw.x();
         const size_t t = (size_t)y * bw + x;
@@ -695,7 +804,8 @@ __global__ void __launch_bounds__(256) k_pose_ffd_grad(const float4* __restrict_
     double s = 0.0;
     if (threadIdx.x < 32)
         for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += (double)red[i][threadIdx.x];
-    block_add(s, 32, out, rd, 0);
+    __shared__ double tot[48];
+    block_add(s, 32, out, rd, 0, gridDim.x, tot);
 }
 
 // The spline's Gauss–Newton terms of one lattice cell (smi.wgsl ffd_cells 2065-2264): block =
@@ -970,7 +1080,7 @@ cudaError_t interleave_features(const float* feat, int n, float4* out, cudaStrea
 namespace {
 // resident blocks of each pose kernel: moments (spline, plain), tangent (spline, plain), ffd_grad
 const std::array<int, 5>& kernel_slots() {
-    static const std::array<int, 5> sl{pose_slots(k_pose_moments<true>), pose_slots(k_pose_moments<false>),
+    static const std::array<int, 5> sl{pose_slots(k_pose_moments<true, 1>), pose_slots(k_pose_moments<false, 1>),
                                        pose_slots(k_pose_tangent<true>), pose_slots(k_pose_tangent<false>),
                                        pose_slots(k_pose_ffd_grad)};
     return sl;
@@ -987,17 +1097,62 @@ size_t pose_red_need(size_t pixels, int n) {
     return (size_t)std::max(n, 1) * b * kMom;
 }
 
-cudaError_t pose_moments(const PoseSide& a, const PoseSide& b, const float* hinv, int n, double* sums, cudaStream_t st,
-                         const PoseFfd& ffd, const unsigned char* mask, const PoseRed& red) {
-    if (ffd.cps && (ffd.g < 2 || ffd.g > kFfdMax)) return cudaErrorInvalidValue;
-    if (n <= 0) return cudaSuccess;
-    dim3 g(pose_blocks((size_t)b.w * b.h, kernel_slots()[ffd.cps ? 0 : 1]), n);
-    if (!red_fits(red, n, (int)g.x, kMom)) return cudaErrorInvalidValue;
-    cudaMemsetAsync(sums, 0, (size_t)n * kMom * sizeof(double), st);
-    if (ffd.cps)
-        k_pose_moments<true><<<g, 256, 0, st>>>(a.feat4, a.w, a.h, b.feat4, b.w, b.h, hinv, sums, ffd, mask, red);
-    else
-        k_pose_moments<false><<<g, 256, 0, st>>>(a.feat4, a.w, a.h, b.feat4, b.w, b.h, hinv, sums, ffd, mask, red);
+namespace {
+// the launch's images, blocks and poses; rows: poses × directions
+cudaError_t pose_launch(const PoseCall& c, int slot, int k, PoseLaunch& L, dim3& g) {
+    for (const PoseFfd& f : c.ffd)
+        if (f.cps && (f.g < 2 || f.g > kFfdMax)) return cudaErrorInvalidValue;
+    const int nd = c.sym ? 2 : 1;
+    const PoseSide* side[2] = {&c.a, &c.b};
+    g = dim3(1, c.n, nd);
+    for (int d = 0; d < 2; ++d) {
+        L.f[d] = side[d]->feat4, L.w[d] = side[d]->w, L.h[d] = side[d]->h;
+        const PoseSide& dst = *side[1 - d];
+        L.nblk[d] = pose_blocks((size_t)dst.w * dst.h, kernel_slots()[slot]);
+        if (d < nd) g.x = std::max(g.x, (unsigned)L.nblk[d]);
+        L.ffd[d] = c.ffd[d];
+    }
+    if (!red_fits(c.red, nd * c.n, (int)g.x, k)) return cudaErrorInvalidValue;
+    L.n = c.n, L.hinv = c.hinv, L.mask = c.mask, L.rd = c.red;
+    L.n_inl = c.hinv_host && nd * c.n <= kPoseInline ? nd * c.n : 0;
+    for (int i = 0; i < 9 * L.n_inl; ++i) L.inl[i] = c.hinv_host[i];
+    return cudaSuccess;
+}
+}  // namespace
+
+cudaError_t pose_moments(const PoseCall& c, double* sums, const PoseScores& sc, cudaStream_t st) {
+    if (c.n <= 0) return cudaSuccess;
+    const bool ffd = c.ffd[0].cps || c.ffd[1].cps;
+    PoseLaunch L{};
+    dim3 g;
+    cudaError_t e = pose_launch(c, ffd ? 0 : 1, kMom, L, g);
+    if (e != cudaSuccess) return e;
+    L.out = sums, L.host = sc.host_sums;
+    L.scored = sc.score != nullptr && c.red.part, L.exact = sc.exact ? 1 : 0;
+    L.coef = sc.coef, L.score = sc.score, L.host_score = sc.host_score;
+    if (!c.red.part && (e = cudaMemsetAsync(sums, 0, (size_t)g.y * g.z * kMom * sizeof(double), st)) != cudaSuccess) return e;
+    // Launches of fewer blocks than SMs (a pose or two of an ordinary image) keep four pixels' taps in
+    // flight: a 256² pair's score takes 33 µs from call to result, 36 with one. Fuller launches lose
+    // more warps to the registers than they gain (two pixels: 8 % slower).
+    if (ffd) k_pose_moments<true, 1><<<g, 256, 0, st>>>(L);
+    else if ((int)(g.x * g.y * g.z) <= kernel_slots()[1] / 3) k_pose_moments<false, 4><<<g, 256, 0, st>>>(L);
+    else k_pose_moments<false, 1><<<g, 256, 0, st>>>(L);
+    return cudaGetLastError();
+}
+
+cudaError_t pose_tangent(const PoseCall& c, const float* coef, const float* gens, bool hess, double* out, double* host,
+                         cudaStream_t st) {
+    if (c.n <= 0) return cudaSuccess;
+    const bool ffd = c.ffd[0].cps || c.ffd[1].cps;
+    PoseLaunch L{};
+    dim3 g;
+    cudaError_t e = pose_launch(c, ffd ? 2 : 3, kGrad, L, g);
+    if (e != cudaSuccess) return e;
+    L.out = out, L.host = host, L.coef = const_cast<float*>(coef), L.hess = hess ? 1 : 0;
+    for (int i = 0; i < 144; ++i) L.gens[i] = gens[i];
+    if (!c.red.part && (e = cudaMemsetAsync(out, 0, (size_t)g.y * g.z * kGrad * sizeof(double), st)) != cudaSuccess) return e;
+    if (ffd) k_pose_tangent<true><<<g, 256, 0, st>>>(L);
+    else k_pose_tangent<false><<<g, 256, 0, st>>>(L);
     return cudaGetLastError();
 }
 
@@ -1020,24 +1175,8 @@ cudaError_t pose_ffd_grad(const PoseSide& a, const PoseSide& b, const float* hin
 }
 
 cudaError_t pose_coefs(const double* sums, int n, bool exact, float* coef, double* score, cudaStream_t st) {
-    k_pose_coefs<<<(n + 63) / 64, 64, 0, st>>>(sums, n, exact ? 1 : 0, 1e-4, coef, score);
-    return cudaGetLastError();
-}
-
-cudaError_t pose_tangent(const PoseSide& a, const PoseSide& b, const float* hinv, const float* coef, const float* gens,
-                         int n, bool hess, double* out, cudaStream_t st, const PoseFfd& ffd, const unsigned char* mask,
-                         const PoseRed& red) {
-    if (ffd.cps && (ffd.g < 2 || ffd.g > kFfdMax)) return cudaErrorInvalidValue;
     if (n <= 0) return cudaSuccess;
-    dim3 g(pose_blocks((size_t)b.w * b.h, kernel_slots()[ffd.cps ? 2 : 3]), n);
-    if (!red_fits(red, n, (int)g.x, kGrad)) return cudaErrorInvalidValue;
-    cudaMemsetAsync(out, 0, (size_t)n * kGrad * sizeof(double), st);
-    if (ffd.cps)
-        k_pose_tangent<true><<<g, 256, 0, st>>>(a.feat4, a.w, a.h, b.feat4, b.w, b.h, hinv, coef, gens, hess ? 1 : 0, out, ffd,
-                                                mask, red);
-    else
-        k_pose_tangent<false><<<g, 256, 0, st>>>(a.feat4, a.w, a.h, b.feat4, b.w, b.h, hinv, coef, gens, hess ? 1 : 0, out,
-                                                 ffd, mask, red);
+    k_pose_coefs<<<(n + 3) / 4, 128, 0, st>>>(sums, n, exact ? 1 : 0, 1e-4, coef, score);
     return cudaGetLastError();
 }
 

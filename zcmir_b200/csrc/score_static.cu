@@ -140,15 +140,15 @@ bool Engine::score_static(const double* Hs, uint32_t n_poses, double* out3) {
     // The moment sums accumulate with atomics and are the only part of the array that must
     // start at zero: pose_moments clears its n × 45 sums on the stream before accumulating. The
     // inverse poses, coefficients and scores are written in full before they are read.
-    if (!cuda_ok(pose_moments(pa, pb, hinv, n, sums, st), "score_static")) return false;
-    if (sym && !cuda_ok(pose_moments(pb, pa, hinv + (size_t)n * 9, n, sums + (size_t)n * kMom, st), "score_static"))
-        return false;
+    PoseCall pc;
+    pc.a = pa, pc.b = pb, pc.sym = sym, pc.hinv = hinv, pc.n = n;
+    if (!cuda_ok(pose_moments(pc, sums, PoseScores{}, st), "score_static")) return false;
     if (!cuda_ok(pose_coefs(sums, m, exact, coef, score, st), "score_static")) return false;
     double sc[kRows];
     if (!cuda_ok(cudaMemcpyAsync(sc, score, (size_t)m * sizeof(double), cudaMemcpyDeviceToHost, st), "score_static") ||
         !cuda_ok(cudaStreamSynchronize(st), "score_static"))
         return false;
-    counts[0] += (sym ? 2 : 1) + 1;  // launches, submits, reads, waits
+    counts[0] += 2;  // launches, submits, reads, waits
     counts[1]++;
     counts[2]++;
     counts[3]++;
