@@ -87,6 +87,11 @@ int32_t zcb_stack_load(zc_engine* e, uint32_t n, const float* const* images, con
 int32_t zcb_sweep_stack(zc_engine* e, const double H0[9], uint32_t n_peak, float* scores, uint32_t* idx, size_t cap,
                         double* info, size_t info_len, zc_shift_result* stack_out, size_t n_out);
 
+/* zc_set_image_rgba for 8-bit pixels of 1 (gray: R = G = B), 3 (RGB) or 4 (RGBA) interleaved channels,
+ * uploaded as they are: the same image, preprocessing and errors, without expanding it to RGBA8 on the
+ * host first. No counterpart in the reference (its upload takes RGBA8 only, src/exports.zig). 0 / −1. */
+int32_t zcb_set_image_u8(zc_engine* e, uint32_t side, const uint8_t* data, uint32_t w, uint32_t h, uint32_t channels);
+
 /* Scores of n poses (Hs: n row-major 3×3 maps, each as zc_score's H) into out[3n], per pose the
  * mean, forward and inverse score exactly as zc_score writes them, allocating no device memory.
  * No counterpart in the reference (whose only pose score is zc_score, src/exports.zig:417). For
@@ -142,9 +147,11 @@ int32_t zcb_prop_train(float* params, size_t np, const float* x, const int32_t* 
  * linear layer to logits [n][216] (24 rotation × 9 log-scale bins, index 9·r + s). Weights are
  * used rounded to BF16, activations stored in BF16, every product summed in FP32 (mma.sync
  * m16n8k16). params: zcb_cnn_nparams() float32 (W1 [32][3][3][8], b1, W2 [64][3][3][32], b2,
- * W3 [64][3][3][64], b3, W4 [128][3][3][64], b4, Wfc [216][128], bfc). The calls allocate and
- * free their own device memory; 0 / −1 with the message from zcb_cnn_error. */
+ * W3 [64][3][3][64], b3, W4 [128][3][3][64], b4, Wfc [216][128], bfc). The calls take
+ * their device memory from a pool of their own, which keeps at most 64 MB between calls until
+ * zcb_cnn_release gives it back; 0 / −1 with the message from zcb_cnn_error. */
 size_t zcb_cnn_nparams(void);
+void zcb_cnn_release(void);
 size_t zcb_cnn_error(char* buf, size_t cap);
 int32_t zcb_cnn_forward(const float* params, size_t np, const uint16_t* x, uint32_t n, float* logits);
 /* the mean softmax cross-entropy over labels (0..215) of a batch of n ≤ 4096, and its gradient */

@@ -65,6 +65,7 @@ SIGS = {
     "zc_set_image": ([P, U32, f32p, U32, U32], I32),
     "zc_set_image_gray": ([P, U32, f32p, U32, U32, U32], I32),
     "zc_set_image_rgba": ([P, U32, u8p, U32, U32], I32),
+    "zcb_set_image_u8": ([P, U32, u8p, U32, U32, U32], I32),
     "zc_work_image": ([P, U32, f32p, SZ], I32),
     "zc_features": ([P, U32, f32p, SZ], I32),
     "zc_moments": ([P, f64p, f64p], I32),
@@ -107,6 +108,7 @@ SIGS = {
     "zcb_prop_grad": ([f32p, SZ, f32p, ctypes.POINTER(ctypes.c_int32), U32, f32p, f32p], I32),
     "zcb_prop_train": ([f32p, SZ, f32p, ctypes.POINTER(ctypes.c_int32), U32, U32, U32, ctypes.c_float, U32, f32p], I32),
     "zcb_cnn_nparams": ([], SZ),
+    "zcb_cnn_release": ([], None),
     "zcb_cnn_error": ([ctypes.c_char_p, SZ], SZ),
     "zcb_cnn_forward": ([f32p, SZ, ctypes.POINTER(ctypes.c_uint16), U32, f32p], I32),
     "zcb_cnn_grad": ([f32p, SZ, ctypes.POINTER(ctypes.c_uint16), ctypes.POINTER(ctypes.c_int32), U32, f32p, f32p], I32),

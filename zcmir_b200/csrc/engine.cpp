@@ -179,13 +179,14 @@ bool Engine::set_image(int s, const float* data, int w, int h, bool preprocess) 
     return build_side(s);
 }
 
-bool Engine::set_image_rgba(int s, const unsigned char* rgba, int w, int h) {
-    if (s < 0 || s > 1 || w < 8 || h < 8 || !rgba) return fail("set_image_rgba: BadImage");
+bool Engine::set_image_u8(int s, const unsigned char* px, int w, int h, int channels) {
+    if (s < 0 || s > 1 || w < 8 || h < 8 || !px || (channels != 1 && channels != 3 && channels != 4))
+        return fail("set_image_rgba: BadImage");
     Side& sd = side[s];
     const size_t n = (size_t)w * h;
-    if (!cuda_ok(pp_rgba_.ensure(n * 4), "set_image_rgba") || !cuda_ok(sd.raw.ensure(n * 4), "set_image_rgba") ||
-        !cuda_ok(cudaMemcpyAsync(pp_rgba_.p, rgba, n * 4, cudaMemcpyHostToDevice, st), "set_image_rgba") ||
-        !cuda_ok(rgba_to_gray(pp_rgba_.as<unsigned char>(), (int)n, sd.raw.as<float>(), st), "set_image_rgba"))
+    if (!cuda_ok(pp_rgba_.ensure(n * channels), "set_image_rgba") || !cuda_ok(sd.raw.ensure(n * 4), "set_image_rgba") ||
+        !cuda_ok(cudaMemcpyAsync(pp_rgba_.p, px, n * channels, cudaMemcpyHostToDevice, st), "set_image_rgba") ||
+        !cuda_ok(u8_to_gray(pp_rgba_.as<unsigned char>(), (int)n, channels, sd.raw.as<float>(), st), "set_image_rgba"))
         return false;
     counts[0] += 1;
     sd.has = true;

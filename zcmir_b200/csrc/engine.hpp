@@ -208,8 +208,9 @@ class Engine {
 
     // images and features
     bool set_image(int s, const float* data, int w, int h, bool preprocess);
-    // RGBA8 → gray (0.299 R + 0.587 G + 0.114 B), always preprocessed (src/engine.zig:422-426)
-    bool set_image_rgba(int s, const unsigned char* rgba, int w, int h);
+    // 8-bit pixels of 1, 3 or 4 channels → gray (0.299 R + 0.587 G + 0.114 B), always preprocessed
+    // (src/engine.zig:422-426)
+    bool set_image_u8(int s, const unsigned char* px, int w, int h, int channels);
     bool need_images();
     // both sides present and their features built (enqueued) for the current settings; with
     // join, the engine stream also waits for the builds made on a stream of their own

@@ -139,7 +139,11 @@ int32_t zc_set_image(zc_engine* e, uint32_t side, const float* data, uint32_t w,
 }
 
 int32_t zc_set_image_rgba(zc_engine* e, uint32_t side, const uint8_t* data, uint32_t w, uint32_t h) {
-    return guarded(e, "set_image_rgba", [&] { return e->set_image_rgba((int)side, data, (int)w, (int)h); });
+    return guarded(e, "set_image_rgba", [&] { return e->set_image_u8((int)side, data, (int)w, (int)h, 4); });
+}
+
+int32_t zcb_set_image_u8(zc_engine* e, uint32_t side, const uint8_t* data, uint32_t w, uint32_t h, uint32_t channels) {
+    return guarded(e, "set_image_rgba", [&] { return e->set_image_u8((int)side, data, (int)w, (int)h, (int)channels); });
 }
 
 int32_t zc_work_image(zc_engine* e, uint32_t side, float* out, size_t len) {

@@ -150,7 +150,7 @@ cudaError_t sweep_peaks(const float* maps, int nx, int ny, size_t map_stride, in
                         float* ps, uint32_t* pi, cudaStream_t st);
 
 // ── preprocessing (preprocess.cu); with `half` every output is rounded to f16 texels ──
-cudaError_t rgba_to_gray(const unsigned char* rgba, int n, float* gray, cudaStream_t st);
+cudaError_t u8_to_gray(const unsigned char* px, int n, int channels, float* gray, cudaStream_t st);
 size_t clahe_scratch_bytes(int grid, int bins);
 cudaError_t clahe(const float* src, int w, int h, double clip, int bins, int grid, bool half, void* scratch,
                   float* dst, cudaStream_t st);

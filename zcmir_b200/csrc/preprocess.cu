@@ -16,11 +16,21 @@ namespace {
 
 __device__ __forceinline__ float texel(float v, bool half) { return half ? __half2float(__float2half_rn(v)) : v; }
 
-// packed RGBA8 → 0.299 R + 0.587 G + 0.114 B with each channel i/255 rounded to f32
-__global__ void k_rgba_gray(const uchar4* __restrict__ rgba, int n, float* __restrict__ gray) {
+// 8-bit pixels of C channels (1: gray, taken as R = G = B; 3; 4: the fourth ignored) → 0.299 R +
+// 0.587 G + 0.114 B with each channel i/255 rounded to f32. Gray and colour images go up as they are,
+// one to three bytes a pixel, not expanded to four on the host.
+template <int C>
+__global__ void k_u8_gray(const unsigned char* __restrict__ px, int n, float* __restrict__ gray) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uchar4 p = rgba[i];
-        const float r = __fdiv_rn((float)p.x, 255.f), g = __fdiv_rn((float)p.y, 255.f), b = __fdiv_rn((float)p.z, 255.f);
+        unsigned char v[3];
+        if constexpr (C == 4) {
+            const uchar4 p = reinterpret_cast<const uchar4*>(px)[i];
+            v[0] = p.x, v[1] = p.y, v[2] = p.z;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[k] = px[(size_t)i * C + (C == 3 ? k : 0)];
+        }
+        const float r = __fdiv_rn((float)v[0], 255.f), g = __fdiv_rn((float)v[1], 255.f), b = __fdiv_rn((float)v[2], 255.f);
         gray[i] = __fadd_rn(__fadd_rn(__fmul_rn(0.299f, r), __fmul_rn(0.587f, g)), __fmul_rn(0.114f, b));
     }
 }
@@ -187,8 +197,11 @@ int grid1(int n) {
 
 }  // namespace
 
-cudaError_t rgba_to_gray(const unsigned char* rgba, int n, float* gray, cudaStream_t st) {
-    k_rgba_gray<<<grid1(n), 256, 0, st>>>(reinterpret_cast<const uchar4*>(rgba), n, gray);
+cudaError_t u8_to_gray(const unsigned char* px, int n, int channels, float* gray, cudaStream_t st) {
+    if (channels == 1) k_u8_gray<1><<<grid1(n), 256, 0, st>>>(px, n, gray);
+    else if (channels == 3) k_u8_gray<3><<<grid1(n), 256, 0, st>>>(px, n, gray);
+    else if (channels == 4) k_u8_gray<4><<<grid1(n), 256, 0, st>>>(px, n, gray);
+    else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
 

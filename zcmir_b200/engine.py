@@ -229,15 +229,19 @@ class Engine:
 
     # images
     def set_image(self, side, img, preprocess=True):
-        """Side 0 (moving) or 1 (fixed). uint8 images go up as RGBA8, which the engine always
-        preprocesses; anything else as float32 gray, preprocessed (CLAHE / band pass / invert of
+        """Side 0 (moving) or 1 (fixed). uint8 images go up as they are (gray, RGB or RGBA), which the
+        engine always preprocesses; anything else as float32 gray, preprocessed (CLAHE / band pass / invert of
         the settings) when ``preprocess``."""
         a = np.asarray(img)
         if a.dtype == np.uint8:
             if not preprocess:
                 raise ValueError("uint8 images are always preprocessed; pass a float gray image to skip it")
-            px = rgba8(a)
-            self.call("zc_set_image_rgba", side, px.ctypes.data_as(N.u8p), px.shape[1], px.shape[0])
+            if a.ndim == 2:
+                a = a[:, :, None]
+            if a.ndim != 3 or a.shape[2] not in (1, 3, 4):
+                raise ValueError(f"a uint8 image is (h, w), (h, w, 3) or (h, w, 4); got shape {a.shape}")
+            px = np.ascontiguousarray(a)
+            self.call("zcb_set_image_u8", side, px.ctypes.data_as(N.u8p), px.shape[1], px.shape[0], px.shape[2])
             return
         g = gray32(a)
         self.call("zc_set_image_gray", side, _f32(g), g.shape[1], g.shape[0], int(bool(preprocess)))
