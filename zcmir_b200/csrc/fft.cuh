@@ -345,6 +345,20 @@ __host__ __device__ constexpr int line_tl(int n) {
     return tl < 512 ? tl : 512;
 }
 
+// Threads per line of the inverse columns: one group of a pass each where no group has more than 9
+// points (192 = 8·8·3, 576 = 8·8·9) and a line's block stays small, so that 40 registers hold a thread
+// and twice the loads are in flight; else as line_tl. Inverse columns of 192²: 409 → 351 µs, of 576²
+// 27 → 23; of 729² (81 threads) they lost 3 %, of 1536² (192) a third.
+__host__ __device__ constexpr int col_inv_tl(int n) {
+    int most = 0;
+    for (int s = 0; s < mix_stages(n); s += group_len(n, s)) {
+        const int p = radix_prod(n, s, group_len(n, s));
+        if (p > 9) return line_tl(n);
+        if (p > 3 && n / p > most) most = n / p;
+    }
+    return most > 0 && most <= 72 ? most : line_tl(n);
+}
+
 // Stages S .. S + CNT − 1 on the P points v of group k (k = j mod NS), in registers. LO: the
 // points v[t], t ≥ P/2, are zero (the line's upper half; only for an even first radix).
 template <int N, int S, int CNT, int NS, bool INV, bool LO, int P>
@@ -537,6 +551,8 @@ __device__ __forceinline__ void mix_fft_in(float2* __restrict__ buf, const float
 // run_io<INV, LO>(buf, t, act, in, out) (mix_fft_io's contract) and run_in<INV, LO>(buf, t, act,
 // in); LO: the caller guarantees in(y) = 0 for y ≥ n/2, so a compile-time line reads only y < n/2.
 struct GenericLine {
+    static constexpr int kTl = 0, kTx = 0, kRowT = 512;  // kTx 0: tile and threads chosen at the launch
+    __host__ GenericLine inv() const { return *this; }
     LinePlan p;
     __device__ __forceinline__ const GenericLine& fresh() const { return *this; }
     __host__ __device__ __forceinline__ int n() const { return p.n; }
@@ -565,6 +581,12 @@ struct GenericLine {
 // A compile-time line of N = 2^a·3^b points, TPL threads per line.
 template <int N, int TPL = line_tl(N)>
 struct FixedLine {
+    static constexpr int kTl = TPL;
+    static constexpr int kTx = TPL <= 32 ? 16 : TPL <= 48 ? 8 : TPL <= 256 ? 4 : 2;  // columns per block
+    static constexpr int kRowT = 2 * TPL <= 256 ? 256 : 512;                          // threads of a block of rows
+    static constexpr bool kOne = TPL > line_tl(N);                                    // one group of points a thread
+    using Inv = FixedLine<N, col_inv_tl(N)>;                                          // the inverse columns' line
+    __host__ Inv inv() const { return Inv{tw}; }
     const float2* tw;
     // the same line with a twiddle pointer the compiler takes for a new one: a loop over lines then
     // reads its twiddles through L1 each time instead of hoisting dozens of them into spills

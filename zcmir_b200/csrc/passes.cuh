@@ -23,8 +23,8 @@ namespace zc {
 
 // Line pitch of a column tile. Lines of 1024 points and more come in tiles of at most 8 lines
 // (512 threads of N/16) and keep line_pitch's ≡ 4 (mod 16), a compile-time constant for
-// compile-time lines; shorter lines come in wide tiles (the sweep's 192-point columns: 33 lines)
-// whose warps touch 32 lines at one point each, which tile_pitch's odd pitch spreads over all
+// compile-time lines; shorter lines come in wider tiles (the sweep's 192-point columns: 16 lines)
+// whose half-warps touch 16 lines at one point each, which tile_pitch's odd pitch spreads over all
 // bank pairs (≡ 4 put them in 4).
 __host__ __device__ __forceinline__ constexpr int col_pitch(int n, int tx) {
     return n >= 1024 ? line_pitch(n) : tile_pitch(n, tx);
@@ -134,18 +134,23 @@ __global__ void __launch_bounds__(512, 1) k_fwd_rows(const float* __restrict__ g
 // Column FFTs of the half spectra, in place: block = a tile of tx columns of one plane; rows
 // ≥ rows_in read as zero. Thread (column c, line thread t), c fastest, so each load or store of
 // a warp covers 8 rows × 4 adjacent columns (whole 32-byte sectors); the first butterflies read
-// global memory and the last write it (run_io), with only the middle stages in shared memory.
+// global memory and the last write it (run_io), with only the middle stages in shared memory. With
+// npad the planes' columns lie end to end, npad to a plane, and tiles cross from one to the next.
 // LO: rows_in ≤ n/2, so the first butterflies read only rows y < n/2 (the rest are zero).
-template <class F, bool INV, bool LO, int MAXT>
-__global__ void __launch_bounds__(MAXT, 1024 / MAXT) k_cols(float2* __restrict__ half, size_t pstride, int WP, int ncols,
-                                                 int rows_in, F f, int tx) {
+template <class F, bool INV, bool LO, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) k_cols(float2* __restrict__ half, size_t pstride, int WP, int ncols,
+                                                 int npad, int planes, int rows_in, F f, int txr) {
     extern __shared__ float2 smem[];
-    const int x0 = blockIdx.x * tx;
-    float2* base = half + (size_t)blockIdx.y * pstride;
+    const int tx = F::kTx && MINB > 1 ? F::kTx : txr;  // (a constant cost 3072 points 8 %)
     const int pl = col_pitch(f.n(), tx);
-    const int c = threadIdx.x % tx, t = threadIdx.x / tx, col = x0 + c;
-    const bool okc = col < ncols;
-    float2* p = base + col;
+    const int c = threadIdx.x % tx, t = threadIdx.x / tx;
+    int plane = blockIdx.y, col = blockIdx.x * tx + c;
+    if (npad) {
+        plane = col / npad;
+        col -= plane * npad;
+    }
+    const bool okc = plane < planes && col < ncols;
+    float2* p = half + (size_t)(okc ? plane : 0) * pstride + col;
     f.template run_io<INV, LO>(
         smem + c * pl, t, true,
         [&](int y) { return (okc && y < rows_in) ? p[(size_t)y * WP] : make_float2(0.f, 0.f); },
@@ -157,17 +162,22 @@ __global__ void __launch_bounds__(MAXT, 1024 / MAXT) k_cols(float2* __restrict__
 // ── inverse: products and column IFFTs ──────────────────────────────────────────────────────
 
 // block (correlation slot k, column tile, item): P = A·conj(B) on the tile, inverse column FFT
-// → Q; item b reads ha + b·abs, hb + b·bbs and writes Q + b·qbs
-template <class F, int MAXT>
-__global__ void __launch_bounds__(MAXT, 1024 / MAXT) k_inv_cols(const float2* __restrict__ ha, const float2* __restrict__ hb,
-                                                     size_t pstride, int WP, int ncols, CorrPlanDev plan, F f, int tx,
+// → Q; item b reads ha + b·abs, hb + b·bbs and writes Q + b·qbs. npad: as k_cols, over the correlations.
+template <class F, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) k_inv_cols(const float2* __restrict__ ha, const float2* __restrict__ hb,
+                                                     size_t pstride, int WP, int ncols, int npad, CorrPlanDev plan, F f, int txr,
                                                      float2* __restrict__ Q, size_t abs_, size_t bbs, size_t qbs) {
     extern __shared__ float2 smem[];
-    const int k = blockIdx.x;
-    const int x0 = blockIdx.y * tx;
     const size_t item = blockIdx.z;
-    const int c = threadIdx.x % tx, t = threadIdx.x / tx, col = x0 + c;
-    const bool okc = col < ncols;
+    const int tx = F::kTx ? F::kTx : txr;
+    const int c = threadIdx.x % tx, t = threadIdx.x / tx;
+    int k = blockIdx.x, col = blockIdx.y * tx + c;
+    if (npad) {
+        k = (blockIdx.x * tx + c) / npad;
+        col = blockIdx.x * tx + c - k * npad;
+    }
+    const bool okc = k < plan.n_corr && col < ncols;
+    if (!okc) k = 0;
     const float2* A = ha + item * abs_ + (size_t)plan.ca[k] * pstride + col;
     const float2* B = hb + item * bbs + (size_t)plan.cb[k] * pstride + col;
     float2* O = Q + item * qbs + (size_t)k * pstride + col;
@@ -188,10 +198,11 @@ __global__ void __launch_bounds__(MAXT, 1024 / MAXT) k_inv_cols(const float2* __
 // spectrum, conj(Q1) + i·conj(Q2) mirrored above it, its inverse FFT the two real rows, written
 // over Q1's and Q2's row (a row of WP complex holds the nx reals). The task's lines are in one
 // block and every line reads its inputs before the block's first barrier and writes after it, so
-// writing in place is safe. S = 2: two lines of nx/2 points per task, line s the outputs
+// writing in place is safe. Blocks of 256 threads, four per SM (two of 512 left the barriers of whole
+// blocks exposed: rows of 2048 points 169 → 143 µs, 192: 453 → 409). S = 2: two lines of nx/2 points per task, line s the outputs
 // x ≡ s (mod 2) after one decimation-in-frequency step.
 template <class F, int S>
-__global__ void __launch_bounds__(512, 2) k_inv_rows(float2* __restrict__ Q, size_t pstride, int WP, int nx, int ntask,
+__global__ void __launch_bounds__(F::kRowT, 1024 / F::kRowT) k_inv_rows(float2* __restrict__ Q, size_t pstride, int WP, int nx, int ntask,
                                                      int n_corr, F f, int lpb, const float2* __restrict__ tw_nx,
                                                      size_t qbs) {
     extern __shared__ float2 smem[];
@@ -229,8 +240,8 @@ __global__ void __launch_bounds__(512, 2) k_inv_rows(float2* __restrict__ Q, siz
 }
 
 inline int lines_per_block(int tl, int want_threads) { return std::max(1, want_threads / tl); }
-// column tile: as many lines as maxt threads hold (no more than the columns), within the shared
-// memory of 1024 / maxt blocks per SM; whole 32-byte sectors (4 columns) where it can be
+// column tile of a runtime line: as many lines as maxt threads hold (no more than the columns), within
+// the shared memory of 1024 / maxt blocks per SM; whole 32-byte sectors (4 columns) where it can be
 inline int col_tile(int n, int tl, int ncols, int maxt) {
     int tx = std::min(lines_per_block(tl, maxt), ncols);
     const size_t room = (maxt > 512 ? 220 : 110) * 1024;
@@ -240,28 +251,57 @@ inline int col_tile(int n, int tl, int ncols, int maxt) {
     const int tiles = (ncols + tx - 1) / tx;
     return (ncols + tiles - 1) / tiles;
 }
-// Threads of a column block: 512, two blocks per SM, while 4 lines (a 32-byte sector of columns)
-// fit; longer lines take one block of 1024.
-__host__ __device__ constexpr int col_threads(int tl) { return 4 * tl <= 512 ? 512 : 1024; }
 
-template <class F, int MAXT>
-cudaError_t launch_cols(Pass p, F f, const PassArgs& a, cudaStream_t st) {
+// Blocks per SM the column kernels of a compile-time line are compiled for. The passes wait on their
+// loads (2 to 4 blocks of 64-register threads left the schedulers 66 % idle), so the blocks are small
+// (kTx columns) and take the registers that 1152 (forward) or 1280 threads (inverse) per SM leave, 56 or
+// 48 for the 16 points of a thread; 1536 threads (40 registers) spill, except where a thread holds 9
+// points at most (col_inv_tl). Longer lines: two blocks while that is 48 registers (2304 points: 491 →
+// 302 µs; the forward pass of 2592 lost 15 %), else one. Inverse columns of 104 sweep maps of 192²:
+// 600 → 351 µs, 256²: 590 → 390; of a map of 864²: 55 → 49, 1536²: 172 → 136.
+template <class F>
+__host__ __device__ constexpr int col_blocks(bool inverse) {
+    constexpr int T = F::kTx * F::kTl;
+    if (T == 0 || T > (inverse ? 720 : 640)) return 1;
+    if (T > 512) return 2;
+    const int want = !inverse ? 1152 : F::kOne ? 1536 : 1280;
+    return want / T > 0 ? want / T : 1;
+}
+
+template <class F, Pass P, int MAXT, int MINB>
+cudaError_t launch_cols(F f, const PassArgs& a, cudaStream_t st) {
     const MapGeom& g = a.g;
     const size_t pstride = (size_t)g.ny * g.WP;
-    const int tl = f.tl(), ncols = g.nx / 2 + 1, tx = col_tile(g.ny, tl, ncols, MAXT), tiles = (ncols + tx - 1) / tx;
+    const int tl = f.tl(), ncols = g.nx / 2 + 1, tx = F::kTx ? F::kTx : col_tile(g.ny, tl, ncols, MAXT);
+    // short lines: the planes' columns laid end to end, each plane's rounded up to whole sectors (97
+    // columns in tiles of 16 would leave 13 % of the threads idle)
+    const int npad = F::kTx && tl <= 32 ? (ncols + 3) / 4 * 4 : 0, tiles = (ncols + tx - 1) / tx;
     const size_t sm = (size_t)tx * col_pitch(g.ny, tx) * sizeof(float2);
     cudaError_t e;
-    if (p == Pass::FwdCols) {
-        auto k = 2 * g.ch <= g.ny ? k_cols<F, false, true, MAXT> : k_cols<F, false, false, MAXT>;
+    if constexpr (P == Pass::FwdCols) {
+        const int planes = a.plan->n_real * a.batch;
+        auto k = 2 * g.ch <= g.ny ? k_cols<F, false, true, MAXT, MINB> : k_cols<F, false, false, MAXT, MINB>;
         if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
-        k<<<dim3(tiles, a.plan->n_real * a.batch), tx * tl, sm, st>>>(a.half, pstride, g.WP, ncols, g.ch, f, tx);
+        const dim3 grid = npad ? dim3((planes * npad + tx - 1) / tx) : dim3(tiles, planes);
+        k<<<grid, tx * tl, sm, st>>>(a.half, pstride, g.WP, ncols, npad, planes, g.ch, f, tx);
     } else {
-        auto k = k_inv_cols<F, MAXT>;
+        auto k = k_inv_cols<F, MAXT, MINB>;
         if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
-        k<<<dim3(a.plan->n_corr, tiles, a.batch), tx * tl, sm, st>>>(a.half, a.half_b, pstride, g.WP, ncols, *a.plan, f, tx,
-                                                                     a.Q, a.half_stride, a.b_stride, a.q_stride);
+        const dim3 grid = npad ? dim3((a.plan->n_corr * npad + tx - 1) / tx, 1, a.batch) : dim3(a.plan->n_corr, tiles, a.batch);
+        k<<<grid, tx * tl, sm, st>>>(a.half, a.half_b, pstride, g.WP, ncols, npad, *a.plan, f, tx, a.Q, a.half_stride,
+                                     a.b_stride, a.q_stride);
     }
     return cudaGetLastError();
+}
+template <Pass P, class F>
+cudaError_t run_cols(F f, const PassArgs& a, cudaStream_t st) {
+    if constexpr (F::kTx != 0) {
+        constexpr int T = F::kTx * F::kTl, B = col_blocks<F>(P == Pass::InvCols);
+        return launch_cols<F, P, (B > 1 || T <= 512 ? T : 1024), B>(f, a, st);
+    } else {
+        // 512 threads, two blocks per SM, while 4 lines (a 32-byte sector of columns) fit
+        return 4 * f.tl() <= 512 ? launch_cols<F, P, 512, 2>(f, a, st) : launch_cols<F, P, 1024, 1>(f, a, st);
+    }
 }
 
 // One pass over a batch with line policy F.
@@ -285,12 +325,12 @@ cudaError_t run_pass(Pass p, F f, const PassArgs& a, cudaStream_t st) {
                                                        pstride, a.grid_stride, a.half_stride);
         return cudaGetLastError();
     }
-    if (p == Pass::FwdCols || p == Pass::InvCols)
-        return col_threads(tl) == 512 ? launch_cols<F, 512>(p, f, a, st) : launch_cols<F, 1024>(p, f, a, st);
-    // rows: whole tasks (S lines) per block, up to 512 threads
+    if (p == Pass::FwdCols) return run_cols<Pass::FwdCols>(f, a, st);
+    if (p == Pass::InvCols) return run_cols<Pass::InvCols>(f.inv(), a, st);
+    // rows: whole tasks (S lines) per block of up to kRowT threads
     if (a.S != 1 && a.S != 2) return cudaErrorInvalidConfiguration;
-    const int lpb = std::max(a.S, lines_per_block(tl, 512) / a.S * a.S), ntask = g.ny * ((plan.n_corr + 1) / 2);
-    if (lpb * tl > 512) return cudaErrorInvalidConfiguration;
+    const int lpb = std::max(a.S, lines_per_block(tl, F::kRowT) / a.S * a.S), ntask = g.ny * ((plan.n_corr + 1) / 2);
+    if (lpb * tl > F::kRowT) return cudaErrorInvalidConfiguration;
     const size_t sm = (size_t)lpb * padded_len(f.n()) * sizeof(float2);
     auto k = a.S == 1 ? k_inv_rows<F, 1> : k_inv_rows<F, 2>;
     if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
