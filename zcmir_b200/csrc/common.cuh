@@ -18,6 +18,43 @@ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 __device__ __forceinline__ float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 
+// ── pairs of float32 in one 64-bit register: two operations an instruction, each rounded as the
+// scalar one ──
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// ⌊f⌋ and its integer for a pixel coordinate: adding 2²³ rounding down leaves the integer in the low
+// mantissa bits (exact for 0 ≤ f < 2²³), four additions on the full-rate pipes instead of a rounding
+// and a conversion on the quarter-rate one. For any other f (negative, larger, infinite, NaN) the
+// integer, taken as unsigned, is 2²³ or more: the one test i < n, n ≤ 2²³, rejects them all.
+__device__ __forceinline__ unsigned floor_index(float f, float& fl) {
+    const float t = __fadd_rd(f, 8388608.f);
+    fl = __fsub_rn(t, 8388608.f);
+    return __float_as_uint(t) - 0x4B000000u;
+}
+
 // warp sum of a double
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll

@@ -177,8 +177,8 @@ bool Engine::sweep_maps(const Mat3& H0, const SweepGrid& gv, int G, bool exact, 
         if (!c.tw) return fail("sweep: twiddles: out of device memory");
     }
     const size_t fgrid = (size_t)5 * Fx * Fy;
-    const size_t na = (size_t)A.w * A.h, nb = (size_t)B.w * B.h;
-    bool ok = cuda_ok(sw_il_[0].ensure(na * 20), "sweep") && cuda_ok(sw_il_[1].ensure(nb * 20), "sweep") &&
+    bool ok = cuda_ok(sw_il_[0].ensure(sweep_interleaved_bytes(A.w, A.h)), "sweep") &&
+              cuda_ok(sw_il_[1].ensure(sweep_interleaved_bytes(B.w, B.h)), "sweep") &&
               cuda_ok(sw_poses_.ensure(poses.size() * 4), "sweep") && cuda_ok(sw_fgrid_.ensure(fgrid * 4), "sweep") &&
               cuda_ok(sw_fhalf_.ensure(fhalf_max * 8), "sweep") && cuda_ok(sw_grid_.ensure(grid_max * 4), "sweep") &&
               cuda_ok(sw_half_.ensure(half_max * 8), "sweep") && cuda_ok(sw_q_.ensure(q_max * 8), "sweep") &&
@@ -214,8 +214,8 @@ bool Engine::sweep_maps(const Mat3& H0, const SweepGrid& gv, int G, bool exact, 
     // every launch of the sweep's maps, in order; returns the launch count (−1 on an error)
     auto enqueue = [&]() -> int {
         int launches = 0;
-        if (!cuda_ok(sweep_interleave(A.stack.as<float>(), (int)na, sw_il_[0].as<float4>(), st), "sweep") ||
-            !cuda_ok(sweep_interleave(B.stack.as<float>(), (int)nb, sw_il_[1].as<float4>(), st), "sweep") ||
+        if (!cuda_ok(sweep_interleave(A.stack.as<float>(), A.w, A.h, sw_il_[0].as<float4>(), st), "sweep") ||
+            !cuda_ok(sweep_interleave(B.stack.as<float>(), B.w, B.h, sw_il_[1].as<float4>(), st), "sweep") ||
             !cuda_ok(sweep_pack(ilb, B.w, B.h, sw_poses_.as<float>(), nm, 1, Fx, Fy, cv, nullptr, 0, 0, 0, 0,
                                 sw_fgrid_.as<float>(), nullptr, st),
                      "sweep"))

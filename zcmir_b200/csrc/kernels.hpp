@@ -136,9 +136,10 @@ struct SweepCanvas {
     float ox, oy, cell;
     int G;
 };
-// plane-major 5-plane stack of n pixels → n float4 (w, w f0, w f1, w f2) followed by the fifth
-// plane (w f3) as n floats: 20 bytes per pixel
-cudaError_t sweep_interleave(const float* stack, int n, float4* il, cudaStream_t st);
+// plane-major 5-plane stack of w × h pixels → float4 (w, w f0, w f1, w f2) followed by the fifth
+// plane (w f3) as floats, in tiles: sweep_interleaved_bytes of them
+size_t sweep_interleaved_bytes(int w, int h);
+cudaError_t sweep_interleave(const float* stack, int w, int h, float4* il, cudaStream_t st);
 // the windows [batch][5][win_y][win_x] of slots slot0.. (poses: 12 floats per slot: dest →
 // source map, taps, first window cell); with fw (the fixed window's weights, [Fy][Fx] at cell
 // (fx0, fy0)) each item's zero-lag overlap into n0[batch] (cleared here)

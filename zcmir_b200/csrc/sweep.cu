@@ -9,95 +9,127 @@
 namespace zc {
 namespace {
 
-// plane-major [5][n] → n float4 (w, w f0, w f1, w f2), then the fifth plane (w f3) as n floats:
-// a bilinear tap is one 16-byte load per corner plus a scalar from a plane eight pixels to a
-// sector (sweep.wgsl interleave)
-__global__ void k_interleave(const float* __restrict__ stack, int n, float4* __restrict__ il) {
-    float* p4 = reinterpret_cast<float*>(il + n);
+// The stacks as the taps read them: pixels (w, w f0, w f1, w f2) as float4, then w f3 as floats, both
+// in tiles of 4 × 2 pixels (a 128-byte line of the first, a 32-byte sector of the second). A tap's
+// lanes follow a turned line through the image; in rows of pixels each lane of a steep one is in a
+// line of its own, and the lines per load, not the bytes, bound the pass (L1 84 % busy, 37 % of the
+// issue slots). 3240 poses of a 512² pair: 10.25 ms in rows with cells straddling passes, 8.6 in whole
+// passes and paired products, 7.3 in tiles; gathering the four f3 of a tap in one load as well gave 2 %
+// for 60 % more memory. Pixel (x, y) is at
+// tile_x(x) + tile_y(y, row), row = 8 · tiles across; pixels past the image's edge are never read.
+__host__ __device__ __forceinline__ constexpr unsigned tile_row(int w) { return ((unsigned)w + 3) / 4 * 8; }
+__host__ __device__ __forceinline__ constexpr size_t tile_cells(int w, int h) { return (size_t)tile_row(w) * (((unsigned)h + 1) / 2); }
+__device__ __forceinline__ unsigned tile_x(unsigned x) { return x + (x & ~3u); }
+__device__ __forceinline__ unsigned tile_y(unsigned y, unsigned row) { return 4 * y + (y >> 1) * (row - 8); }
+
+__global__ void k_interleave(const float* __restrict__ stack, int w, int h, float4* __restrict__ il) {
+    const int n = w * h;
+    float* p4 = reinterpret_cast<float*>(il + tile_cells(w, h));
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        il[i] = make_float4(stack[i], stack[(size_t)n + i], stack[2 * (size_t)n + i], stack[3 * (size_t)n + i]);
-        p4[i] = stack[4 * (size_t)n + i];
+        const int y = i / w;
+        const unsigned o = tile_x(i - y * w) + tile_y(y, tile_row(w));
+        il[o] = make_float4(stack[i], stack[(size_t)n + i], stack[2 * (size_t)n + i], stack[3 * (size_t)n + i]);
+        p4[o] = stack[4 * (size_t)n + i];
     }
 }
 
-// Warp w of a block takes the 32 cells x0 .. x0 + 31 of row y of item z's window; the item's
-// pose is poses[(slot0 + z)·12 ..]: the dest → source map (row-major 3×3, 1-based pixels), taps
-// per side, the window's first canvas cell. The cell's value is the mean of k×k bilinear taps of
-// the source stack at the cell's sub-points (sweep.wgsl tap, pack_sweep); a tap whose 2×2
-// footprint leaves the image adds nothing. Cells past the G×G canvas are zero. Output plane-major
-// [5][win_y][win_x] per item. The taps run across the lanes: in each pass, groups of k lanes take
-// ⌊32/k⌋ cells, lane (g, tx) summing tap column tx of its cell over the k tap rows, so adjacent
-// lanes read adjacent pixels (one cache line serves several lanes) instead of pixels a cell apart;
-// each group's k column sums are then added across its lanes and handed to the lane that owns
-// the cell. With fixed weights fw ([Fy][Fx], the fixed window at canvas cell (fx0, fy0)) the
-// item's zero-lag overlap Σ w_moving · w_fixed over the cells both windows cover accumulates into
-// n0[z] (sweep.wgsl zero_lag reads the same value off the correlation of the weight planes).
-__global__ void __launch_bounds__(256) k_sweep_pack(const float4* __restrict__ il, int sw, int sh,
-                                                    const float* __restrict__ poses, int slot0, int win_x, int win_y,
-                                                    SweepCanvas cv, const float* __restrict__ fw, int fx0, int fy0,
-                                                    int Fx, int Fy, float* __restrict__ grid, double* __restrict__ n0) {
-    const int lane = threadIdx.x & 31;
-    const int x0 = blockIdx.x * 32, y = blockIdx.y * 8 + (threadIdx.x >> 5), z = blockIdx.z;
-    const float* P = poses + (size_t)(slot0 + z) * 12;
-    const int cy = (int)P[11] + y;
-    const int x = x0 + lane;
-    const bool in_win = x < win_x && y < win_y;
-    const int k = min(max((int)P[9], 1), 32), cpw = 32 / k;
-    const float* p4 = reinterpret_cast<const float*>(il + (size_t)sw * sh);  // the fifth plane
+constexpr int kPackTaps = 6;  // the most taps per side that a sweep's cells take
+// cells of a strip of k taps per side: whole passes of ⌊32/k⌋ cells
+__host__ __device__ constexpr int pack_strip(int k) { return 32 / (32 / k) * (32 / k); }
+
+// The K×K taps of a strip of W = pack_strip(K) cells (30 or 32) of a window's row, cells xw0 .. of canvas row cy;
+// lane L < W returns cell xw0 + L's sums in s. The taps run across the lanes: in each pass, groups of
+// K lanes take ⌊32/K⌋ cells, lane (g, tx) summing tap column tx of its cell over the K tap rows, so
+// adjacent lanes read adjacent pixels (one cache line serves several lanes) instead of pixels a cell
+// apart; the lane that owns a cell then adds its group's K column sums.
+template <int K>
+__device__ __forceinline__ void pack_cells(float (&s)[5], const float4* __restrict__ il, int sw, int sh, const float* P,
+                                           const SweepCanvas& cv, int xw0, int win_x, int cy, int lane) {
+    constexpr int CPW = 32 / K;
+    const ulonglong2* u = reinterpret_cast<const ulonglong2*>(il);
+    const float* p4 = reinterpret_cast<const float*>(il + tile_cells(sw, sh));  // the fifth plane
+    const unsigned row = tile_row(sw);
     const float h0 = P[0], h1 = P[1], h2 = P[2], h3 = P[3], h4 = P[4], h5 = P[5], h6 = P[6], h7 = P[7], h8 = P[8];
-    const float inv = 1.f / (float)(k * k);
-    const int grp = lane / k, tx = lane - grp * k;
-    float s[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int c0 = 0; c0 < 32; c0 += cpw) {
-        const int xw = x0 + c0 + grp, cx = (int)P[10] + xw;
-        const bool act = grp < cpw && c0 + grp < 32 && xw < win_x && y < win_y && cx < cv.G && cy < cv.G;
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool affine = h6 == 0.f && h7 == 0.f && h8 == 1.f;  // qz is 1 then
+    const float inv = 1.f / (float)(K * K);
+    const int grp = lane / K, tx = lane - grp * K, cx0 = (int)P[10] + xw0;
+    const unsigned wlim = (unsigned)(sw - 1), hlim = (unsigned)(sh - 1);
+#pragma unroll 1
+    for (int c0 = 0; c0 < pack_strip(K) && xw0 + c0 < win_x; c0 += CPW) {
+        const int xw = xw0 + c0 + grp, cx = cx0 + c0 + grp;
+        f32x2 a01 = 0, a23 = 0;
         float a4 = 0.f;
-        if (act) {
-            const float px = cv.ox + ((float)cx + ((float)tx + 0.5f) / (float)k) * cv.cell;
-            for (int ty = 0; ty < k; ++ty) {
-                const float py = cv.oy + ((float)cy + ((float)ty + 0.5f) / (float)k) * cv.cell;
-                const float qx = h0 * px + h1 * py + h2;
-                const float qy = h3 * px + h4 * py + h5;
-                const float qz = h6 * px + h7 * py + h8;
-                if (fabsf(qz) < 1e-8f) continue;
-                // affine poses (qz = 1): the division is exact, skip it
-                const float fx = (qz == 1.f ? qx : qx / qz) - 1.0f, fy = (qz == 1.f ? qy : qy / qz) - 1.0f;
-                const float flx = floorf(fx), fly = floorf(fy);
-                // x0 ≥ 0 and x0 + 1 < w (NaN fails both), before any float → int conversion
-                if (!(flx >= 0.f && fly >= 0.f && flx < (float)(sw - 1) && fly < (float)(sh - 1))) continue;
-                const int ix = (int)flx, iy = (int)fly;
+        if (grp < CPW && xw < win_x && cx < cv.G && cy < cv.G) {
+            const float px = cv.ox + ((float)cx + ((float)tx + 0.5f) / (float)K) * cv.cell;
+#pragma unroll
+            for (int ty = 0; ty < K; ++ty) {
+                const float py = cv.oy + ((float)cy + ((float)ty + 0.5f) / (float)K) * cv.cell;
+                float qx = h0 * px + h1 * py + h2;
+                float qy = h3 * px + h4 * py + h5;
+                if (!affine) {
+                    const float qz = h6 * px + h7 * py + h8;
+                    if (fabsf(qz) < 1e-8f) continue;
+                    if (qz != 1.f) qx = qx / qz, qy = qy / qz;
+                }
+                const float fx = qx - 1.0f, fy = qy - 1.0f;
+                float flx, fly;
+                const unsigned ix = floor_index(fx, flx), iy = floor_index(fy, fly);
+                if (ix >= wlim || iy >= hlim) continue;  // x0 ≥ 0 and x0 + 1 < w
                 const float ax = fx - flx, ay = fy - fly;
                 const float w00 = (1.f - ax) * (1.f - ay), w10 = ax * (1.f - ay), w01 = (1.f - ax) * ay, w11 = ax * ay;
-                const size_t i00 = (size_t)iy * sw + ix, i01 = i00 + sw;
-                const float4 p00 = __ldg(&il[i00]), p10 = __ldg(&il[i00 + 1]);
-                const float4 p01 = __ldg(&il[i01]), p11 = __ldg(&il[i01 + 1]);
-                a.x += w00 * p00.x + w10 * p10.x + w01 * p01.x + w11 * p11.x;
-                a.y += w00 * p00.y + w10 * p10.y + w01 * p01.y + w11 * p11.y;
-                a.z += w00 * p00.z + w10 * p10.z + w01 * p01.z + w11 * p11.z;
-                a.w += w00 * p00.w + w10 * p10.w + w01 * p01.w + w11 * p11.w;
-                a4 += w00 * __ldg(&p4[i00]) + w10 * __ldg(&p4[i00 + 1]) + w01 * __ldg(&p4[i01]) +
-                      w11 * __ldg(&p4[i01 + 1]);
+                const unsigned X0 = tile_x(ix), X1 = tile_x(ix + 1), Y0 = tile_y(iy, row), Y1 = tile_y(iy + 1, row);
+                const unsigned i00 = X0 + Y0, i10 = X1 + Y0, i01 = X0 + Y1, i11 = X1 + Y1;
+                const ulonglong2 p00 = __ldg(u + i00), p10 = __ldg(u + i10), p01 = __ldg(u + i01), p11 = __ldg(u + i11);
+                const f32x2 v00 = pack2(w00, w00), v10 = pack2(w10, w10), v01 = pack2(w01, w01), v11 = pack2(w11, w11);
+                a01 = add2(a01, fma2(v11, p11.x, fma2(v01, p01.x, fma2(v00, p00.x, mul2(v10, p10.x)))));
+                a23 = add2(a23, fma2(v11, p11.y, fma2(v01, p01.y, fma2(v00, p00.y, mul2(v10, p10.y)))));
+                a4 += w00 * __ldg(&p4[i00]) + w10 * __ldg(&p4[i10]) + w01 * __ldg(&p4[i01]) + w11 * __ldg(&p4[i11]);
             }
         }
-        // the group's k column sums, added in every lane of the group (k is the same for the warp)
-        float t[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int j = 0; j < k; ++j) {
-            const int src = min(grp * k + j, 31);
-            t[0] += __shfl_sync(0xffffffffu, a.x, src);
-            t[1] += __shfl_sync(0xffffffffu, a.y, src);
-            t[2] += __shfl_sync(0xffffffffu, a.z, src);
-            t[3] += __shfl_sync(0xffffffffu, a.w, src);
-            t[4] += __shfl_sync(0xffffffffu, a4, src);
-        }
-        // lane L owns strip cell L: this pass holds it when c0 ≤ L < c0 + cpw, in group L − c0
-        const int mine = lane - c0;
-        const bool here = mine >= 0 && mine < cpw;
-        const int src = here ? mine * k : 0;
+        float a[5];
+        unpack2(a01, a[0], a[1]);
+        unpack2(a23, a[2], a[3]);
+        a[4] = a4;
+        // lane L owns cell L of the strip: this pass holds it when c0 ≤ L < c0 + CPW, in group L − c0
+        const bool here = lane >= c0 && lane < c0 + CPW;
+        const int src = here ? (lane - c0) * K : 0;
 #pragma unroll
         for (int p = 0; p < 5; ++p) {
-            const float v = __shfl_sync(0xffffffffu, t[p], src);
-            if (here) s[p] = v * inv;
+            float t = 0.f;
+#pragma unroll
+            for (int j = 0; j < K; ++j) t += __shfl_sync(0xffffffffu, a[p], src + j);
+            if (here) s[p] = t * inv;
+        }
+    }
+}
+
+// Warp w of a block takes a strip of the cells (30 or 32) of row y of item z's window; the item's
+// pose is poses[(slot0 + z)·12 ..]: the dest → source map (row-major 3×3, 1-based pixels), taps per
+// side (1 to 6), the window's first canvas cell. The cell's value is the mean of k×k bilinear taps of
+// the source stack at the cell's sub-points (sweep.wgsl tap, pack_sweep); a tap whose 2×2
+// footprint leaves the image adds nothing. Cells past the G×G canvas are zero. Output plane-major
+// [5][win_y][win_x] per item. With fixed weights fw ([Fy][Fx], the fixed window at canvas cell
+// (fx0, fy0)) the item's zero-lag overlap Σ w_moving · w_fixed over the cells both windows cover
+// accumulates into n0[z] (sweep.wgsl zero_lag reads the same value off the correlation of the weight planes).
+__global__ void __launch_bounds__(256, 4) k_sweep_pack(const float4* __restrict__ il, int sw, int sh,
+                                                       const float* __restrict__ poses, int slot0, int win_x, int win_y,
+                                                       SweepCanvas cv, const float* __restrict__ fw, int fx0, int fy0,
+                                                       int Fx, int Fy, float* __restrict__ grid, double* __restrict__ n0) {
+    const int lane = threadIdx.x & 31;
+    const int y = blockIdx.y * 8 + (threadIdx.x >> 5), z = blockIdx.z;
+    const float* P = poses + (size_t)(slot0 + z) * 12;
+    const int cy = (int)P[11] + y, k = min(max((int)P[9], 1), kPackTaps);
+    const int strip = pack_strip(k), x0 = blockIdx.x * strip, x = x0 + lane;
+    const bool in_win = lane < strip && x < win_x && y < win_y;
+    float s[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    if (y < win_y) {
+        switch (k) {
+            case 1: pack_cells<1>(s, il, sw, sh, P, cv, x0, win_x, cy, lane); break;
+            case 2: pack_cells<2>(s, il, sw, sh, P, cv, x0, win_x, cy, lane); break;
+            case 3: pack_cells<3>(s, il, sw, sh, P, cv, x0, win_x, cy, lane); break;
+            case 4: pack_cells<4>(s, il, sw, sh, P, cv, x0, win_x, cy, lane); break;
+            case 5: pack_cells<5>(s, il, sw, sh, P, cv, x0, win_x, cy, lane); break;
+            default: pack_cells<6>(s, il, sw, sh, P, cv, x0, win_x, cy, lane); break;
         }
     }
     if (in_win) {
@@ -199,10 +231,12 @@ __global__ void __launch_bounds__(1024) k_sweep_peaks(const float* __restrict__ 
 
 }  // namespace
 
-cudaError_t sweep_interleave(const float* stack, int n, float4* il, cudaStream_t st) {
-    int blocks = (n + 255) / 256;
+size_t sweep_interleaved_bytes(int w, int h) { return tile_cells(w, h) * 20; }
+
+cudaError_t sweep_interleave(const float* stack, int w, int h, float4* il, cudaStream_t st) {
+    int blocks = (w * h + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    k_interleave<<<blocks, 256, 0, st>>>(stack, n, il);
+    k_interleave<<<blocks, 256, 0, st>>>(stack, w, h, il);
     return cudaGetLastError();
 }
 
@@ -213,7 +247,7 @@ cudaError_t sweep_pack(const float4* il, int sw, int sh, const float* poses, int
         const cudaError_t e = cudaMemsetAsync(n0, 0, (size_t)batch * sizeof(double), st);
         if (e != cudaSuccess) return e;
     }
-    dim3 g((win_x + 31) / 32, (win_y + 7) / 8, batch);
+    dim3 g((win_x + 29) / 30, (win_y + 7) / 8, batch);  // strips of 30 cells at least
     k_sweep_pack<<<g, 256, 0, st>>>(il, sw, sh, poses, slot0, win_x, win_y, cv, fw, fx0, fy0, Fx, Fy, grid, n0);
     return cudaGetLastError();
 }
