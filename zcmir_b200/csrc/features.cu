@@ -208,27 +208,28 @@ __global__ void k_whiten(float* __restrict__ feat, int n, const float* __restric
 // Autocorrelation partial sums (smi.wgsl:935-975): one block per 32×32 tile with an 8-px halo in
 // shared memory (zero outside the image, so a pair with either pixel outside adds nothing and
 // every lag sums exactly the pairs inside the image). A lag and its negative sum the same pairs, so
-// only the 153 lags with dy ≥ 0 are formed (the negative ones mirrored at the end): half the
-// multiply-adds that bound the kernel (1024²: 120 → 65 µs). Register-blocked: thread (plane p, row
-// lag dy, row group g) takes the tile rows g, g + 8, …, and for each holds the row (32 values) and
-// its partner row at dy with the column halo (48 values) in registers, then accumulates all 17
-// column lags (544 FMAs per 20 vector shared loads). The row groups' f32 sums are added in shared
+// only the 153 lags with dy ≥ 0 are formed (the negative ones mirrored at the end). Register-blocked:
+// thread (plane p, row lag dy, row group g) takes the tile rows g, g + 8, …, and walks each in steps of
+// 8 columns with their 8 values and the 24 of the partner row at dy that the 17 column lags pair them
+// with in registers, 16 of which the next step keeps (544 FMAs per 20 vector shared loads). Rows are
+// 52 floats apart: at 48 the 8 rows that a quarter of a warp reads lay in two groups of banks and the
+// loads, not the FMAs, bound the kernel (1024 × 768: 43 → 30 µs, with the columns taken in steps). The row groups' f32 sums are added in shared
 // memory; partials [tile][153][4].
 constexpr int kAcfTile = 32, kAcfHalo = 8, kAcfSpan = kAcfTile + 2 * kAcfHalo, kAcfHigh = kAcfTile + kAcfHalo, kAcfGroups = 8;
 constexpr int kAcfThreads = 4 * 9 * kAcfGroups;  // 288
-constexpr int kAcfPlane = kAcfHigh * kAcfSpan;
+constexpr int kAcfPitch = kAcfSpan + 4, kAcfPlane = kAcfHigh * kAcfPitch;
 
 __global__ void __launch_bounds__(kAcfThreads) k_acf(const float* __restrict__ feat, int w, int h,
                                                      float* __restrict__ part) {
     __shared__ __align__(16) float sh[4 * kAcfPlane];
     const int x0 = blockIdx.x * kAcfTile, y0 = blockIdx.y * kAcfTile;
     const size_t n = (size_t)w * h;
-    for (int k = threadIdx.x; k < kAcfPlane; k += blockDim.x) {
-        const int gx = x0 - kAcfHalo + k % kAcfSpan, gy = y0 + k / kAcfSpan;
+    for (int k = threadIdx.x; k < kAcfHigh * kAcfSpan; k += blockDim.x) {
+        const int x = k % kAcfSpan, y = k / kAcfSpan, gx = x0 - kAcfHalo + x, gy = y0 + y;
         const bool in = gx >= 0 && gx < w && gy < h;
         const size_t i = in ? (size_t)gy * w + gx : 0;
 #pragma unroll
-        for (int p = 0; p < 4; ++p) sh[p * kAcfPlane + k] = in ? feat[p * n + i] : 0.0f;
+        for (int p = 0; p < 4; ++p) sh[p * kAcfPlane + y * kAcfPitch + x] = in ? feat[p * n + i] : 0.0f;
     }
     __syncthreads();
     const int g = threadIdx.x % kAcfGroups, dy = (threadIdx.x / kAcfGroups) % 9, p = threadIdx.x / (kAcfGroups * 9);
@@ -237,23 +238,23 @@ __global__ void __launch_bounds__(kAcfThreads) k_acf(const float* __restrict__ f
 #pragma unroll
     for (int d = 0; d < 17; ++d) acc[d] = 0.f;
     for (int ty = g; ty < kAcfTile; ty += kAcfGroups) {
-        float a[32], b[48];
-        const float4* ar = reinterpret_cast<const float4*>(pl + ty * kAcfSpan + kAcfHalo);
-        const float4* br = reinterpret_cast<const float4*>(pl + (ty + dy) * kAcfSpan);
+        const float4* ar = reinterpret_cast<const float4*>(pl + ty * kAcfPitch + kAcfHalo);
+        const float4* br = reinterpret_cast<const float4*>(pl + (ty + dy) * kAcfPitch);
+        auto take = [](float* to, const float4& v) { to[0] = v.x, to[1] = v.y, to[2] = v.z, to[3] = v.w; };
+        float a[8], b[24];  // columns x .. x + 7; partner columns x − 8 .. x + 15
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const float4 v = ar[q];
-            a[4 * q] = v.x, a[4 * q + 1] = v.y, a[4 * q + 2] = v.z, a[4 * q + 3] = v.w;
+        for (int q = 0; q < 4; ++q) take(b + 4 * q, br[q]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            take(a, ar[2 * c]), take(a + 4, ar[2 * c + 1]);
+            take(b + 16, br[4 + 2 * c]), take(b + 20, br[5 + 2 * c]);
+#pragma unroll
+            for (int x = 0; x < 8; ++x)
+#pragma unroll
+                for (int d = 0; d < 17; ++d) acc[d] = fmaf(a[x], b[x + d], acc[d]);
+#pragma unroll
+            for (int x = 0; x < 16; ++x) b[x] = b[x + 8];
         }
-#pragma unroll
-        for (int q = 0; q < 12; ++q) {
-            const float4 v = br[q];
-            b[4 * q] = v.x, b[4 * q + 1] = v.y, b[4 * q + 2] = v.z, b[4 * q + 3] = v.w;
-        }
-#pragma unroll
-        for (int d = 0; d < 17; ++d)
-#pragma unroll
-            for (int x = 0; x < 32; ++x) acc[d] = fmaf(a[x], b[x + d], acc[d]);
     }
     __syncthreads();
     // the row groups' sums: red[g][p·153 + lag] in the (now free) staging array
