@@ -286,7 +286,7 @@ bool Engine::build_side(int s) {
     bool ok = cuda_ok(sd.work.ensure(n * 4), "features") && cuda_ok(sd.feat.ensure(n * 16), "features") &&
               cuda_ok(sd.feat4.ensure(n * 16), "features") &&
               cuda_ok(sd.mag.ensure(n * 4), "features") && cuda_ok(sd.stack.ensure(n * 20), "features") &&
-              cuda_ok(rtmp.ensure(n * 4), "features") && cuda_ok(stats.ensure(22 * 8), "features") &&
+              cuda_ok(rtmp.ensure(n * 4), "features") && cuda_ok(stats.ensure(kFeatStats * 8), "features") &&
               cuda_ok(hist.ensure(256 * 4), "features") && cuda_ok(wt.ensure(20 * 4), "features") &&
               cuda_ok(part.ensure((size_t)ntiles * kAcfSums * 4), "features") &&
               cuda_ok(sd.acf_dev.ensure(1156 * 8), "features");
@@ -301,11 +301,10 @@ bool Engine::build_side(int s) {
     if (sd.acf_ev && !cuda_ok(cudaStreamWaitEvent(bs, sd.acf_ev, 0), "features")) return false;
     if (!bake(s, bs)) return false;
     if (!cuda_ok(build_features(sd.work.as<float>(), sd.w, sd.h, mode, half, rtmp.as<float>(), sd.feat.as<float>(),
-                                sd.mag.as<float>(), sd.stack.as<float>(), fsc, bs),
-                 "features") ||
-        !cuda_ok(interleave_features(sd.feat.as<float>(), (int)n, sd.feat4.as<float4>(), bs), "features"))
+                                sd.feat4.as<float4>(), sd.mag.as<float>(), sd.stack.as<float>(), fsc, bs),
+                 "features"))
         return false;
-    counts[0] += 12;
+    counts[0] += half ? 7 : 6;
     if (!sd.built_ev && !cuda_ok(cudaEventCreateWithFlags(&sd.built_ev, cudaEventDisableTiming), "features")) return false;
     if (!cuda_ok(cudaEventRecord(sd.built_ev, bs), "features")) return false;
     // the autocorrelation (only the calibrated score's correlation area needs it) runs on a

@@ -8,6 +8,8 @@
 // in float32).
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.hpp"
 
@@ -71,22 +73,31 @@ __global__ void k_hist(const float* __restrict__ g, int n, const double* stats, 
 }
 
 // mid-rank r = (cdf[b] + ½hist[b]) / N · 2 − 1 (smi.wgsl:401-420); every block scans the
-// 256 bins itself
-__global__ void k_rank(const float* __restrict__ g, int n, const double* stats, const unsigned* hist,
-                       float* __restrict__ rank) {
-    __shared__ unsigned sh_h[256], sh_c[256];
-    __shared__ unsigned sh_tot;
-    if (threadIdx.x < 256) sh_h[threadIdx.x] = hist[threadIdx.x];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned acc = 0;
-        for (int i = 0; i < 256; ++i) {
-            sh_c[i] = acc;
-            acc += sh_h[i];
-        }
-        sh_tot = acc > 0 ? acc : 1u;
+// 256 bins itself, a thread a bin (one thread's walk over them was most of the launch)
+__global__ void __launch_bounds__(kThreads) k_rank(const float* __restrict__ g, int n, const double* stats,
+                                                const unsigned* __restrict__ hist, float* __restrict__ rank) {
+    static_assert(kThreads == 256, "a thread per bin");
+    __shared__ unsigned sh_h[256], sh_c[256], sh_w[8];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned own = hist[threadIdx.x];
+    unsigned c = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, c, o);
+        if (lane >= o) c += v;
     }
+    if (lane == 31) sh_w[wid] = c;
     __syncthreads();
+    unsigned all = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if (i < wid) c += sh_w[i];
+        all += sh_w[i];
+    }
+    sh_h[threadIdx.x] = own;
+    sh_c[threadIdx.x] = c - own;
+    __syncthreads();
+    const unsigned sh_tot = all > 0 ? all : 1u;
     const float mean = mean_of(stats, n), spread = spread_of(stats, n);
     const float tot = (float)sh_tot;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -96,112 +107,148 @@ __global__ void k_rank(const float* __restrict__ g, int n, const double* stats, 
     }
 }
 
-// [r, r², Sobel |∇r|, fourth] with clamp-to-edge borders (smi.wgsl:422-462)
-__global__ void k_feats(const float* __restrict__ r, int w, int h, int mode, float* __restrict__ feat,
-                        float* __restrict__ mag) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= w || y >= h) return;
-    auto t = [&](int dx, int dy) {
-        const int xx = min(max(x + dx, 0), w - 1), yy = min(max(y + dy, 0), h - 1);
-        return __ldg(&r[(size_t)yy * w + xx]);
-    };
-    const float c = t(0, 0);
-    float gx = __fadd_rn(-t(-1, -1), t(1, -1));
-    gx = __fsub_rn(gx, __fmul_rn(2.0f, t(-1, 0)));
-    gx = __fadd_rn(gx, __fmul_rn(2.0f, t(1, 0)));
-    gx = __fsub_rn(gx, t(-1, 1));
-    gx = __fadd_rn(gx, t(1, 1));
-    float gy = __fsub_rn(-t(-1, -1), __fmul_rn(2.0f, t(0, -1)));
-    gy = __fsub_rn(gy, t(1, -1));
-    gy = __fadd_rn(gy, t(-1, 1));
-    gy = __fadd_rn(gy, __fmul_rn(2.0f, t(0, 1)));
-    gy = __fadd_rn(gy, t(1, 1));
-    const float g = __fsqrt_rn(__fadd_rn(__fmul_rn(gx, gx), __fmul_rn(gy, gy)));
-    float f3 = 0.0f;
-    if (mode == 0) {
-        f3 = __fadd_rn(__fadd_rn(__fadd_rn(t(-1, 0), t(1, 0)), t(0, -1)), t(0, 1));
-        f3 = __fsub_rn(f3, __fmul_rn(4.0f, c));
-    } else if (mode == 2) {
-        f3 = __fmul_rn(__fmul_rn(c, c), c);
-    }
-    const size_t n = (size_t)w * h, i = (size_t)y * w + x;
-    feat[i] = c;
-    feat[n + i] = __fmul_rn(c, c);
-    feat[2 * n + i] = g;
-    feat[3 * n + i] = f3;
-    mag[i] = g;
-}
-
-// Σx_i (4) and Σx_i x_j (16) in float64 (smi.wgsl:531-551)
-__global__ void k_featmom(const float* __restrict__ feat, int n, double* mom) {
-    __shared__ double sh[32];
-    double a[20];
-#pragma unroll
-    for (int k = 0; k < 20; ++k) a[k] = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double x[4];
-#pragma unroll
-        for (int p = 0; p < 4; ++p) x[p] = (double)feat[(size_t)p * n + i];
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            a[p] += x[p];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) a[4 + p * 4 + q] += x[p] * x[q];
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 20; ++k) {
-        const double v = block_sum(a[k], sh);
-        if (threadIdx.x == 0) atomicAdd(&mom[k], v);
-    }
-}
-
-// global ridge whitening L⁻¹ and μ (smi.wgsl:553-585), float64, stored as f32
-__global__ void k_chol(const double* mom, int n, float ridge, float* wt) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// global ridge whitening L⁻¹ and μ (smi.wgsl:553-585), float64, stored as f32; mom: Σx_i (4), then
+// Σx_i x_j for j ≤ i, row by row (10)
+__device__ void whitening(const double (&mom)[14], int n, float ridge, float* wt) {
     const double nn = fmax((double)n, 1.0);
-    double mu[4], G[16], L[16] = {0}, X[16];
+    double mu[4], G[16], L[16], X[16];
+#pragma unroll
     for (int i = 0; i < 4; ++i) mu[i] = mom[i] / nn;
+#pragma unroll
     for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) G[i * 4 + j] = mom[4 + i * 4 + j] / nn - mu[i] * mu[j];
+#pragma unroll
+        for (int j = 0; j <= i; ++j) G[i * 4 + j] = mom[4 + i * (i + 1) / 2 + j] / nn - mu[i] * mu[j];
     double tr = 0.0;
+#pragma unroll
     for (int i = 0; i < 4; ++i) tr += G[i * 5];
     const double rg = (double)ridge * fmax(tr * 0.25, 1e-12);
+#pragma unroll
     for (int i = 0; i < 4; ++i) G[i * 5] += rg;
+#pragma unroll
     for (int i = 0; i < 4; ++i)
+#pragma unroll
         for (int j = 0; j <= i; ++j) {
             double s = G[i * 4 + j];
+#pragma unroll
             for (int k = 0; k < j; ++k) s -= L[i * 4 + k] * L[j * 4 + k];
             if (i == j) L[i * 5] = sqrt(fmax(s, 1e-12));
             else L[i * 4 + j] = s / L[j * 5];
         }
+#pragma unroll
     for (int col = 0; col < 4; ++col)
+#pragma unroll
         for (int i = 0; i < 4; ++i) {
             double s = (i == col) ? 1.0 : 0.0;
+#pragma unroll
             for (int k = 0; k < i; ++k) s -= L[i * 4 + k] * X[k * 4 + col];
             X[i * 4 + col] = s / L[i * 5];
         }
+#pragma unroll
     for (int i = 0; i < 16; ++i) wt[i] = (float)X[i];
+#pragma unroll
     for (int i = 0; i < 4; ++i) wt[16 + i] = (float)mu[i];
 }
 
-// x ← L⁻¹(x − μ), products rounded one by one in j order (smi.wgsl:587-599)
-__global__ void k_whiten(float* __restrict__ feat, int n, const float* __restrict__ wt) {
+// [r, r², Sobel |∇r|, fourth] with clamp-to-edge borders (smi.wgsl:422-462), and with them Σx_i (4)
+// and the lower triangle of Σx_i x_j (10) in float64 (smi.wgsl:531-551), which the last block turns
+// into the whitening. Small images are latency: the features, their moments and the one-thread
+// Cholesky as three launches took 16 µs of a 256² side's build (now 8), the last two mostly 40 barriers and
+// a chain through local memory. stats: [2..15] the moments, [16] the blocks done (all zeroed before).
+constexpr int kFeatRows = 8, kFeatMoms = 14;
+__global__ void __launch_bounds__(32 * kFeatRows) k_feats(const float* __restrict__ r, int w, int h, int mode,
+                                                          float* __restrict__ feat, float* __restrict__ mag, double* stats,
+                                                          float* __restrict__ wt) {
+    const size_t n = (size_t)w * h;
+    const int tx = (w + 31) / 32, tiles = tx * ((h + kFeatRows - 1) / kFeatRows);
+    double a[kFeatMoms];
+#pragma unroll
+    for (int k = 0; k < kFeatMoms; ++k) a[k] = 0.0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int x = tile % tx * 32 + (threadIdx.x & 31), y = tile / tx * kFeatRows + (threadIdx.x >> 5);
+        if (x >= w || y >= h) continue;
+        auto t = [&](int dx, int dy) {
+            const int xx = min(max(x + dx, 0), w - 1), yy = min(max(y + dy, 0), h - 1);
+            return __ldg(&r[(size_t)yy * w + xx]);
+        };
+        const float c = t(0, 0);
+        float gx = __fadd_rn(-t(-1, -1), t(1, -1));
+        gx = __fsub_rn(gx, __fmul_rn(2.0f, t(-1, 0)));
+        gx = __fadd_rn(gx, __fmul_rn(2.0f, t(1, 0)));
+        gx = __fsub_rn(gx, t(-1, 1));
+        gx = __fadd_rn(gx, t(1, 1));
+        float gy = __fsub_rn(-t(-1, -1), __fmul_rn(2.0f, t(0, -1)));
+        gy = __fsub_rn(gy, t(1, -1));
+        gy = __fadd_rn(gy, t(-1, 1));
+        gy = __fadd_rn(gy, __fmul_rn(2.0f, t(0, 1)));
+        gy = __fadd_rn(gy, t(1, 1));
+        const float g = __fsqrt_rn(__fadd_rn(__fmul_rn(gx, gx), __fmul_rn(gy, gy)));
+        float f3 = 0.0f;
+        if (mode == 0) {
+            f3 = __fadd_rn(__fadd_rn(__fadd_rn(t(-1, 0), t(1, 0)), t(0, -1)), t(0, 1));
+            f3 = __fsub_rn(f3, __fmul_rn(4.0f, c));
+        } else if (mode == 2) {
+            f3 = __fmul_rn(__fmul_rn(c, c), c);
+        }
+        const size_t i = (size_t)y * w + x;
+        const float f[4] = {c, __fmul_rn(c, c), g, f3};
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            feat[(size_t)p * n + i] = f[p];
+            a[p] += (double)f[p];
+#pragma unroll
+            for (int q = 0; q <= p; ++q) a[4 + p * (p + 1) / 2 + q] += (double)f[p] * (double)f[q];
+        }
+        mag[i] = g;
+    }
+    __shared__ double part[kFeatRows][kFeatMoms];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < kFeatMoms; ++k) {
+        const double v = warp_sum(a[k]);
+        if (lane == 0) part[wid][k] = v;
+    }
+    __syncthreads();
+    if (wid != 0) return;
+    if (lane < kFeatMoms) {
+        double v = 0.0;
+#pragma unroll
+        for (int i = 0; i < kFeatRows; ++i) v += part[i][lane];
+        atomicAdd(&stats[2 + lane], v);
+        __threadfence();
+    }
+    __syncwarp();
+    if (lane != 0) return;
+    unsigned* done = reinterpret_cast<unsigned*>(&stats[2 + kFeatMoms]);
+    if (atomicAdd(done, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    double mom[kFeatMoms];
+#pragma unroll
+    for (int k = 0; k < kFeatMoms; ++k) mom[k] = __ldcg(&stats[2 + k]);
+    whitening(mom, (int)n, 1e-4f, wt);
+}
+
+// x ← L⁻¹(x − μ), products rounded one by one in j order (smi.wgsl:587-599), in all the places the
+// features are kept: by plane, by pixel (feat4), and the stack [w, w f0..w f3] with w = 1
+// (smi.wgsl:608-624)
+__global__ void k_whiten(float* __restrict__ feat, int n, const float* __restrict__ wt, float4* __restrict__ feat4,
+                         float* __restrict__ stack) {
     __shared__ float X[20];
     if (threadIdx.x < 20) X[threadIdx.x] = wt[threadIdx.x];
     __syncthreads();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float d[4];
+        float d[4], f[4];
 #pragma unroll
         for (int p = 0; p < 4; ++p) d[p] = __fsub_rn(feat[(size_t)p * n + i], X[16 + p]);
+        stack[i] = 1.0f;
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
-            float s = __fmul_rn(X[p * 4], d[0]);
+            f[p] = __fmul_rn(X[p * 4], d[0]);
 #pragma unroll
-            for (int q = 1; q < 4; ++q) s = __fadd_rn(s, __fmul_rn(X[p * 4 + q], d[q]));
-            feat[(size_t)p * n + i] = s;
+            for (int q = 1; q < 4; ++q) f[p] = __fadd_rn(f[p], __fmul_rn(X[p * 4 + q], d[q]));
+            feat[(size_t)p * n + i] = f[p];
+            stack[(size_t)(p + 1) * n + i] = f[p];
         }
+        feat4[i] = make_float4(f[0], f[1], f[2], f[3]);
     }
 }
 
@@ -306,39 +353,31 @@ __global__ void __launch_bounds__(320) k_pair_area(const double* __restrict__ a,
     if (threadIdx.x == 0) *area = fmax(1.0, fmax(1.0, s / 16.0) * per_cell);
 }
 
-// [w, w f0..w f3] with w = 1 (smi.wgsl:608-624)
-__global__ void k_stack(const float* __restrict__ feat, int n, float* __restrict__ stack) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        stack[i] = 1.0f;
-#pragma unroll
-        for (int p = 0; p < 4; ++p) stack[(size_t)(p + 1) * n + i] = feat[(size_t)p * n + i];
-    }
-}
-
+// Blocks of a launch over n pixels: one a pixel per thread, up to 8 per SM; the sums', whose blocks end
+// in atomic additions to the same few places, at most two per SM
 int grid_for(int n) {
     const int b = (n + kThreads - 1) / kThreads;
     return b < 148 * 8 ? (b > 0 ? b : 1) : 148 * 8;
 }
 
+int sum_grid(int n) { return grid_for(n) < 148 * 2 ? grid_for(n) : 148 * 2; }
+
 }  // namespace
 
-cudaError_t build_features(float* gray, int w, int h, int mode, bool half, float* rank, float* feat, float* mag,
-                           float* stack, FeatScratch& s, cudaStream_t st) {
+cudaError_t build_features(float* gray, int w, int h, int mode, bool half, float* rank, float* feat, float4* feat4,
+                           float* mag, float* stack, FeatScratch& s, cudaStream_t st) {
     const int n = w * h;
-    const int gb = grid_for(n);
-    cudaMemsetAsync(s.stats, 0, 22 * sizeof(double), st);
+    const int gb = grid_for(n), gs = sum_grid(n), tiles = ((w + 31) / 32) * ((h + kFeatRows - 1) / kFeatRows);
+    static_assert(2 + kFeatMoms < kFeatStats, "the moments and the count of blocks done");
+    cudaMemsetAsync(s.stats, 0, kFeatStats * sizeof(double), st);
     cudaMemsetAsync(s.hist, 0, 256 * sizeof(unsigned), st);
     if (half) k_quant_half<<<gb, kThreads, 0, st>>>(gray, n);
-    k_sum<<<gb, kThreads, 0, st>>>(gray, n, s.stats);
-    k_sumsq<<<gb, kThreads, 0, st>>>(gray, n, s.stats);
-    k_hist<<<gb, kThreads, 0, st>>>(gray, n, s.stats, s.hist);
+    k_sum<<<gs, kThreads, 0, st>>>(gray, n, s.stats);
+    k_sumsq<<<gs, kThreads, 0, st>>>(gray, n, s.stats);
+    k_hist<<<gs, kThreads, 0, st>>>(gray, n, s.stats, s.hist);
     k_rank<<<gb, kThreads, 0, st>>>(gray, n, s.stats, s.hist, rank);
-    dim3 b2(32, 8), g2((w + 31) / 32, (h + 7) / 8);
-    k_feats<<<g2, b2, 0, st>>>(rank, w, h, mode, feat, mag);
-    k_featmom<<<grid_for(n) < 296 ? grid_for(n) : 296, kThreads, 0, st>>>(feat, n, s.stats + 2);
-    k_chol<<<1, 32, 0, st>>>(s.stats + 2, n, 1e-4f, s.wt);
-    k_whiten<<<gb, kThreads, 0, st>>>(feat, n, s.wt);
-    k_stack<<<gb, kThreads, 0, st>>>(feat, n, stack);
+    k_feats<<<std::min(tiles, 148 * 4), 32 * kFeatRows, 0, st>>>(rank, w, h, mode, feat, mag, s.stats, s.wt);
+    k_whiten<<<gb, kThreads, 0, st>>>(feat, n, s.wt, feat4, stack);
     return cudaGetLastError();
 }
 

@@ -12,8 +12,9 @@ namespace zc {
 // ── per-image features (features.cu) ──
 constexpr int kAcfSums = 153 * 4;  // lags dy = 0..8, dx = −8..8, of 4 planes
 // Scratch the feature build needs on the device (sizes in bytes are fixed; see features.cu).
+constexpr int kFeatStats = 17;
 struct FeatScratch {
-    double* stats = nullptr;     // [0] Σg, [1] Σ(g − mean)², [2..21] whitening moments
+    double* stats = nullptr;     // kFeatStats: Σg, Σ(g − mean)², 14 whitening moments, the count of blocks done
     unsigned* hist = nullptr;    // 256 bins
     float* wt = nullptr;         // L⁻¹ (16) and μ (4) of the whitening
     float* acf_part = nullptr;   // per-tile autocorrelation partial sums, kAcfSums per 32 × 32 tile
@@ -21,10 +22,10 @@ struct FeatScratch {
     double* acf = nullptr;       // 289 × 4 normalised autocorrelation
 };
 
-// gray (w×h f32, device) → feat (4 planes), mag (1 plane), stack (5 planes). mode: 0 laplacian,
+// gray (w×h f32, device) → feat (4 planes), feat4 (the same by pixel), mag (1 plane), stack (5 planes). mode: 0 laplacian,
 // 1 three, 2 cubic. `half`: quantise the input to f16 first (in place on `gray`).
 cudaError_t build_features(float* gray, int w, int h, int mode, bool half, float* rank_tmp, float* feat,
-                           float* mag, float* stack, FeatScratch& s, cudaStream_t st);
+                           float4* feat4, float* mag, float* stack, FeatScratch& s, cudaStream_t st);
 // the features' autocorrelation sums at |τ| ≤ 8 (289 lags × 4 planes, device doubles in s.acf;
 // per-tile partials in s.acf_part)
 cudaError_t autocorrelation(const float* feat, int w, int h, FeatScratch& s, cudaStream_t st);
@@ -189,8 +190,6 @@ struct PoseSide {
     const float4* feat4;  // the same planes interleaved, one float4 per pixel
     int w, h;
 };
-// the 4 plane-major feature planes of n pixels interleaved into one float4 per pixel
-cudaError_t interleave_features(const float* feat, int n, float4* out, cudaStream_t st);
 // A cubic B-spline on top of the pose: g × g control points (x, y per point, in half-image units
 // of the lattice's image), on b (the destination: it moves b's pixel before H⁻¹) or, source, on a
 // (it moves the sample after H⁻¹). cps null: no spline.

@@ -1031,23 +1031,10 @@ int pose_slots(K k) {
 
 }  // namespace
 
-namespace {
-__global__ void k_feat_interleave(const float* __restrict__ feat, int n, float4* __restrict__ out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[i] = make_float4(feat[i], feat[(size_t)n + i], feat[2 * (size_t)n + i], feat[3 * (size_t)n + i]);
-}
-}  // namespace
-
 void pose_tune(unsigned px_per_thread, unsigned min_blocks, unsigned max_blocks) {
     if (px_per_thread) g_px_per_thread = std::min(px_per_thread, 4096u);
     if (min_blocks) g_min_blocks = std::min(min_blocks, 4096u);
     if (max_blocks) g_max_blocks = std::min(max_blocks, 4096u);
-}
-
-cudaError_t interleave_features(const float* feat, int n, float4* out, cudaStream_t st) {
-    const int blocks = std::min((n + 255) / 256, 148 * 8);
-    k_feat_interleave<<<std::max(blocks, 1), 256, 0, st>>>(feat, n, out);
-    return cudaGetLastError();
 }
 
 namespace {
