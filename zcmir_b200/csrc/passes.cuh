@@ -198,8 +198,10 @@ __global__ void __launch_bounds__(MAXT, MINB) k_inv_cols(const float2* __restric
 // spectrum, conj(Q1) + i·conj(Q2) mirrored above it, its inverse FFT the two real rows, written
 // over Q1's and Q2's row (a row of WP complex holds the nx reals). The task's lines are in one
 // block and every line reads its inputs before the block's first barrier and writes after it, so
-// writing in place is safe. Blocks of 256 threads, four per SM (two of 512 left the barriers of whole
-// blocks exposed: rows of 2048 points 169 → 143 µs, 192: 453 → 409). S = 2: two lines of nx/2 points per task, line s the outputs
+// writing in place is safe. Blocks of few lines, 1024 threads of them per SM: a line's barriers then hold
+// up no more than its block, and the others' loads go on (two blocks of 512, then four of 256, then
+// kRowT: 4096² rows and score of 18 correlations 1405 → 1281 µs, 104 sweep maps of 192² 453 → 409 →
+// 333). S = 2: two lines of nx/2 points per task, line s the outputs
 // x ≡ s (mod 2) after one decimation-in-frequency step.
 template <class F, int S>
 __global__ void __launch_bounds__(F::kRowT, 1024 / F::kRowT) k_inv_rows(float2* __restrict__ Q, size_t pstride, int WP, int nx, int ntask,
@@ -304,6 +306,25 @@ cudaError_t run_cols(F f, const PassArgs& a, cudaStream_t st) {
     }
 }
 
+template <class F>
+cudaError_t run_rows(F f, const PassArgs& a, cudaStream_t st) {
+    const MapGeom& g = a.g;
+    const CorrPlanDev& plan = *a.plan;
+    const size_t pstride = (size_t)g.ny * g.WP;
+    const int tl = f.tl();
+    cudaError_t e;
+    // rows: whole tasks (S lines) per block of up to kRowT threads
+    if (a.S != 1 && a.S != 2) return cudaErrorInvalidConfiguration;
+    const int lpb = std::max(a.S, lines_per_block(tl, F::kRowT) / a.S * a.S), ntask = g.ny * ((plan.n_corr + 1) / 2);
+    if (lpb * tl > F::kRowT) return cudaErrorInvalidConfiguration;
+    const size_t sm = (size_t)lpb * padded_len(f.n()) * sizeof(float2);
+    auto k = a.S == 1 ? k_inv_rows<F, 1> : k_inv_rows<F, 2>;
+    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
+    k<<<dim3((ntask + lpb / a.S - 1) / (lpb / a.S), a.batch), lpb * tl, sm, st>>>(a.Q, pstride, g.WP, g.nx, ntask, plan.n_corr,
+                                                                                  f, lpb, a.tw_nx, a.q_stride);
+    return cudaGetLastError();
+}
+
 // One pass over a batch with line policy F.
 template <class F>
 cudaError_t run_pass(Pass p, F f, const PassArgs& a, cudaStream_t st) {
@@ -327,16 +348,7 @@ cudaError_t run_pass(Pass p, F f, const PassArgs& a, cudaStream_t st) {
     }
     if (p == Pass::FwdCols) return run_cols<Pass::FwdCols>(f, a, st);
     if (p == Pass::InvCols) return run_cols<Pass::InvCols>(f.inv(), a, st);
-    // rows: whole tasks (S lines) per block of up to kRowT threads
-    if (a.S != 1 && a.S != 2) return cudaErrorInvalidConfiguration;
-    const int lpb = std::max(a.S, lines_per_block(tl, F::kRowT) / a.S * a.S), ntask = g.ny * ((plan.n_corr + 1) / 2);
-    if (lpb * tl > F::kRowT) return cudaErrorInvalidConfiguration;
-    const size_t sm = (size_t)lpb * padded_len(f.n()) * sizeof(float2);
-    auto k = a.S == 1 ? k_inv_rows<F, 1> : k_inv_rows<F, 2>;
-    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
-    k<<<dim3((ntask + lpb / a.S - 1) / (lpb / a.S), a.batch), lpb * tl, sm, st>>>(a.Q, pstride, g.WP, g.nx, ntask, plan.n_corr,
-                                                                                  f, lpb, a.tw_nx, a.q_stride);
-    return cudaGetLastError();
+    return run_rows(f.row(), a, st);
 }
 
 }  // namespace
