@@ -335,9 +335,13 @@ cudaError_t run_pass(Pass p, F f, const PassArgs& a, cudaStream_t st) {
     cudaError_t e;
     if (p == Pass::FwdRows) {
         const int n_cplx = (plan.n_real + 1) / 2;
-        // the row's lines at once where 512 threads hold them (5 planes: 3 lines), else up to 256
-        // threads of lines (one line of more for the longest rows: 8192 points, 512 threads)
-        const int lines = std::min(n_cplx, n_cplx <= 3 && n_cplx * tl <= 512 ? n_cplx : lines_per_block(tl, 256));
+        // The row's 3 lines at once (5 planes) where 512 threads hold them, else up to 256 threads of its 8.
+        // Lines of whole warps, two or more of them: as many as 128 threads hold, one at least; the row's
+        // others follow, and other rows' blocks fill the barriers (two sides of a map of 2048²: 98 → 76 µs,
+        // 1536²: 90 → 77, 1024²: 28 → 25; 72 and 81 threads a line lost up to a third).
+        const int lines = std::min(n_cplx, tl >= 64 && tl % 32 == 0          ? lines_per_block(tl, 128)
+                                           : n_cplx <= 3 && n_cplx * tl <= 512 ? n_cplx
+                                                                               : lines_per_block(tl, 256));
         const int products = plan.planes[plan.n_real - 1] >= 5;
         const size_t sm = (size_t)lines * padded_len(g.nx) * sizeof(float2) + (size_t)(products ? 9 : 5) * g.cw * sizeof(float);
         auto k = 2 * g.cw <= g.nx ? k_fwd_rows<F, true> : k_fwd_rows<F, false>;
