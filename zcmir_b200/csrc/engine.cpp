@@ -690,7 +690,7 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
         if (have[s]) {
             kept_grid(s, grid);
         } else {
-            spec_key_[s].clear();  // until this side's passes are queued
+            forget_side(s);  // until this side's passes are queued
             if (!canvas_side(s, grid)) return false;
             counts[0] += job.identity_grid ? 1 : 2;
         }

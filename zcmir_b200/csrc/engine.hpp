@@ -336,13 +336,18 @@ class Engine {
     // canvas and forward transforms. Cleared by every other user of those buffers.
     std::array<std::vector<uint64_t>, 2> spec_key_;
     int spec_planes_[2] = {0, 0};                  // leading planes of the side whose spectra are kept
-    std::array<std::vector<uint64_t>, 2> box_key_;  // what the sides' moment tables were built from
+    // What the sides' moment tables were built from. Forgotten with the spectra: a captured map's replay
+    // rewrites the tables too, and runs no host code that would say so.
+    std::array<std::vector<uint64_t>, 2> box_key_;
     bool spectra_cache_ = true;     // ZCMIR_B200_SPECTRA_CACHE=0 at creation: always rebuild
     bool spectra_cache_off_ = false;  // set while a benchmark times whole maps
     uint64_t build_counter_ = 0;
     void forget_spectra() {
-        spec_key_[0].clear();
-        spec_key_[1].clear();
+        for (int s = 0; s < 2; ++s) forget_side(s);
+    }
+    void forget_side(int s) {
+        spec_key_[s].clear();
+        box_key_[s].clear();
     }
     // the batched Gauss–Newton refine's device state (gn_batch_dev)
     DevBuf gn_H_, gn_Htry_, gn_valid_, gn_active_, gn_cur_;
