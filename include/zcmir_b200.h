@@ -89,7 +89,10 @@ int32_t zcb_sweep_stack(zc_engine* e, const double H0[9], uint32_t n_peak, float
 
 /* zc_set_image_rgba for 8-bit pixels of 1 (gray: R = G = B), 3 (RGB) or 4 (RGBA) interleaved channels,
  * uploaded as they are: the same image, preprocessing and errors, without expanding it to RGBA8 on the
- * host first. No counterpart in the reference (its upload takes RGBA8 only, src/exports.zig). 0 / −1. */
+ * host first. No counterpart in the reference (its upload takes RGBA8 only, src/exports.zig). 0 / −1.
+ * The pixels may be changed or freed on return, here and after zc_set_image_rgba. After zc_set_image and
+ * zc_set_image_gray the same holds for pageable memory; page-locked memory is still being read, and must
+ * stay until a call that returns results (a score, a map, the features) has returned. */
 int32_t zcb_set_image_u8(zc_engine* e, uint32_t side, const uint8_t* data, uint32_t w, uint32_t h, uint32_t channels);
 
 /* Scores of n poses (Hs: n row-major 3×3 maps, each as zc_score's H) into out[3n], per pose the

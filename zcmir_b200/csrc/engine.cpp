@@ -179,22 +179,44 @@ bool Engine::set_image(int s, const float* data, int w, int h, bool preprocess) 
     return build_side(s);
 }
 
+// Whether a copy from host memory at p may still be reading it when its call returns: page-locked (or
+// managed) memory is read by the copy engine in stream order, pageable memory is staged first.
+static bool read_after_return(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type != cudaMemoryTypeUnregistered;
+}
+
 bool Engine::set_image_u8(int s, const unsigned char* px, int w, int h, int channels) {
     if (s < 0 || s > 1 || w < 8 || h < 8 || !px || (channels != 1 && channels != 3 && channels != 4))
         return fail("set_image_rgba: BadImage");
     Side& sd = side[s];
     const size_t n = (size_t)w * h;
+    // The caller's pixels are its own again on return (a ring of capture buffers is refilled at once): a
+    // copy from page-locked memory is waited for, after the build behind it is queued.
+    const bool wait = read_after_return(px);
+    if (wait && !up_ev_ && !cuda_ok(cudaEventCreateWithFlags(&up_ev_, cudaEventDisableTiming), "set_image_rgba")) return false;
     if (!cuda_ok(pp_rgba_.ensure(n * channels), "set_image_rgba") || !cuda_ok(sd.raw.ensure(n * 4), "set_image_rgba") ||
-        !cuda_ok(cudaMemcpyAsync(pp_rgba_.p, px, n * channels, cudaMemcpyHostToDevice, st), "set_image_rgba") ||
-        !cuda_ok(u8_to_gray(pp_rgba_.as<unsigned char>(), (int)n, channels, sd.raw.as<float>(), st), "set_image_rgba"))
+        !cuda_ok(cudaMemcpyAsync(pp_rgba_.p, px, n * channels, cudaMemcpyHostToDevice, st), "set_image_rgba"))
         return false;
-    counts[0] += 1;
-    sd.has = true;
-    sd.w = w;
-    sd.h = h;
-    sd.preprocess = true;
-    sd.built = false;
-    return build_side(s);
+    const bool marked = wait && cuda_ok(cudaEventRecord(up_ev_, st), "set_image_rgba");
+    auto build = [&] {
+        if (!cuda_ok(u8_to_gray(pp_rgba_.as<unsigned char>(), (int)n, channels, sd.raw.as<float>(), st), "set_image_rgba"))
+            return false;
+        counts[0] += 1;
+        sd.has = true;
+        sd.w = w;
+        sd.h = h;
+        sd.preprocess = true;
+        sd.built = false;
+        return build_side(s);
+    };
+    const bool ok = build();
+    if (!wait) return ok;
+    return cuda_ok(marked ? cudaEventSynchronize(up_ev_) : cudaStreamSynchronize(st), "set_image_rgba") && ok && marked;
 }
 
 std::string Engine::bake_key() const {

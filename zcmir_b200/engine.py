@@ -231,7 +231,9 @@ class Engine:
     def set_image(self, side, img, preprocess=True):
         """Side 0 (moving) or 1 (fixed). uint8 images go up as they are (gray, RGB or RGBA), which the
         engine always preprocesses; anything else as float32 gray, preprocessed (CLAHE / band pass / invert of
-        the settings) when ``preprocess``."""
+        the settings) when ``preprocess``. The array may be changed or dropped on return, with one exception:
+        a contiguous float32 array in page-locked memory is uploaded while later work is queued, and must stay
+        as it is until a call that returns results (a score, a map, the features) has returned."""
         a = np.asarray(img)
         if a.dtype == np.uint8:
             if not preprocess:
