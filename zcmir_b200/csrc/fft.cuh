@@ -562,6 +562,7 @@ __device__ __forceinline__ void mix_fft_in(float2* __restrict__ buf, const float
 // in); LO: the caller guarantees in(y) = 0 for y ≥ n/2, so a compile-time line reads only y < n/2.
 struct GenericLine {
     static constexpr int kTl = 0, kTx = 0, kRowT = 512;  // kTx 0: tile and threads chosen at the launch
+    static constexpr bool kLong = false;
     __host__ GenericLine inv() const { return *this; }
     __host__ GenericLine row() const { return *this; }
     LinePlan p;
@@ -597,6 +598,7 @@ struct FixedLine {
     // threads of a block of rows: two short lines or more, or one of whole warps
     static constexpr int kRowT = TPL <= 32 ? 64 : TPL <= 64 || TPL == 128 ? 128 : TPL <= 256 ? 256 : 512;
     static constexpr bool kOne = TPL > line_tl(N);                                    // one group of points a thread
+    static constexpr bool kLong = N > 5184;  // a full row's staged products do not fit beside the line
     using Inv = FixedLine<N, col_inv_tl(N)>;                                          // the inverse columns' line
     __host__ Inv inv() const { return Inv{tw}; }
     using Row = FixedLine<N, row_tl(N)>;                                               // the inverse rows' line

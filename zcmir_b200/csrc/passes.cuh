@@ -55,25 +55,33 @@ namespace {
 
 // Real correlation plane r of a staged row: rows 0..4 the premultiplied samples s = [w, w f0..w f3],
 // rows 5..8 f_i = s_{1+i} / s_0 (0 where s_0 ≤ 1e-6) (smi.wgsl:641-649): planes 0 → w, 1..4 → w f_i,
-// 5..14 → s_i f_j. p: its samples' row, q: the row it is multiplied by (null for planes 0..4).
+// 5..14 → s_i f_j. p: its samples' row, q: the row it is multiplied by (null for planes 0..4). RECIP: row 5
+// is 1 / s_0 in place of the f_i, multiplied in at each use (the same products, rounded the same).
+template <bool RECIP>
 struct RealPlane {
-    const float *p, *q;
-    __device__ __forceinline__ RealPlane(int r, const float* row, int cw) : p(row + r * cw), q(nullptr) {
+    const float *p, *q, *inv;
+    __device__ __forceinline__ RealPlane(int r, const float* row, int cw) : p(row + r * cw), q(nullptr), inv(row + 5 * cw) {
         if (r < 5) return;
         const int k = r - 5;
         const int ti = (k < 4) ? 0 : (k < 7) ? 1 : (k < 9) ? 2 : 3;
         const int tj = (k < 4) ? k : (k < 7) ? k - 3 : (k < 9) ? k - 5 : 3;
         p = row + (1 + ti) * cw;
-        q = row + (5 + tj) * cw;
+        q = row + ((RECIP ? 1 : 5) + tj) * cw;
     }
-    __device__ __forceinline__ float operator()(int x) const { return q ? p[x] * q[x] : p[x]; }
+    __device__ __forceinline__ float operator()(int x) const {
+        if (!q) return p[x];
+        return RECIP ? __fmul_rn(p[x], __fmul_rn(q[x], inv[x])) : p[x] * q[x];
+    }
 };
+
+// shared memory a block may ask for, less the row kernel's own static array
+constexpr size_t kRowShared = 227 * 1024 - 64;
 
 // One block per grid row y < ch; lines = packed plane pairs (2z, 2z+1), lpb of them at a time.
 // The row's samples are staged in shared memory once (after the line buffers).
 // Batched over blockIdx.y: item b reads grid + b·gbs and writes half + b·hbs.
-// LO: cw ≤ nx/2, so the first butterflies read only the row's lower half.
-template <class F, bool LO>
+// LO: cw ≤ nx/2, so the first butterflies read only the row's lower half. RECIP: as RealPlane.
+template <class F, bool LO, bool RECIP>
 __global__ void __launch_bounds__(512, 1) k_fwd_rows(const float* __restrict__ grid, int cw, int ch, int WP,
                                                      CorrPlanDev plan, F f, int lpb, int products,
                                                      float2* __restrict__ half, size_t pstride, size_t gbs,
@@ -87,7 +95,7 @@ __global__ void __launch_bounds__(512, 1) k_fwd_rows(const float* __restrict__ g
     const int t = threadIdx.x - line * tl;
     const int pl = padded_len(nx);
     float2* buf = smem + (line < lpb ? line : 0) * pl;
-    float* row = reinterpret_cast<float*>(smem + lpb * pl);  // [9][cw] (RealPlane)
+    float* row = reinterpret_cast<float*>(smem + lpb * pl);  // [9][cw], [6][cw] or [5][cw] (RealPlane)
     __shared__ int planes[16];
     if (threadIdx.x < 16) planes[threadIdx.x] = threadIdx.x < plan.n_real ? plan.planes[threadIdx.x] : -1;
     const size_t gn = (size_t)cw * ch;
@@ -97,8 +105,10 @@ __global__ void __launch_bounds__(512, 1) k_fwd_rows(const float* __restrict__ g
         for (int p = 0; p < 5; ++p) row[p * cw + x] = v[p] = __ldg(&grid[p * gn + (size_t)y * cw + x]);
         if (products) {
             const float inv = v[0] <= 1e-6f ? 0.f : 1.f / v[0];
+            if (RECIP) row[5 * cw + x] = inv;
+            else
 #pragma unroll
-            for (int p = 1; p < 5; ++p) row[(4 + p) * cw + x] = v[p] * inv;
+                for (int p = 1; p < 5; ++p) row[(4 + p) * cw + x] = v[p] * inv;
         }
     }
     __syncthreads();
@@ -107,7 +117,7 @@ __global__ void __launch_bounds__(512, 1) k_fwd_rows(const float* __restrict__ g
         const int z = z0 + line;
         const bool act = line < lpb && z < n_cplx;
         const bool has_b = act && 2 * z + 1 < plan.n_real;
-        const RealPlane ra(act ? planes[2 * z] : 0, row, cw), rb(has_b ? planes[2 * z + 1] : 0, row, cw);
+        const RealPlane<RECIP> ra(act ? planes[2 * z] : 0, row, cw), rb(has_b ? planes[2 * z + 1] : 0, row, cw);
         // the first butterflies read the staged rows directly (real planes ra + i·rb, zero past cw)
         f.fresh().template run_in<false, LO>(buf, t, act, [&](int x) {
             float2 v = make_float2(0.f, 0.f);
@@ -343,8 +353,17 @@ cudaError_t run_pass(Pass p, F f, const PassArgs& a, cudaStream_t st) {
                                            : n_cplx <= 3 && n_cplx * tl <= 512 ? n_cplx
                                                                                : lines_per_block(tl, 256));
         const int products = plan.planes[plan.n_real - 1] >= 5;
-        const size_t sm = (size_t)lines * padded_len(g.nx) * sizeof(float2) + (size_t)(products ? 9 : 5) * g.cw * sizeof(float);
-        auto k = 2 * g.cw <= g.nx ? k_fwd_rows<F, true> : k_fwd_rows<F, false>;
+        auto smem = [&](int rows) { return (size_t)lines * padded_len(g.nx) * sizeof(float2) + (size_t)rows * g.cw * sizeof(float); };
+        size_t sm = smem(products ? 9 : 5);
+        auto k = 2 * g.cw <= g.nx ? k_fwd_rows<F, true, false> : k_fwd_rows<F, false, false>;
+        // A roto-scale grid has as many cells to a row as the line has points: from 5832 points on, nine rows
+        // of them and the line do not fit shared memory, six do up to 6912.
+        if constexpr (F::kLong) {
+            if (products && 2 * g.cw > g.nx && sm > kRowShared) {
+                sm = smem(6);
+                k = k_fwd_rows<F, false, true>;
+            }
+        }
         if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
         k<<<dim3(g.ch, a.batch), lines * tl, sm, st>>>(a.grid, g.cw, g.ch, g.WP, plan, f, lines, products, a.half,
                                                        pstride, a.grid_stride, a.half_stride);
