@@ -148,6 +148,9 @@ bool Engine::fail(const std::string& m) {
 
 bool Engine::cuda_ok(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return true;
+    // the runtime keeps the error of a refused call until it is read: this call reports it, so that the next
+    // call's launches, checked by cudaGetLastError, are not blamed for it
+    cudaGetLastError();
     return fail(std::string(what) + ": CUDA error: " + cudaGetErrorString(e));
 }
 
