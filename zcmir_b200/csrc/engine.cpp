@@ -833,8 +833,8 @@ bool Engine::shift_map(const Mat3& Hm, bool exact, bool calibrated, unsigned cap
     if (profiling)
         for (auto& e : ev) cudaEventCreate(&e);
     if (!run_map(job, profiling ? ev : nullptr, map)) return false;
-    unsigned char host[32];
-    if (!cuda_ok(cudaMemcpyAsync(host, res_.p, 32, cudaMemcpyDeviceToHost, st), "shift_map")) return false;
+    unsigned char host[kMapRecord];
+    if (!cuda_ok(cudaMemcpyAsync(host, res_.p, kMapRecord, cudaMemcpyDeviceToHost, st), "shift_map")) return false;
     counts[2]++;
     if (!cuda_ok(cudaStreamSynchronize(st), "shift_map") ||
         (map && !cuda_ok(cudaStreamSynchronize(copy_st_), "shift_map")))
@@ -853,18 +853,22 @@ bool Engine::shift_map(const Mat3& Hm, bool exact, bool calibrated, unsigned cap
     }
     unsigned long long best;
     float zero;
-    unsigned fault;
     memcpy(&best, host, 8);
     memcpy(&zero, host + 8, 4);
-    memcpy(&fault, host + 24, 4);
-    if (fault)
-        return fail("shift_map: the inverse column pass gave up waiting for its operand copies (fault " +
-                    std::to_string(fault) + "); the map is not valid");
-    memcpy(&fault, host + 28, 4);
-    if (dft_pieces_ && fault)
-        return fail("shift_map: the tensor-core column stage gave up waiting for its products; the map is not valid");
+    if (!map_valid(host, "shift_map")) return false;
     if (!finish_acf()) return false;
     map_result(job, best, zero, pair_area(), out);
+    return true;
+}
+
+bool Engine::map_valid(const unsigned char* rec, const std::string& what) {
+    unsigned fault[2];
+    memcpy(fault, rec + 24, 8);
+    if (fault[0])
+        return fail(what + ": the inverse column pass gave up waiting for its operand copies (fault " +
+                    std::to_string(fault[0]) + "); the map is not valid");
+    if (dft_pieces_ && fault[1])
+        return fail(what + ": the tensor-core column stage gave up waiting for its products; the map is not valid");
     return true;
 }
 

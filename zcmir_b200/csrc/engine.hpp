@@ -166,6 +166,11 @@ struct SideSwap {
     ~SideSwap() { std::swap(a, b); }
 };
 
+// A map's result as run_map leaves it at the head of its result buffer: the best key (u64), the zero-lag
+// score (f32, at 8), the zero-lag overlap (f64, at 16), the fault words (u32) of the inverse columns (24) and of
+// the tensor-core column stage (28, set to 0 only by maps that run it).
+constexpr size_t kMapRecord = 32;
+
 // Stages of a map timed by the profiler / the benchmark entry point.
 enum Stage { kCanvas = 0, kFwdRows, kFwdCols, kInvCols, kInvRows, kNumStages };
 extern const char* const kStageNames[kNumStages];
@@ -232,6 +237,8 @@ class Engine {
     bool shift_map(const Mat3& H, bool exact, bool calibrated, unsigned cap, double min_overlap, zc_shift_result* out,
                    float* map, size_t map_len);
     bool shift_map_settings(const Mat3& H, zc_shift_result* out, float* map, size_t map_len);
+    // whether a map's record (kMapRecord) has no fault word set, else false with the error under `what`
+    bool map_valid(const unsigned char* rec, const std::string& what);
     // a map's result from its best key (score bits, inverted index), zero-lag score and the
     // pair's correlation area
     void map_result(const MapJob& job, unsigned long long best, float zero, double area, zc_shift_result* out);

@@ -28,7 +28,7 @@ bool Engine::stack_load(int n, const float* const* images, const int* ws, const 
     for (int i = 0; i < n; ++i)
         if (!images[i] || ws[i] < 8 || hs[i] < 8) return fail("stack_maps: BadImage (slice " + std::to_string(i) + ")");
     if ((int)stack_.size() < n) stack_.resize(n);
-    if (!cuda_ok(stack_res_.ensure((size_t)(n - 1) * 24), "stack_maps")) return false;
+    if (!cuda_ok(stack_res_.ensure((size_t)(n - 1) * kMapRecord), "stack_maps")) return false;
     // every slice's features, once (the current settings: feature mode, f16 input)
     for (int i = 0; i < n; ++i) {
         SideSwap sw(side[0], stack_[i]);
@@ -67,8 +67,8 @@ int Engine::stack_enqueue() {
         SideSwap mv(side[0], stack_[k]);
         SideSwap fx(side[1], stack_[k - 1]);
         ok = run_map(stack_jobs_[k - 1], nullptr) &&
-             cuda_ok(cudaMemcpyAsync(stack_res_.as<unsigned char>() + (k - 1) * 24, res_.p, 24, cudaMemcpyDeviceToDevice,
-                                     st),
+             cuda_ok(cudaMemcpyAsync(stack_res_.as<unsigned char>() + (k - 1) * kMapRecord, res_.p, kMapRecord,
+                                     cudaMemcpyDeviceToDevice, st),
                      "stack_maps");
     }
     spectra_cache_off_ = cache_off;
@@ -78,18 +78,20 @@ int Engine::stack_enqueue() {
 
 bool Engine::stack_collect(zc_shift_result* out) {
     const size_t m = stack_jobs_.size();
-    std::vector<unsigned char> host(m * 24);
+    std::vector<unsigned char> host(m * kMapRecord);
     if (!cuda_ok(cudaMemcpyAsync(host.data(), stack_res_.p, host.size(), cudaMemcpyDeviceToHost, st), "stack_maps") ||
         !cuda_ok(cudaStreamSynchronize(st), "stack_maps"))
         return false;
     counts[1]++;
     counts[2]++;
     counts[3]++;
+    for (size_t k = 0; k < m; ++k)
+        if (!map_valid(host.data() + k * kMapRecord, "stack_maps: pair " + std::to_string(k + 1))) return false;
     for (size_t k = 0; k < m; ++k) {
         unsigned long long best;
         float zero;
-        std::memcpy(&best, host.data() + k * 24, 8);
-        std::memcpy(&zero, host.data() + k * 24 + 8, 4);
+        std::memcpy(&best, host.data() + k * kMapRecord, 8);
+        std::memcpy(&zero, host.data() + k * kMapRecord + 8, 4);
         map_result(stack_jobs_[k], best, zero, stack_areas_[k], &out[k]);
     }
     return true;
