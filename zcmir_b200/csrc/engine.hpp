@@ -417,7 +417,7 @@ class Engine {
     DevBuf pose_hinv_, pose_sums_, pose_coef_, pose_score_, pose_tsum_;
     // the pose kernels' per-block totals and per-pose tickets (their sums added in block order)
     DevBuf pose_part_, pose_ticket_;
-    bool pose_red(int n, PoseRed& r);
+    bool pose_red(int n, int least, PoseRed& r);
     DevBuf rs_fwd_, rs_inv_, rs_map_;
     DevBuf pp_rgba_, pp_clahe_, pp_tmp_, pp_mm_;
     std::vector<Side> stack_;

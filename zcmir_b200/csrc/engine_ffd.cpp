@@ -111,7 +111,7 @@ bool Engine::ffd_gradient(const Mat3& H, double* score, double* grad, size_t len
     ok = cuda_ok(cudaMemcpyAsync(ffd_dev_.p, h.data(), h.size() * 4, cudaMemcpyHostToDevice, st), "ffd_gradient") &&
          cuda_ok(cudaMemcpyAsync(dh, hinv, sizeof hinv, cudaMemcpyHostToDevice, st), "ffd_gradient");
     PoseRed rd;
-    ok = ok && pose_red(nd, rd);
+    ok = ok && pose_red(nd, nd, rd);
     PoseCall pc;
     pc.a = pa, pc.b = pb, pc.sym = sym, pc.hinv = dh, pc.n = 1, pc.ffd[0] = ff, pc.ffd[1] = fi, pc.red = rd;
     PoseScores ps;

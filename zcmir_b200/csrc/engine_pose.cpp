@@ -48,14 +48,23 @@ std::string json_str(const std::string& t) {
 
 void Engine::log_event(const std::string& text) { events.push_back("{\"kind\":\"log\",\"text\":" + json_str(text) + "}"); }
 
-// scratch for n poses per launch onto either side: the pose kernels then add each pose's
-// block totals in block order (the same sums on every run, in any batch); fresh tickets are zeroed
-bool Engine::pose_red(int n, PoseRed& r) {
+// Scratch for the block totals of n rows (a pose in one direction, onto either side), or of as many as
+// kPoseScratch holds (at least `least`, what one pose takes): a launch takes as many poses as there are rows
+// for. The pose kernels then add each row's block totals in block order (the same sums on every run, in any
+// batch); fresh tickets are zeroed. 128 MB are 1600 rows of a 1024² pair, 220 blocks each: a launch of them is
+// long against the gap to the next. A card too full for that gets by with fewer.
+constexpr size_t kPoseScratch = (size_t)128 << 20;
+
+bool Engine::pose_red(int n, int least, PoseRed& r) {
     const size_t px = std::max((size_t)side[0].w * side[0].h, (size_t)side[1].w * side[1].h);
+    const size_t row = pose_red_need(px, 1) * sizeof(double), lo = (size_t)std::max(least, 1);
+    size_t rows = std::max(lo, std::min((size_t)std::max(n, 1), kPoseScratch / row));
+    while (pose_part_.ensure(rows * row) != cudaSuccess) {
+        if (cudaGetLastError() != cudaErrorMemoryAllocation || rows == lo) return fail("pose sums: out of device memory");
+        rows = std::max(lo, rows / 2);
+    }
     const uint64_t gen = pose_ticket_.gen;
-    if (!cuda_ok(pose_part_.ensure(pose_red_need(px, n) * sizeof(double)), "pose sums") ||
-        !cuda_ok(pose_ticket_.ensure((size_t)std::max(n, 1) * sizeof(unsigned)), "pose sums"))
-        return false;
+    if (!cuda_ok(pose_ticket_.ensure(rows * sizeof(unsigned)), "pose sums")) return false;
     if (pose_ticket_.gen != gen && !cuda_ok(cudaMemsetAsync(pose_ticket_.p, 0, pose_ticket_.cap, st), "pose sums"))
         return false;
     r = PoseRed{pose_part_.as<double>(), pose_ticket_.as<unsigned>(), pose_part_.cap / sizeof(double),
@@ -106,7 +115,7 @@ bool Engine::eval_poses(const std::vector<Mat3>& Hs, bool grad, bool hess, std::
     float* coef = pose_coef_.as<float>();
     // a live spline moves the samples of both directions (src/pair.zig:127-150)
     if (!(pose_cps ? ffd_pose_dirs(pose_cps, n, pc.ffd[0], pc.ffd[1]) : ffd_dirs(pc.ffd[0], pc.ffd[1]))) return false;
-    if (!pose_red((int)m, pc.red)) return false;
+    if (!pose_red((int)m, nd, pc.red)) return false;
     const PoseScores ps{exact, coef, pose_score_.as<double>(), hs, hsc};
     if (!cuda_ok(pose_moments(pc, pose_sums_.as<double>(), ps, st), "moments")) return false;
     counts[0] += 1;

@@ -494,7 +494,7 @@ bool Engine::gn_batch_dev(const std::vector<Mat3>& Hs, unsigned iters, const std
     at.a = PoseSide{A.feat.as<float>(), A.feat4.as<float4>(), A.w, A.h};
     at.b = PoseSide{B.feat.as<float>(), B.feat4.as<float4>(), B.w, B.h};
     at.sym = sym, at.hinv = dh;
-    if (!pose_red((int)mt, at.red)) return false;
+    if (!pose_red((int)mt, nd, at.red)) return false;
     tries = at;
     at.n = n, at.mask = act;
     tries.n = (int)nt, tries.mask = valid;

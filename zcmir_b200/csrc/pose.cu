@@ -31,7 +31,7 @@ __device__ __forceinline__ int tri4(int i, int j) {
 }
 
 // The block's k ≤ 48 float64 totals (thread t < k holds total t; the others pass anything) added
-// into out[0 .. k) of row `row` (a pose in one direction) of nblk blocks. With r.part: every block
+// into out[0 .. k) of the launch's row `row` (a pose in one direction) of nblk blocks. With r.part: every block
 // stores its totals at part[(row · cap + block) · k], cap the grid's blocks per row, then the row's
 // last block to finish (the old value of its ticket is nblk − 1) adds them in a fixed order — group
 // g of ⌊256 / k⌋ threads takes blocks g, g + groups, …, and thread t adds the groups' totals 0, 1, …
@@ -96,9 +96,10 @@ __device__ __forceinline__ int warp_first(int lane) {
 struct PoseLaunch {
     const float4* f[2];
     int w[2], h[2];
-    int n;                 // poses
+    int n;                 // poses of the call
+    int p0;                // the launch's first: poses p0 .. p0 + gridDim.y − 1
     int nblk[2];           // blocks per pose of each direction
-    const float* hinv;     // inverse poses: direction 0's n, then direction 1's
+    const float* hinv;     // inverse poses, a row each: direction 0's n, then direction 1's
     PoseFfd ffd[2];
     const unsigned char* mask;
     PoseRed rd;
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(256, FFD ? 2 : U == 1 ? 3 : 1) k_pose_moments(
     __shared__ float red[8][48];
     __shared__ float cps[2 * kFfdMax * kFfdMax];
     __shared__ double tot[48];
-    const int pose = blockIdx.y, d = blockIdx.z, row = d * L.n + pose, nblk = L.nblk[d];
+    const int pose = L.p0 + blockIdx.y, d = blockIdx.z, row = d * L.n + pose, nblk = L.nblk[d];
     if ((int)blockIdx.x >= nblk || (L.mask && !L.mask[pose])) return;  // a masked pose's sums are read by nobody
     const float4 *__restrict__ fa = L.f[d], *__restrict__ fb = L.f[1 - d];
     const int aw = L.w[d], ah = L.h[d], bw = L.w[1 - d], bh = L.h[1 - d];
@@ -491,7 +492,7 @@ __global__ void __launch_bounds__(256, FFD ? 2 : U == 1 ? 3 : 1) k_pose_moments(
     double s = 0.0;
     if (threadIdx.x < kMom)
         for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += (double)red[i][threadIdx.x];
-    if (!block_add(s, kMom, L.out + (size_t)row * kMom, L.rd, row, nblk, tot)) return;
+    if (!block_add(s, kMom, L.out + (size_t)row * kMom, L.rd, d * gridDim.y + blockIdx.y, nblk, tot)) return;
     if (L.host && threadIdx.x < kMom) L.host[(size_t)row * kMom + threadIdx.x] = tot[threadIdx.x];
     if (L.scored && threadIdx.x < 32)
         score_warp(tot, L.exact, 1e-4, L.coef + (size_t)row * kCoef, L.score + row, L.host_score ? L.host_score + row : nullptr);
@@ -518,7 +519,7 @@ __global__ void __launch_bounds__(256) k_pose_tangent(const __grid_constant__ Po
     __shared__ float red[8][48];
     __shared__ float cps[2 * kFfdMax * kFfdMax];
     __shared__ double tot[48];
-    const int pose = blockIdx.y, d = blockIdx.z, row = d * L.n + pose, nblk = L.nblk[d], hess = L.hess;
+    const int pose = L.p0 + blockIdx.y, d = blockIdx.z, row = d * L.n + pose, nblk = L.nblk[d], hess = L.hess;
     if ((int)blockIdx.x >= nblk || (L.mask && !L.mask[pose])) return;  // a masked pose's sums are read by nobody
     const float4 *__restrict__ fa = L.f[d], *__restrict__ fb = L.f[1 - d];
     const int aw = L.w[d], ah = L.h[d], bw = L.w[1 - d], bh = L.h[1 - d];
@@ -651,7 +652,7 @@ __global__ void __launch_bounds__(256) k_pose_tangent(const __grid_constant__ Po
     double s = 0.0;
     if (threadIdx.x < kGrad)
         for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += (double)red[i][threadIdx.x];
-    if (!block_add(s, kGrad, L.out + (size_t)row * kGrad, L.rd, row, nblk, tot)) return;
+    if (!block_add(s, kGrad, L.out + (size_t)row * kGrad, L.rd, d * gridDim.y + blockIdx.y, nblk, tot)) return;
     if (L.host && threadIdx.x < kGrad) L.host[(size_t)row * kGrad + threadIdx.x] = tot[threadIdx.x];
 }
 
@@ -1058,13 +1059,14 @@ size_t pose_red_need(size_t pixels, int n) {
 }
 
 namespace {
-// the launch's images, blocks and poses; rows: poses × directions
+// the call's images, blocks per row and poses; g.y: the poses of a launch, as many as the scratch holds
+// rows for (and a grid has rows). A pose's sums do not depend on which poses share its launch.
 cudaError_t pose_launch(const PoseCall& c, int slot, int k, PoseLaunch& L, dim3& g) {
     for (const PoseFfd& f : c.ffd)
         if (f.cps && (f.g < 2 || f.g > kFfdMax)) return cudaErrorInvalidValue;
     const int nd = c.sym ? 2 : 1;
     const PoseSide* side[2] = {&c.a, &c.b};
-    g = dim3(1, c.n, nd);
+    g = dim3(1, 1, nd);
     for (int d = 0; d < 2; ++d) {
         L.f[d] = side[d]->feat4, L.w[d] = side[d]->w, L.h[d] = side[d]->h;
         const PoseSide& dst = *side[1 - d];
@@ -1072,10 +1074,23 @@ cudaError_t pose_launch(const PoseCall& c, int slot, int k, PoseLaunch& L, dim3&
         if (d < nd) g.x = std::max(g.x, (unsigned)L.nblk[d]);
         L.ffd[d] = c.ffd[d];
     }
-    if (!red_fits(c.red, nd * c.n, (int)g.x, k)) return cudaErrorInvalidValue;
+    if (!red_fits(c.red, nd, (int)g.x, k)) return cudaErrorInvalidValue;
+    g.y = (unsigned)std::min(c.n, 65535);
+    if (c.red.part) g.y = (unsigned)std::min<size_t>(g.y, std::min(c.red.tickets, c.red.cap / ((size_t)g.x * k)) / nd);
     L.n = c.n, L.hinv = c.hinv, L.mask = c.mask, L.rd = c.red;
     L.n_inl = c.hinv_host && nd * c.n <= kPoseInline ? nd * c.n : 0;
     for (int i = 0; i < 9 * L.n_inl; ++i) L.inl[i] = c.hinv_host[i];
+    return cudaSuccess;
+}
+
+// launch(grid, poses) for every g.y poses of the call, in order
+template <class K>
+cudaError_t pose_launches(int n, dim3 g, PoseLaunch& L, K&& launch) {
+    for (const int step = (int)g.y; L.p0 < n; L.p0 += step) {
+        g.y = (unsigned)std::min(step, n - L.p0);
+        launch(g);
+        if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
+    }
     return cudaSuccess;
 }
 }  // namespace
@@ -1090,14 +1105,15 @@ cudaError_t pose_moments(const PoseCall& c, double* sums, const PoseScores& sc, 
     L.out = sums, L.host = sc.host_sums;
     L.scored = sc.score != nullptr && c.red.part, L.exact = sc.exact ? 1 : 0;
     L.coef = sc.coef, L.score = sc.score, L.host_score = sc.host_score;
-    if (!c.red.part && (e = cudaMemsetAsync(sums, 0, (size_t)g.y * g.z * kMom * sizeof(double), st)) != cudaSuccess) return e;
+    if (!c.red.part && (e = cudaMemsetAsync(sums, 0, (size_t)c.n * g.z * kMom * sizeof(double), st)) != cudaSuccess) return e;
     // Launches of fewer blocks than SMs (a pose or two of an ordinary image) keep four pixels' taps in
     // flight: a 256² pair's score takes 33 µs from call to result, 36 with one. Fuller launches lose
     // more warps to the registers than they gain (two pixels: 8 % slower).
-    if (ffd) k_pose_moments<true, 1><<<g, 256, 0, st>>>(L);
-    else if ((int)(g.x * g.y * g.z) <= kernel_slots()[1] / 3) k_pose_moments<false, 4><<<g, 256, 0, st>>>(L);
-    else k_pose_moments<false, 1><<<g, 256, 0, st>>>(L);
-    return cudaGetLastError();
+    return pose_launches(c.n, g, L, [&](dim3 b) {
+        if (ffd) k_pose_moments<true, 1><<<b, 256, 0, st>>>(L);
+        else if ((int)(b.x * b.y * b.z) <= kernel_slots()[1] / 3) k_pose_moments<false, 4><<<b, 256, 0, st>>>(L);
+        else k_pose_moments<false, 1><<<b, 256, 0, st>>>(L);
+    });
 }
 
 cudaError_t pose_tangent(const PoseCall& c, const float* coef, const float* gens, bool hess, double* out, double* host,
@@ -1110,10 +1126,11 @@ cudaError_t pose_tangent(const PoseCall& c, const float* coef, const float* gens
     if (e != cudaSuccess) return e;
     L.out = out, L.host = host, L.coef = const_cast<float*>(coef), L.hess = hess ? 1 : 0;
     for (int i = 0; i < 144; ++i) L.gens[i] = gens[i];
-    if (!c.red.part && (e = cudaMemsetAsync(out, 0, (size_t)g.y * g.z * kGrad * sizeof(double), st)) != cudaSuccess) return e;
-    if (ffd) k_pose_tangent<true><<<g, 256, 0, st>>>(L);
-    else k_pose_tangent<false><<<g, 256, 0, st>>>(L);
-    return cudaGetLastError();
+    if (!c.red.part && (e = cudaMemsetAsync(out, 0, (size_t)c.n * g.z * kGrad * sizeof(double), st)) != cudaSuccess) return e;
+    return pose_launches(c.n, g, L, [&](dim3 b) {
+        if (ffd) k_pose_tangent<true><<<b, 256, 0, st>>>(L);
+        else k_pose_tangent<false><<<b, 256, 0, st>>>(L);
+    });
 }
 
 cudaError_t pose_ffd_cells(const PoseSide& a, const PoseSide& b, const float* hinv, const float* hpose,
