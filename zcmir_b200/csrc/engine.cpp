@@ -74,6 +74,7 @@ CorrPlanDev corr_plan_dev(bool exact, bool three, int box_mode) {
 }
 
 Engine::Engine(int dev) : device(dev) {
+    if (const char* v = getenv("ZCMIR_B200_ROW_PASS")) row_pass = v;
     if (const char* v = getenv("ZCMIR_B200_SPECTRA_CACHE")) spectra_cache_ = atoi(v) != 0;
     cudaSetDevice(dev);
     cudaGetDeviceProperties(&prop, dev);
@@ -778,12 +779,13 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
         counts[0] += 1;
     }
     if (!ev && !st_after_aux()) return false;
-    const bool tmem = job.box.mode == 0 && rows_tmem_supported(g.nx, job.plan.n_corr);
+    const bool tmem = row_pass != "split" && job.box.mode == 0 && rows_tmem_supported(g.nx, job.plan.n_corr);
     job.box.ta = box_a_.as<float>(), job.box.tb = box_b_.as<float>();
     if (!tmem &&
         !cuda_ok(inverse_rows(q_.as<float2>(), g, job.plan, job.line, job.S, twiddles(g.nx), st), "inverse rows"))
         return false;
     auto scores = [&](int y0, int rows) {
+        counts[0] += 1;
         if (tmem)
             return cuda_ok(inverse_rows_score_tmem(q_.as<float2>(), g, job.plan, twiddles(g.nx), job.cp, n00,
                                                    map_.as<float>(), best, zero, st, y0, rows),
@@ -819,7 +821,7 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
         return false;
     }
     rec(5);
-    counts[0] += 5;  // zero lag, inverse columns, rows, scores, result
+    counts[0] += tmem ? 2 : 3;  // the zero lag, the inverse columns, the rows where they are a pass of their own
     return true;
 }
 

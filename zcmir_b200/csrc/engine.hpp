@@ -204,7 +204,10 @@ class Engine {
     // counters since the last zc_gpu_counts: launches, submits, reads, waits
     uint32_t counts[4] = {0, 0, 0, 0};
     bool profiling = false;
-    // profiling (zc_profile):
+    // the last pass of maps with 2048-point rows and no moment tables: "tmem" (rows and score in one kernel,
+    // the sums in tensor memory) or "split" (the two passes every other map takes); from ZCMIR_B200_ROW_PASS
+    // at creation, "tmem" by default
+    std::string row_pass = "tmem";
     std::map<std::string, std::pair<double, uint32_t>> prof;  // name → (ms, count)
 
     bool fail(const std::string& m);
