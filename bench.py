@@ -3,8 +3,9 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
 One step = one full shift map of the pair at the identity pose (canvas → both sides' real planes
-→ forward FFTs → 45 correlation products → inverse FFTs → per-shift exact, calibrated score →
-argmax), the images' features resident in HBM. Device time per step is taken with CUDA events
+→ forward FFTs and moment tables → correlation products → inverse FFTs → per-shift exact, calibrated
+score of all 45 correlation sums → argmax; at a translation 18 of the 45 are transformed and 27 are read
+from the tables), the images' features resident in HBM. The roofline fractions count the work that ran. Device time per step is taken with CUDA events
 on the engine's stream, W untimed steps first, an L2 flush (a 256 MB write) between timed steps
 outside the timed spans. `e2e` is the same metric through the public API (Engine.set_images
 from pinned host buffers + Engine.shift_map copying the map back to pinned host memory).
@@ -134,7 +135,7 @@ def stage_bytes(p):
     a cell) of the sides whose moments are not transformed."""
     nx, ny, cw, ch, P, C = p["nx"], p["ny"], p["cw"], p["ch"], p["n_real"], p["n_corr"]
     half = (nx // 2 + 1) * 8
-    tables = {18: 2, 11: 2, 32: 1, 20: 1}.get(C, 0)
+    tables = tabled_sides(p)
     return {
         "canvas": 2 * (5 * p["canvas_w"] * p["canvas_h"] * 4) * 2 + tables * cw * ch * (2 * 20 + 64),
         "fwd_rows": 2 * 5 * cw * ch * 4 + P * ch * half,
@@ -200,23 +201,25 @@ def sweep_work(tuned, Fx, Fy):
     return total_b, total_f
 
 
-def survey_bytes(p):
-    """The whole map's compulsory HBM bytes (both stacks read, both sides' half spectra of all 15
-    planes written and read once, the map written)."""
-    nx, ny, P = p["nx"], p["ny"], 15
-    return 2 * 5 * p["canvas_w"] * p["canvas_h"] * 4 + 2 * (2 * P * nx * (ny // 2 + 1) * 8) + nx * ny * 4
+def tabled_sides(p):
+    """How many sides' moment sums a map reads from summed-area tables, from its transformed correlations
+    (45 or 28 of four or three features: none; without the tabled ones 32 or 20, then 18 or 11)."""
+    return {18: 2, 11: 2, 32: 1, 20: 1}.get(p["n_corr"], 0)
 
 
-def survey_flops(p):
-    """The whole map's FP32 flops by the survey's counting rule: both sides' forward FFTs over the
-    canvas rows and all columns (packed complex lines), the inverse 2-D FFTs of the packed
-    correlations, the conjugate products and about 300 flops of scoring per shift. The rule counts the
-    method's 15 planes and 45 correlations, of which a map transforms those in its plan."""
-    nx, ny, ch, P, C = p["nx"], p["ny"], p["ch"], 15, 45
+def map_work(p):
+    """(bytes, flops) of one map as it ran: n_real planes of both sides and n_corr correlations transformed,
+    the other sums read from tables. Bytes: both stacks read, those half spectra and the tables (64 bytes a
+    cell) written and read once, the map written. FP32 flops by the survey's counting rule: forward FFTs
+    over the canvas rows and all columns and inverse 2-D FFTs, two real planes to a complex line, the
+    conjugate products and about 300 flops of scoring per shift."""
+    nx, ny, cw, ch, P, C = p["nx"], p["ny"], p["cw"], p["ch"], p["n_real"], p["n_corr"]
     lx, ly = np.log2(nx), np.log2(ny)
-    fwd = 2 * ((P + 1) // 2) * 5 * (nx * lx * ch + ny * ly * nx)
-    inv = ((C + 1) // 2) * 5 * nx * ny * np.log2(nx * ny)
-    return float(fwd + inv + 10 * C * nx * ny + 300 * nx * ny)
+    b = (2 * 5 * p["canvas_w"] * p["canvas_h"] * 4 + 2 * P * ny * (nx // 2 + 1) * 8 + 2 * tabled_sides(p) * cw * ch * 64
+         + nx * ny * 4)
+    f = (P / 2 * 5 * (nx * lx * ch + ny * ly * nx) + C / 2 * 5 * nx * ny * np.log2(nx * ny) + 10 * C * nx * ny
+         + 300 * nx * ny)
+    return b, float(f)
 
 
 def fp32_peak_tflops():
@@ -579,6 +582,7 @@ def run_gpu(args, rank, ws, local):
         if tf.exists():
             traffic = json.loads(tf.read_text()).get(top)
         fp32 = fp32_peak_tflops()
+        work_b, work_f = map_work(r)
         line = {
             "metric": METRIC, "value": ws * 1000.0 / ms, "unit": "maps/s", "n_gpus": ws, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
@@ -596,12 +600,11 @@ def run_gpu(args, rank, ws, local):
                                            "of an earlier run of this command (profiles/traffic.json), not measured by this run",
                          "peak_source": peak_kind,
                          "algorithmic_bytes_per_launch": b_launch, "launch_ms": t_launch,
-                         "map_algorithmic_bytes": survey_bytes(r),
-                         "map_frac": survey_bytes(r) / (ms * 1e-3) / 1e9 / hbm,
-                         "map_fp32": {"flops_per_map": survey_flops(r),
-                                      "tflops": survey_flops(r) / (ms * 1e-3) / 1e12,
+                         "map_algorithmic_bytes": work_b,
+                         "map_frac": work_b / (ms * 1e-3) / 1e9 / hbm,
+                         "map_fp32": {"flops_per_map": work_f, "tflops": work_f / (ms * 1e-3) / 1e12,
                                       "peak_tflops": fp32, "peak_source": "measured in this run (zcb_fp32_peak)",
-                                      "frac": (survey_flops(r) / (ms * 1e-3) / 1e12 / fp32) if fp32 else None}},
+                                      "frac": (work_f / (ms * 1e-3) / 1e12 / fp32) if fp32 else None}},
             "e2e": {"value": ws / e2e_s, "unit": "maps/s", "h2d_bytes_per_step": int(pm.nbytes + pf.nbytes),
                     "d2h_bytes_per_step": int(2048 * 2048 * 4 + 88)},
             "gpu_launches": int(launches),
