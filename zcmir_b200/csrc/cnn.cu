@@ -376,8 +376,8 @@ struct Net {
         return false;
     }
     // Every buffer from one allocation, out of the calls' memory pool: a network lives for one call, and
-    // two dozen cudaMallocs and frees took 5 of the 6.6 ms of a 64-pair forward call, now 1.3 (one of each still
-    // 0.9). What: 0 forward, 1 gradients, 2 training.
+    // two dozen cudaMallocs and frees took 5 of the 6.6 ms of a 64-pair forward call, now 1.4 to 1.7 (one of
+    // each still 0.9). What: 0 forward, 1 gradients, 2 training.
     bool alloc(int batch, int what) {
         B = batch;
         if (!ok(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream")) return false;

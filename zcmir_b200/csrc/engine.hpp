@@ -234,8 +234,8 @@ class Engine {
     // maps
     BoxSums box_sums(const MapJob& job) const;
     bool plan_map(const Mat3& H, bool exact, bool calibrated, unsigned cap, double min_overlap, MapJob& job);
-    // host_map (nullable): with the tensor-memory row pass, the map is copied there in row
-    // chunks on the copy stream during the pass (the caller synchronises copy_st_)
+    // host_map (nullable): the map is copied there in chunks of rows on the copy stream while the
+    // next chunk is scored (the caller synchronises copy_st_)
     bool run_map(MapJob& job, cudaEvent_t* ev /* kNumStages+1 events or null */, float* host_map = nullptr);
     bool shift_map(const Mat3& H, bool exact, bool calibrated, unsigned cap, double min_overlap, zc_shift_result* out,
                    float* map, size_t map_len);

@@ -434,7 +434,7 @@ void Engine::sweep_make_peaks(SweepOut& out, int n_peak) {
 }
 
 // gn_batch with the loop on the device: per iteration the poses' inverse maps, their moments,
-// coefficients and tangent sums (masked to the poses still moving), then one warp per pose builds
+// coefficients and tangent sums (masked to the poses still moving), then a block per pose builds
 // the candidates (k_gn_propose), the candidates are scored, and k_gn_select keeps the first that
 // beats each pose's score. The host reads the moved flags once per kGnBatch iterations, to stop
 // when no pose moves; the iterations past the last move only launch masked-out kernels.

@@ -199,17 +199,18 @@ struct PoseFfd {
     int source = 0;
     int stride = 0;  // floats between poses' control points (0: one set for every pose)
 };
-// How a pose's blocks add their float64 totals. With part set, each block stores its totals in
-// part and the pose's last block to finish adds them in block order, so the sums are the same on
-// every run and in every batch; ticket: one counter per pose of the launch, zero before it (each
-// is put back to zero). Without part: float64 atomics, in the order the blocks finish.
+// How the blocks of a row (a pose in one direction) add their float64 totals. With part set, each block
+// stores its totals in part and the row's last block to finish adds them in block order, so the sums are
+// the same on every run and in every batch; ticket: one counter per row of a launch, zero before it (each
+// is put back to zero). A call of more rows than part and ticket hold runs as several launches. Without
+// part: float64 atomics, in the order the blocks finish.
 struct PoseRed {
     double* part = nullptr;
     unsigned* ticket = nullptr;
     size_t cap = 0;      // doubles at part
     size_t tickets = 0;  // counters at ticket
 };
-// doubles of PoseRed::part any pose kernel needs for n poses onto an image of `pixels` pixels
+// doubles of PoseRed::part any pose kernel needs for n rows onto an image of `pixels` pixels
 size_t pose_red_need(size_t pixels, int n);
 // The pose kernels' launch shape (zc_tune_parts): pixels per thread, the least and the most
 // blocks per pose (0 keeps the current value). It changes the order of the cross-block sums, so

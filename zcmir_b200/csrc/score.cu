@@ -3,7 +3,8 @@
 // Plane k of an item is ny rows of 2·WP floats (the rows pass writes them over the half spectra). A
 // block scores 256 shifts at a time, one a thread, of the padded rows laid end to end; while it does,
 // the next 256 shifts' sums are copied to shared memory (cp.async, 16 bytes a copy), so the float64
-// centring and Cholesky wait on no load of a plane and spend no instructions on its address. A 1296 ×
+// centring and Cholesky wait on no load of a plane and spend no instructions on its address. With moment
+// tables (modes 1 and 2) a shift's 16 or 32 corner reads are plain loads in front of them. A 1296 ×
 // 1536 map of 45 correlations: rows 403 + score 109 µs, against 3643 µs with the row's sums held in
 // shared memory; the sweep's 104 maps of 192²: 455 + 144 against 608 µs.
 #include "box.cuh"

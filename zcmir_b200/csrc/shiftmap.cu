@@ -215,9 +215,10 @@ cudaError_t inverse_columns(const float2* ha, const float2* hb, const MapGeom& g
     return dispatch_pass(Pass::InvCols, col, a, st);
 }
 
-// Rows of 972 to 1944 points (but 1024) of plans whose row of sums is large are split in two. The
-// transform takes the same time either way; the split keeps the rounding of the sums, and with it
-// which shifts sit on the overlap floor, that these rows have always had.
+// Even rows of up to 1944 points, but 1024, whose plan has over 40000 sums a row (45 correlations: from
+// 972 points on; 28: from 1458) are split in two. The transform takes the same time either way; the split
+// keeps the rounding of the sums, and with it which shifts sit on the overlap floor, that these rows have
+// always had. n_corr: the plan's correlations, tabled ones among them.
 int row_split(int nx, int n_corr) {
     return nx % 2 == 0 && nx != 1024 && nx < 2048 && n_corr * nx > 40000 ? 2 : 1;
 }

@@ -7,8 +7,10 @@
 
 Maps: builds the seeded segmented pair (zcmir_b200.synth.pair_segmented) at n², uploads it, then
 runs `--maps` maps at the identity pose (exact, calibrated) through the C ABI, printing the plan
-and the peak. Each map launches, in order: warp_stack, paste_stack, lag0, fwd_rows ×2, cols ×2,
-inv_cols, inv_rows. --dft-stage P (1–3): the forward column FFTs' first stage on the tensor
+and the peak. Each map launches, on the engine's stream: warp_stack, paste_stack, fwd_rows ×2, cols ×2
+(of a side's samples, then of its products where they are transformed), inv_cols, pair_area, inv_rows
+and score (rows_tmem in place of both for 2048-point rows without tables); beside them lag0 and, per side
+whose moments are tabled, box_sums, box_scan and box_write. --dft-stage P (1–3): the forward column FFTs' first stage on the tensor
 cores in P BF16 pieces (zcb_set_dft_stage; cols ×2 become k_dft16_tc, cols, copy per side).
 --stages: per-stage device times of the maps after the first (CUDA events, zc_profile_report).
 
@@ -16,13 +18,13 @@ Sweeps (--sweep): the seeded similarity pair (zcmir_b200.synth.pair_similarity) 
 `--maps` sweeps of nth rotations × ns scales in [0.8, 1.25] on a 128² canvas (3240 candidate maps
 by default) through zcb_sweep. Each sweep launches interleave ×2 and the fixed window's pack, then
 per plane size the fixed window's fwd_rows and cols, then per batch pack, fwd_rows, cols,
-inv_cols, rows and peaks.
+inv_cols, inv_rows, score and peaks.
 
 Searches (--search): the same pair and sweep grid, then `--maps` whole searches from the
 identity pose (the sweep, its peaks' non-maximum suppression, the batched Gauss–Newton screen and
-the finalists' climbs): after the sweep's launches, each Gauss–Newton step evaluates its poses
-with pose_moments (forward and inverse direction), pose_coefs and, for the gradient,
-pose_tangent.
+the finalists' climbs): after the sweep's launches, each Gauss–Newton step launches
+gn_hinv, pose_moments (both directions, scored), pose_tangent, gn_propose, and for its candidates gn_hinv,
+pose_moments and gn_select.
 """
 import argparse
 
