@@ -59,9 +59,9 @@ bool Engine::pose_red(int n, int least, PoseRed& r) {
     const size_t px = std::max((size_t)side[0].w * side[0].h, (size_t)side[1].w * side[1].h);
     const size_t row = pose_red_need(px, 1) * sizeof(double), lo = (size_t)std::max(least, 1);
     size_t rows = std::max(lo, std::min((size_t)std::max(n, 1), kPoseScratch / row));
-    while (pose_part_.ensure(rows * row) != cudaSuccess) {
-        if (cudaGetLastError() != cudaErrorMemoryAllocation || rows == lo) return fail("pose sums: out of device memory");
-        rows = std::max(lo, rows / 2);
+    for (cudaError_t e; (e = pose_part_.ensure(rows * row)) != cudaSuccess; rows = std::max(lo, rows / 2)) {
+        if (e != cudaErrorMemoryAllocation || rows == lo) return cuda_ok(e, "pose sums");
+        cudaGetLastError();
     }
     const uint64_t gen = pose_ticket_.gen;
     if (!cuda_ok(pose_ticket_.ensure(rows * sizeof(unsigned)), "pose sums")) return false;
