@@ -131,17 +131,16 @@ class Clocks:
 def stage_bytes(p):
     """Algorithmic bytes of each stage of one map (one launch of that kernel per side where it
     runs per side): its compulsory reads and writes in this decomposition. P: the planes both sides
-    transform; the canvas stage also reads the samples twice and writes the moment tables (64 bytes
-    a cell) of the sides whose moments are not transformed."""
+    transform; the canvas stage also reads the samples twice and writes the moment tables
+    of the sides whose moments are not transformed."""
     nx, ny, cw, ch, P, C = p["nx"], p["ny"], p["cw"], p["ch"], p["n_real"], p["n_corr"]
     half = (nx // 2 + 1) * 8
-    tables = tabled_sides(p)
     return {
-        "canvas": 2 * (5 * p["canvas_w"] * p["canvas_h"] * 4) * 2 + tables * cw * ch * (2 * 20 + 64),
+        "canvas": 2 * (5 * p["canvas_w"] * p["canvas_h"] * 4) * 2 + tabled_sides(p) * cw * ch * 2 * 20 + table_bytes(p),
         "fwd_rows": 2 * 5 * cw * ch * 4 + P * ch * half,
         "fwd_cols": P * ch * half + P * ny * half,
         "inv_cols": P * ny * half + C * ny * half,
-        "inv_rows_score": C * ny * half + tables * cw * ch * 64 + nx * ny * 4,
+        "inv_rows_score": C * ny * half + table_bytes(p) + nx * ny * 4,
     }
 
 
@@ -207,15 +206,20 @@ def tabled_sides(p):
     return {18: 2, 11: 2, 32: 1, 20: 1}.get(p["n_corr"], 0)
 
 
+def table_bytes(p):
+    """Those sides' tables: 14 or 9 float64 sums a cell (four or three features; padded to pairs)."""
+    return tabled_sides(p) * p["cw"] * p["ch"] * (80 if p["n_corr"] in (11, 20) else 112)
+
+
 def map_work(p):
     """(bytes, flops) of one map as it ran: n_real planes of both sides and n_corr correlations transformed,
-    the other sums read from tables. Bytes: both stacks read, those half spectra and the tables (64 bytes a
-    cell) written and read once, the map written. FP32 flops by the survey's counting rule: forward FFTs
+    the other sums read from tables. Bytes: both stacks read, those half spectra and the tables written and
+    read once, the map written. FP32 flops by the survey's counting rule: forward FFTs
     over the canvas rows and all columns and inverse 2-D FFTs, two real planes to a complex line, the
     conjugate products and about 300 flops of scoring per shift."""
     nx, ny, cw, ch, P, C = p["nx"], p["ny"], p["cw"], p["ch"], p["n_real"], p["n_corr"]
     lx, ly = np.log2(nx), np.log2(ny)
-    b = (2 * 5 * p["canvas_w"] * p["canvas_h"] * 4 + 2 * P * ny * (nx // 2 + 1) * 8 + 2 * tabled_sides(p) * cw * ch * 64
+    b = (2 * 5 * p["canvas_w"] * p["canvas_h"] * 4 + 2 * P * ny * (nx // 2 + 1) * 8 + 2 * table_bytes(p)
          + nx * ny * 4)
     f = (P / 2 * 5 * (nx * lx * ch + ny * ly * nx) + C / 2 * 5 * nx * ny * np.log2(nx * ny) + 10 * C * nx * ny
          + 300 * nx * ny)

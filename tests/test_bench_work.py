@@ -18,7 +18,7 @@ def test_a_map_is_credited_with_what_it_transforms(n_real, n_corr, tables):
     p = plan(n_real, n_corr)
     b, f = bench.map_work(p)
     half = p["ny"] * (p["nx"] // 2 + 1) * 8
-    assert b == 2 * 5 * 1024 * 700 * 4 + 2 * n_real * half + 2 * tables * 1024 * 700 * 64 + 2048 * 1536 * 4
+    assert b == 2 * 5 * 1024 * 700 * 4 + 2 * n_real * half + 2 * tables * 1024 * 700 * (80 if n_corr in (20, 11) else 112) + 2048 * 1536 * 4
     plane = 2.5 * 2048 * (11 * 700 + np.log2(1536) * 1536)
     corr = (2.5 * np.log2(2048 * 1536) + 10) * 2048 * 1536
     assert f == pytest.approx(n_real * plane + n_corr * corr + 300 * 2048 * 1536, rel=1e-12)

@@ -7,19 +7,20 @@
 // a plane's forward transforms, a product spectrum and two inverse passes. A 1024² pair at a
 // translation transforms 18 correlations and 5 planes per side instead of 45 and 15: inverse columns
 // 369 → 158 µs, inverse rows 393 → 169, forward rows 183 → 90, forward columns 240 → 85, for three
-// launches of 20 + 28 + 30 µs a side beside them (each alone on the card). At a turned pose 32
+// launches of 21 + 33 + 44 µs a side beside them (each alone on the card). At a turned pose 32
 // correlations and 5 + 15 planes are left.
 //
 // Precision: products f_i² are tabled less the weight (their mean over the image is 1 by the
 // whitening; n is added back from the overlap), so entries stay near the field's own excursions. Sums
-// within a tile, the stored prefixes and the entries are float32; the scans over tiles and bands and an
-// entry's last addition are float64. Rms error of a box sum, float32 transform against table, over the 14
-// planes and 400 boxes: 4.6e-3 / 4.3e-4 for blobs of 512², 5.2e-3 / 1.5e-3 under an illumination ramp,
-// 5.7e-3 / 1.6e-3 over a step; at 1500² 6.2e-2 / 1.6e-3 to 7.5e-2 / 7.6e-3. A map's own error is mostly its
-// transformed correlations': its rms is 0.82 to 1.15 of that with all 45 transformed at overlaps of 8 % and
-// more, and up to 1.35 (a step, calibrated) under 2 %.
+// within a tile are float32; those of the tiles and bands, the entries and a box's four corners are
+// float64, so a sum's error scales with its own box, where a float32 transform's scales with both planes'
+// energy: rms 0.04 (300² over 1000 × 900) to 0.8 (8² over 40²) of a transform's over 14 planes, blobs,
+// ramps and flat halves. Float32 entries were not enough: on 300 translations of pairs of 8 to 420
+// pixels a side, half of them ramps, steps or flat halves, the map's argmax left the float64 oracle's 11
+// times against 5 with all 45 correlations transformed; now 4 times, the rms error of cells 0.92 of theirs.
+// It costs a map of 1024² 0.1 ms (score 262 → 326 µs, tables 78 → 98).
 //
-// Built from tiles of 32 columns × 8 rows, a warp each, in three launches, so that the table (64
+// Built from tiles of 32 columns × 8 rows, a warp each, in three launches, so that the table (112
 // bytes a cell) is written once and the samples (20 bytes) are read twice: k_box_sums leaves each
 // tile's column, row and total sums; k_box_scan turns them into what lies above, left and above-left
 // of a tile; k_box_write walks a tile's rows with the columns' running sums in registers and scans
@@ -37,14 +38,14 @@ constexpr int kWarps = 4;  // tiles per block, side by side
 
 // a table's scratch: column sums [band][comp][x], row sums [y][tile][comp], totals [band][tile][comp]
 struct BoxScratch {
-    float *col, *row, *tot;
+    double *col, *row, *tot;
     int nband, ntile;
 };
 __host__ BoxScratch scratch(void* p, int nf, int cw, int ch) {
     const int nc = box_comps(nf);
     BoxScratch s;
     s.nband = (ch + kRows - 1) / kRows, s.ntile = (cw + kTile - 1) / kTile;
-    s.col = static_cast<float*>(p);
+    s.col = static_cast<double*>(p);
     s.row = s.col + (size_t)s.nband * cw * nc;
     s.tot = s.row + (size_t)ch * s.ntile * nc;
     return s;
@@ -124,17 +125,17 @@ __global__ void __launch_bounds__(32 * kWarps) k_box_sums(const float* __restric
     if (owner) sc.tot[((size_t)b * sc.ntile + tile) * NC + comp] = tot;
 }
 
-// exclusive scan of n values `step` apart by one thread in float64, 16 loads in flight
-__device__ __forceinline__ void scan_serial(float* p, int n, size_t step) {
+// exclusive scan of n values `step` apart by one thread, 16 loads in flight
+__device__ __forceinline__ void scan_serial(double* p, int n, size_t step) {
     double a = 0.0;
     for (int i0 = 0; i0 < n; i0 += 16) {
-        float v[16];
+        double v[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = i0 + i < n ? p[(i0 + i) * step] : 0.f;
+        for (int i = 0; i < 16; ++i) v[i] = i0 + i < n ? p[(i0 + i) * step] : 0.0;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            if (i0 + i < n) p[(i0 + i) * step] = (float)a;
-            a += (double)v[i];
+            if (i0 + i < n) p[(i0 + i) * step] = a;
+            a += v[i];
         }
     }
 }
@@ -158,17 +159,28 @@ __global__ void __launch_bounds__(256) k_box_scan(BoxScratch sc, int nc, int cw,
 
 template <int NF>
 __global__ void __launch_bounds__(32 * kWarps) k_box_write(const float* __restrict__ grid, int cw, int ch, BoxScratch sc,
-                                                           float* __restrict__ t) {
+                                                           double* __restrict__ t) {
     constexpr int NC = box_comps(NF), NP = box_pad(NF);
     const int lane = threadIdx.x & 31, tile = blockIdx.x * kWarps + (threadIdx.x >> 5), b = blockIdx.y;
     if (tile >= sc.ntile) return;
     const int x = tile * kTile + lane;
     const size_t gn = (size_t)cw * ch;
     const bool in = x < cw;
-    double left = lane < NC ? (double)sc.tot[((size_t)b * sc.ntile + tile) * NC + lane] : 0.0;  // lane c: comp c
-    float run[NC];  // this column down to the row
+    double left = lane < NC ? sc.tot[((size_t)b * sc.ntile + tile) * NC + lane] : 0.0;  // lane c: comp c
+    // what lies above the band in the tile's columns up to this one; within it, this column down to the row
+    double above[NC];
+    float run[NC];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) run[c] = in ? sc.col[((size_t)b * NC + c) * cw + x] : 0.f;
+    for (int c = 0; c < NC; ++c) {
+        double u = in ? sc.col[((size_t)b * NC + c) * cw + x] : 0.0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double w = __shfl_up_sync(0xffffffffu, u, o);
+            if (lane >= o) u += w;
+        }
+        above[c] = u;
+        run[c] = 0.f;
+    }
 #pragma unroll 2
     for (int r = 0; r < kRows; ++r) {
         const int y = b * kRows + r;
@@ -176,11 +188,11 @@ __global__ void __launch_bounds__(32 * kWarps) k_box_write(const float* __restri
         float s[1 + NF], v[NC];
         load_cell<NF>(s, grid, gn, cw, x, y, in);
         comps_of<NF>(v, s);
-        if (lane < NC) left += (double)sc.row[((size_t)y * sc.ntile + tile) * NC + lane];
-        float o4[NP];
+        if (lane < NC) left += sc.row[((size_t)y * sc.ntile + tile) * NC + lane];
+        double o2[NP];
 #pragma unroll
         for (int c = 0; c < NP; ++c) {
-            o4[c] = 0.f;
+            o2[c] = 0.0;
             if (c >= NC) continue;
             run[c] += v[c];
             float u = run[c];
@@ -189,18 +201,18 @@ __global__ void __launch_bounds__(32 * kWarps) k_box_write(const float* __restri
                 const float w = __shfl_up_sync(0xffffffffu, u, o);
                 if (lane >= o) u += w;
             }
-            o4[c] = (float)(__shfl_sync(0xffffffffu, left, c) + (double)u);
+            o2[c] = __shfl_sync(0xffffffffu, left, c) + (above[c] + (double)u);
         }
         if (in) {
-            float4* p = reinterpret_cast<float4*>(t) + (size_t)y * (NP / 4) * cw + x;
+            double2* p = reinterpret_cast<double2*>(t) + (size_t)y * (NP / 2) * cw + x;
 #pragma unroll
-            for (int q = 0; q < NP / 4; ++q) p[(size_t)q * cw] = make_float4(o4[4 * q], o4[4 * q + 1], o4[4 * q + 2], o4[4 * q + 3]);
+            for (int q = 0; q < NP / 2; ++q) p[(size_t)q * cw] = make_double2(o2[2 * q], o2[2 * q + 1]);
         }
     }
 }
 
 template <int NF>
-cudaError_t build(const float* grid, int cw, int ch, float* t, void* tmp, cudaStream_t st) {
+cudaError_t build(const float* grid, int cw, int ch, double* t, void* tmp, cudaStream_t st) {
     constexpr int NC = box_comps(NF);
     const BoxScratch sc = scratch(tmp, NF, cw, ch);
     const dim3 g((sc.ntile + kWarps - 1) / kWarps, sc.nband);
@@ -213,13 +225,13 @@ cudaError_t build(const float* grid, int cw, int ch, float* t, void* tmp, cudaSt
 
 }  // namespace
 
-size_t box_table_bytes(int nf, int cw, int ch) { return (size_t)box_pad(nf) * ch * cw * sizeof(float); }
+size_t box_table_bytes(int nf, int cw, int ch) { return (size_t)box_pad(nf) * ch * cw * sizeof(double); }
 size_t box_scratch_bytes(int nf, int cw, int ch) {
     const size_t nb = (ch + kRows - 1) / kRows, nt = (cw + kTile - 1) / kTile;
-    return (nb * cw + ch * nt + nb * nt) * box_comps(nf) * sizeof(float);
+    return (nb * cw + ch * nt + nb * nt) * box_comps(nf) * sizeof(double);
 }
 
-cudaError_t box_table(const float* grid, int cw, int ch, int nf, float* t, void* tmp, cudaStream_t st) {
+cudaError_t box_table(const float* grid, int cw, int ch, int nf, double* t, void* tmp, cudaStream_t st) {
     return nf == 3 ? build<3>(grid, cw, ch, t, tmp, st) : build<4>(grid, cw, ch, t, tmp, st);
 }
 

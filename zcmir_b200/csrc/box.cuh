@@ -6,11 +6,15 @@
 namespace zc {
 
 // Comps of a table of nf features: the nf feature sums, then the products in row order, padded to
-// whole float4s. Quad q of entry (x, y), the sums over rows ≤ y and columns ≤ x, is the float4 at
-// (y·quads + q)·cw + x: a warp's entries of consecutive columns are consecutive in memory (whole
+// whole double2s. Pair q of entry (x, y), the sums over rows ≤ y and columns ≤ x, is the double2 at
+// (y·pairs + q)·cw + x: a warp's entries of consecutive columns are consecutive in memory (whole
 // entries side by side made each load touch four times the cache lines).
+//
+// Entries are float64: the four of a box cancel down to its own sum, and rounding that scales with the
+// whole plane's sums would be left in it (a 40 × 8 image over one of 360 × 337, whose covariances are near
+// singular, had the wrong peak from float32 entries).
 __host__ __device__ constexpr int box_comps(int nf) { return nf + nf * (nf + 1) / 2; }
-__host__ __device__ constexpr int box_pad(int nf) { return (box_comps(nf) + 3) / 4 * 4; }
+__host__ __device__ constexpr int box_pad(int nf) { return (box_comps(nf) + 1) / 2 * 2; }
 // product k of nf features in row order: its two features
 __host__ __device__ constexpr int box_i(int k, int nf) {
     int i = 0;
@@ -38,7 +42,7 @@ struct Box {
 // B's box (ta, b); 2: also side B's over A's box (tb, a).
 struct BoxSums {
     int mode = 0;
-    const float *ta = nullptr, *tb = nullptr;
+    const double *ta = nullptr, *tb = nullptr;
     int cw = 0, ch = 0;
     Box a{}, b{};
 };
@@ -46,31 +50,28 @@ struct BoxSums {
 // A table's sums over the box [x0, x1) × [y0, y1) clipped to the grid, all comps: four corner reads of
 // whole entries, of which those on the grid's first row or column are zero and not made. Lanes of
 // consecutive shifts read consecutive entries at the corners that move with the shift and one entry
-// at those the grid's edge holds.
+// at those the grid's edge holds. The sums leave as float32, as a transform's do (their own rounding only;
+// float64 ones would not fit the score's registers).
 template <int NF>
-__device__ __forceinline__ void box_read(float (&v)[box_pad(NF)], const float* __restrict__ t, int cw, int ch, int x0,
+__device__ __forceinline__ void box_read(float (&v)[box_pad(NF)], const double* __restrict__ t, int cw, int ch, int x0,
                                          int x1, int y0, int y1) {
     constexpr int NP = box_pad(NF);
     x0 = max(x0, 0), y0 = max(y0, 0), x1 = min(x1, cw), y1 = min(y1, ch);
 #pragma unroll
     for (int i = 0; i < NP; ++i) v[i] = 0.f;
     if (x1 <= x0 || y1 <= y0) return;
-    auto add = [&](int x, int y, float sign) {
-        const float4* p = reinterpret_cast<const float4*>(t) + (size_t)(y - 1) * (NP / 4) * cw + (x - 1);
+    const double2* p = reinterpret_cast<const double2*>(t);
+    const size_t r0 = (size_t)(y0 - 1) * (NP / 2) * cw, r1 = (size_t)(y1 - 1) * (NP / 2) * cw;
+    const double2 zero = make_double2(0.0, 0.0);
 #pragma unroll
-        for (int q = 0; q < NP / 4; ++q) {
-            const float4 e = __ldg(p + (size_t)q * cw);
-            v[4 * q] = fmaf(sign, e.x, v[4 * q]);
-            v[4 * q + 1] = fmaf(sign, e.y, v[4 * q + 1]);
-            v[4 * q + 2] = fmaf(sign, e.z, v[4 * q + 2]);
-            v[4 * q + 3] = fmaf(sign, e.w, v[4 * q + 3]);
-        }
-    };
-    // neighbouring corners first: each row's difference, then the difference of the rows
-    if (x0 > 0 && y0 > 0) add(x0, y0, 1.f);
-    if (y0 > 0) add(x1, y0, -1.f);
-    if (x0 > 0) add(x0, y1, -1.f);
-    add(x1, y1, 1.f);
+    for (int q = 0; q < NP / 2; ++q) {
+        const size_t o = (size_t)q * cw;
+        const double2 e11 = __ldg(p + r1 + o + x1 - 1);
+        const double2 e01 = x0 > 0 ? __ldg(p + r1 + o + x0 - 1) : zero, e10 = y0 > 0 ? __ldg(p + r0 + o + x1 - 1) : zero;
+        const double2 e00 = x0 > 0 && y0 > 0 ? __ldg(p + r0 + o + x0 - 1) : zero;
+        v[2 * q] = (float)((e11.x - e01.x) - (e10.x - e00.x));
+        v[2 * q + 1] = (float)((e11.y - e01.y) - (e10.y - e00.y));
+    }
 }
 
 }  // namespace zc

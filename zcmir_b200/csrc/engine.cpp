@@ -726,7 +726,7 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
         bk.push_back((uint64_t)(uintptr_t)bt.p), bk.push_back(bt.gen);
         if (have[s] && bk == box_key_[s]) return true;
         if (!aux_after_st() ||
-            !cuda_ok(box_table(grid, g.cw, g.ch, job.cp.nf, bt.as<float>(), box_tmp_.p, aux_st_), "moment tables"))
+            !cuda_ok(box_table(grid, g.cw, g.ch, job.cp.nf, bt.as<double>(), box_tmp_.p, aux_st_), "moment tables"))
             return false;
         counts[0] += 3;
         box_key_[s] = bk;
@@ -780,7 +780,7 @@ bool Engine::run_map(MapJob& job, cudaEvent_t* ev, float* host_map) {
     }
     if (!ev && !st_after_aux()) return false;
     const bool tmem = row_pass != "split" && job.box.mode == 0 && rows_tmem_supported(g.nx, job.plan.n_corr);
-    job.box.ta = box_a_.as<float>(), job.box.tb = box_b_.as<float>();
+    job.box.ta = box_a_.as<double>(), job.box.tb = box_b_.as<double>();
     if (!tmem &&
         !cuda_ok(inverse_rows(q_.as<float2>(), g, job.plan, job.line, job.S, twiddles(g.nx), st), "inverse rows"))
         return false;

@@ -122,7 +122,7 @@ cudaError_t map_scores(const float2* Q, const MapGeom& g, const CombineParams& c
 // cells; t and tmp: box_table_bytes / box_scratch_bytes
 size_t box_table_bytes(int nf, int cw, int ch);
 size_t box_scratch_bytes(int nf, int cw, int ch);
-cudaError_t box_table(const float* grid, int cw, int ch, int nf, float* t, void* tmp, cudaStream_t st);
+cudaError_t box_table(const float* grid, int cw, int ch, int nf, double* t, void* tmp, cudaStream_t st);
 // both passes in one with the sums in tensor memory, a whole row per block (nx = 2048)
 bool rows_tmem_supported(int nx, int n_corr);
 cudaError_t inverse_rows_score_tmem(const float2* Q, const MapGeom& g, const CorrPlanDev& plan, const float2* tw_nx,
