@@ -15,10 +15,12 @@
 // within a tile are float32; those of the tiles and bands, the entries and a box's four corners are
 // float64, so a sum's error scales with its own box, where a float32 transform's scales with both planes'
 // energy: rms 0.04 (300² over 1000 × 900) to 0.8 (8² over 40²) of a transform's over 14 planes, blobs,
-// ramps and flat halves. Float32 entries were not enough: on 300 translations of pairs of 8 to 420
-// pixels a side, half of them ramps, steps or flat halves, the map's argmax left the float64 oracle's 11
-// times against 5 with all 45 correlations transformed; now 4 times, the rms error of cells 0.92 of theirs.
-// It costs a map of 1024² 0.1 ms (score 262 → 326 µs, tables 78 → 98).
+// ramps and flat halves. The score divides the sums by the exact number of pixels they cover. On 1800
+// translations of pairs of 8 to 420 pixels a side, half of them ramps, steps or flat halves, the rms error of
+// a map's cells is 0.61 of that with all 45 correlations transformed, and the argmax leaves the float64
+// oracle's 17 times against 26; turned, 0.91 and 62 against 75. Float32 entries, and the transform's n, were not
+// enough: 25 against 10 in 600 translations. They cost less, by 0.08 ms of a map of 1024² (score 262 against
+// 305 µs, tables 78 against 98).
 //
 // Built from tiles of 32 columns × 8 rows, a warp each, in three launches, so that the table (112
 // bytes a cell) is written once and the samples (20 bytes) are read twice: k_box_sums leaves each

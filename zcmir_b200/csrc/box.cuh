@@ -50,8 +50,10 @@ struct BoxSums {
 // A table's sums over the box [x0, x1) × [y0, y1) clipped to the grid, all comps: four corner reads of
 // whole entries, of which those on the grid's first row or column are zero and not made. Lanes of
 // consecutive shifts read consecutive entries at the corners that move with the shift and one entry
-// at those the grid's edge holds. The sums leave as float32, as a transform's do (their own rounding only;
-// float64 ones would not fit the score's registers).
+// at those the grid's edge holds. A row's two corners are loaded whole before they are used: taken pair by
+// pair, the loads followed one another (score of a 2048² map at a translation 0.45 → 0.33 ms with these). The
+// sums leave as float32, as a transform's do (their own rounding only; float64 ones would not fit the score's
+// registers).
 template <int NF>
 __device__ __forceinline__ void box_read(float (&v)[box_pad(NF)], const double* __restrict__ t, int cw, int ch, int x0,
                                          int x1, int y0, int y1) {
@@ -63,15 +65,25 @@ __device__ __forceinline__ void box_read(float (&v)[box_pad(NF)], const double* 
     const double2* p = reinterpret_cast<const double2*>(t);
     const size_t r0 = (size_t)(y0 - 1) * (NP / 2) * cw, r1 = (size_t)(y1 - 1) * (NP / 2) * cw;
     const double2 zero = make_double2(0.0, 0.0);
+    double d[NP];
+    auto row = [&](size_t r, bool sub) {
+        double2 hi[NP / 2], lo[NP / 2];
 #pragma unroll
-    for (int q = 0; q < NP / 2; ++q) {
-        const size_t o = (size_t)q * cw;
-        const double2 e11 = __ldg(p + r1 + o + x1 - 1);
-        const double2 e01 = x0 > 0 ? __ldg(p + r1 + o + x0 - 1) : zero, e10 = y0 > 0 ? __ldg(p + r0 + o + x1 - 1) : zero;
-        const double2 e00 = x0 > 0 && y0 > 0 ? __ldg(p + r0 + o + x0 - 1) : zero;
-        v[2 * q] = (float)((e11.x - e01.x) - (e10.x - e00.x));
-        v[2 * q + 1] = (float)((e11.y - e01.y) - (e10.y - e00.y));
-    }
+        for (int q = 0; q < NP / 2; ++q) {
+            hi[q] = __ldg(p + r + (size_t)q * cw + x1 - 1);
+            lo[q] = x0 > 0 ? __ldg(p + r + (size_t)q * cw + x0 - 1) : zero;
+        }
+#pragma unroll
+        for (int q = 0; q < NP / 2; ++q) {
+            const double a = hi[q].x - lo[q].x, b = hi[q].y - lo[q].y;
+            d[2 * q] = sub ? d[2 * q] - a : a;
+            d[2 * q + 1] = sub ? d[2 * q + 1] - b : b;
+        }
+    };
+    row(r1, false);
+    if (y0 > 0) row(r0, true);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) v[i] = (float)d[i];
 }
 
 }  // namespace zc

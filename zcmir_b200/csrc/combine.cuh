@@ -98,13 +98,12 @@ __device__ __forceinline__ bool overlap_alive(double n, const CombineParams& p, 
 // Per-shift score (smi.wgsl:825-915, combine_cell): centring, ridge, Cholesky factors and the
 // whitened norm in float64, the calibrated map's Wilson–Hilferty transform in float32; every
 // index known at compile time (NF features, exact or global whitening, calibrated or not), so the 4×4 algebra stays in
-// registers. n: this shift's overlap; `mean(c, 1 / n)` returns correlation c's sum over n (of the 45;
+// registers. n: this shift's overlap, above the floors (overlap_alive); `mean(c, 1 / n)` returns correlation c's sum over n (of the 45;
 // NF = 3 asks for none of the fourth feature's), and every c passed to it is a compile-time constant. Each Cholesky pivot is inverted once (rsqrt) and the
 // substitutions multiply by it.
 template <int NF, bool EXACT, bool CALIB, class G>
-__device__ __forceinline__ float combine_smi(G&& mean, double n, const CombineParams& p, double n00) {
+__device__ __forceinline__ float combine_smi(G&& mean, double n, const CombineParams& p) {
     const double neff = n / fmax(p.area, 1.0);
-    if (!overlap_alive<CALIB>(n, p, n00)) return 0.f;
     const double rn = 1.0 / fmax(n, 1e-8);
     auto S = [&](int c) -> double { return mean(c, rn); };
     double ma[NF], mb[NF], C[NF][NF];
@@ -225,6 +224,7 @@ __device__ __forceinline__ float combine_t(G&& raw, const CombineParams& p, doub
     if constexpr (NF == 1) {
         return combine_ncc(n, n00);
     } else {
+        if (!overlap_alive<CALIB>(n, p, n00)) return 0.f;
         double scale = 0.0;  // inv_nn / n, once per shift
         bool have = false;
         return combine_smi<NF, EXACT, CALIB>(
@@ -232,7 +232,7 @@ __device__ __forceinline__ float combine_t(G&& raw, const CombineParams& p, doub
                 if (!have) scale = p.inv_nn * rn, have = true;
                 return (double)raw(c) * scale;
             },
-            n, p, n00);
+            n, p);
     }
 }
 

@@ -66,11 +66,18 @@ __global__ void __launch_bounds__(kScoreThreads, 2) k_score(const float* __restr
             if constexpr (MODE == 0) {
                 sc = combine_t<NF, EXACT, CALIB>(fft, cpr, n00);
             } else {
-                const double n = (double)fft(0) * cpr.inv_nn;
+                double n = (double)fft(0) * cpr.inv_nn;
                 sc = 0.f;
                 if (overlap_alive<CALIB>(n, cpr, n00)) {
                     // the lag: A's cells b + t against B's box, B's cells a − t against A's
                     const int tx = x <= nx / 2 ? x : x - nx, ty = y <= ny / 2 ? y : y - ny;
+                    // The moments are those of whole pixels, and the score divides by their exact number:
+                    // the boxes' common cells, or the transform's sum rounded. (The transform's error in
+                    // n, cancelled against exact moments, was most of what flat parts' covariances had.)
+                    if (MODE == 2)
+                        n = (double)max(min(bx.b.x1 + tx, bx.a.x1) - max(bx.b.x0 + tx, bx.a.x0), 0) *
+                            (double)max(min(bx.b.y1 + ty, bx.a.y1) - max(bx.b.y0 + ty, bx.a.y0), 0);
+                    else n = rint(n);
                     float va[box_pad(NF)], vb[box_pad(NF)];
                     box_read<NF>(va, bx.ta, bx.cw, bx.ch, bx.b.x0 + tx, bx.b.x1 + tx, bx.b.y0 + ty, bx.b.y1 + ty);
                     if (MODE == 2)
@@ -82,7 +89,7 @@ __global__ void __launch_bounds__(kScoreThreads, 2) k_score(const float* __restr
                             const double v = (double)(from.src[c] == 1 ? va[from.at[c]] : vb[from.at[c]]) * rn;
                             return from.diag[c] ? v + 1.0 : v;
                         },
-                        n, cpr, n00);
+                        n, cpr);
                 }
             }
             const uint32_t idx = (uint32_t)y * (uint32_t)nx + (uint32_t)x;
