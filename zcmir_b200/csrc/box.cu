@@ -20,7 +20,7 @@
 // a map's cells is 0.61 of that with all 45 correlations transformed, and the argmax leaves the float64
 // oracle's 17 times against 26; turned, 0.91 and 62 against 75. Float32 entries, and the transform's n, were not
 // enough: 25 against 10 in 600 translations. They cost less, by 0.08 ms of a map of 1024² (score 262 against
-// 305 µs, tables 78 against 98).
+// 313 µs, tables 78 against 98).
 //
 // Built from tiles of 32 columns × 8 rows, a warp each, in three launches, so that the table (112
 // bytes a cell) is written once and the samples (20 bytes) are read twice: k_box_sums leaves each

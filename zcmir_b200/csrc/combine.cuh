@@ -97,9 +97,10 @@ __device__ __forceinline__ bool overlap_alive(double n, const CombineParams& p, 
 
 // Per-shift score (smi.wgsl:825-915, combine_cell): centring, ridge, Cholesky factors and the
 // whitened norm in float64, the calibrated map's Wilson–Hilferty transform in float32; every
-// index known at compile time (NF features, exact or global whitening, calibrated or not), so the 4×4 algebra stays in
-// registers. n: this shift's overlap, above the floors (overlap_alive); `mean(c, 1 / n)` returns correlation c's sum over n (of the 45;
-// NF = 3 asks for none of the fourth feature's), and every c passed to it is a compile-time constant. Each Cholesky pivot is inverted once (rsqrt) and the
+// index known at compile time (NF features, exact or global whitening, calibrated or not), so the 4×4
+// algebra stays in registers. n: this shift's overlap, above the floors (overlap_alive); `mean(c, 1 / n)`
+// returns correlation c's sum over n (of the 45; NF = 3 asks for none of the fourth feature's), and every c
+// passed to it is a compile-time constant. Each Cholesky pivot is inverted once (rsqrt) and the
 // substitutions multiply by it.
 template <int NF, bool EXACT, bool CALIB, class G>
 __device__ __forceinline__ float combine_smi(G&& mean, double n, const CombineParams& p) {
